@@ -300,8 +300,7 @@ def prepare(case, seed):
 def run(s):
     e = s["engine"]
     if s["kind"] == "scf":
-        tight = dict(max_iter=100, energy_tol=1e-10, density_tol=1e-9, diis_tol=1e-9)
-        r, Da, _ = e.scf(s["Z"], s["xyz"], opts=tight)
+        r, Da, _ = e.scf(s["Z"], s["xyz"], opts=dict(max_iter=100, energy_tol=1e-8, density_tol=1e-7, diis_tol=1e-7))
         return {"e_total": r["e_total"], "D_alpha": Da}
     if s["kind"] == "gradient":
         return e.gradient(s["Z"], s["xyz"], s["Da"], s["Db"], s["W"], precision=s["precision"])[0]
