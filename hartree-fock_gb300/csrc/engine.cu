@@ -206,7 +206,6 @@ struct hfg_engine
     hfg::DevBuf<int2> d_cls_molseg[hfg::kNumPairClasses];
     hfg::DevBuf<unsigned> d_bra_cnt[hfg::kNumQuartetClasses];            // per bra pair: survivors (fp64, fp32)
     hfg::DevBuf<unsigned long long> d_bra_off[hfg::kNumQuartetClasses];  // per bra pair: list offsets
-    hfg::DevBuf<unsigned long long> d_scan_tmp;
 
     // Quartet lists (capacity for the Schwartz threshold they were sized for).
     double cap_thr = -1.0;
@@ -342,37 +341,47 @@ __device__ __forceinline__ float narrow_nonneg(long long b)
     return __int_as_float(((e - 896) << 23) | static_cast<int>((b >> 29) & 0x7fffff));
 }
 
-struct BuildArgs
+// One quartet class of a list build.
+struct ClassBuild
 {
     const int* ids1;
     const double* Q1;
-    int n1;
-    int base1, base2; // sorted-array index of position 0 of each class (what the lists hold)
+    const float* Qf1;
     const double* Q2;
+    const float* Qf2;
     const int2* sh2;     // (sh1, sh2) per ket position
     const int4* seg2;    // ket class segments (equal primitive-pair count, Q descending inside)
     const int2* molseg2; // per molecule: ket segment range
-    bool same_class;
+    unsigned* bra_cnt;             // [n1][2]
+    unsigned long long* bra_off;   // [n1][2] exclusive offsets (pass 1)
+    Quartet* out64;
+    Quartet* out32;
+    unsigned long long cap; // list capacity (the Schwartz-only count): writes beyond it are dropped
+    int qc;
+    int n1;
+    int base1, base2; // sorted-array index of position 0 of each class (what the lists hold)
+    int first_block;  // of the class in the launch over all classes (kBuildWarps bra pairs per block)
+    int same_class;
+};
+constexpr int kBuildWarps = 4;
+
+// All classes of a build, worked through by one launch per pass: 21 launches a pass, each with its own ramp
+// and tail, took 0.12 of the 0.2 ms that the lists of one water cost.
+struct BuildArgs
+{
+    ClassBuild cls[kNumQuartetClasses];
+    int ncls;
     const PairRec* pairs;
-    const double* Mt;
-    const double* Mt2; // 2 * Mt
+    const double* Mt2; // 2 * shell maxima of |dD_tot|
     const double* Ma;
     const double* Mb; // null for RHF
-    const float* Qf1;
-    const float* Qf2;
     const long long* smax_off;
     const int* nsh;
     double sthr, dthr;
     float cutoff;
     int mixed;
-    int pass;                      // 0: count per bra pair, 1: write at the scanned offsets
-    unsigned* bra_cnt;             // [n1][2]
-    const unsigned long long* bra_off; // [n1][2] exclusive offsets (pass 1)
-    Quartet* out64;
-    Quartet* out32;
-    unsigned long long* prim64;
-    unsigned long long* prim32;
-    unsigned long long cap; // list capacity (the Schwartz-only count): writes beyond it are dropped
+    int pass;                   // 0: count per bra pair, 1: write at the scanned offsets
+    unsigned long long* counts; // [2 qc + prec] quartets, then [2 qc + prec] primitive quartets
 };
 
 // Survival list of one quartet class in two deterministic passes, one warp per bra pair.  Ket
@@ -382,32 +391,35 @@ struct BuildArgs
 // bra pair and precision, pass 1 writes them at scanned offsets in candidate order, so the list is
 // ordered by bra pair and, inside a bra pair, by ket primitive count: a warp of the class kernels sees
 // quartets of equal primitive counts.  FP32 / FP64 split by the quartet bound Q_i Q_j max|dD|.
-__global__ void build_lists_kernel(BuildArgs a)
+__global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __grid_constant__ BuildArgs b)
 {
+    int ci = 0;
+    while (ci + 1 < b.ncls && b.cls[ci + 1].first_block <= static_cast<int>(blockIdx.x)) ++ci;
+    const ClassBuild& a = b.cls[ci];
     const int lane = threadIdx.x & 31;
-    const int i    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int i    = (static_cast<int>(blockIdx.x) - a.first_block) * kBuildWarps + (threadIdx.x >> 5);
     if (i >= a.n1)
         return;
     const int pid_i  = a.ids1[i];
     const double Qi  = a.Q1[i];
-    const PairRec pi = a.pairs[pid_i];
+    const PairRec pi = b.pairs[pid_i];
     const int2 ms    = a.molseg2[pi.mol];
-    const long long so = a.smax_off[pi.mol];
-    const int ns = a.nsh[pi.mol];
+    const long long so = b.smax_off[pi.mol];
+    const int ns = b.nsh[pi.mol];
     // The shell-max matrices are symmetric: index them so that the ket shell (which varies across the
     // lanes) is the contiguous one.  Every value here is >= 0, and for non-negative doubles the order of
     // the IEEE bit patterns is the numeric order, so the maxima and the density test run as exact 64-bit
     // integer operations (GB300's FP64 pipe is 1/64 of its FP32 rate); the Schwartz product stays FP64.
     auto bits = [](const double* m, long long i) { return __double_as_longlong(m[i]); };
     const int sa = pi.sh1, sb = pi.sh2;
-    const long long dab = bits(a.Mt2, so + sa + (long long)sb * ns);
-    const long long dthr = __double_as_longlong(a.dthr);
+    const long long dab = bits(b.Mt2, so + sa + (long long)sb * ns);
+    const long long dthr = __double_as_longlong(b.dthr);
     const long long ra = so + (long long)sa * ns, rb2 = so + (long long)sb * ns;
     const float Qfi = a.Qf1[i];
     unsigned c64 = 0, c32 = 0;
     unsigned long long p64 = 0, p32 = 0;
-    const unsigned long long o64 = a.pass ? a.bra_off[2 * i] : 0ull;
-    const unsigned long long o32 = a.pass ? a.bra_off[2 * i + 1] : 0ull;
+    const unsigned long long o64 = b.pass ? a.bra_off[2 * i] : 0ull;
+    const unsigned long long o32 = b.pass ? a.bra_off[2 * i + 1] : 0ull;
     for (int sidx = ms.x; sidx < ms.y; ++sidx)
     {
         const int4 seg = a.seg2[sidx];
@@ -419,7 +431,7 @@ __global__ void build_lists_kernel(BuildArgs a)
         while (lo < hi)
         {
             const int mid = (lo + hi) >> 1;
-            if (Qi * a.Q2[mid] < a.sthr)
+            if (Qi * a.Q2[mid] < b.sthr)
                 hi = mid;
             else
                 lo = mid + 1;
@@ -433,15 +445,15 @@ __global__ void build_lists_kernel(BuildArgs a)
             {
                 const int2 scd = a.sh2[j];
                 const int sc = scd.x, sd = scd.y;
-                long long md = max(dab, bits(a.Mt2, so + sc + (long long)sd * ns));
-                md = max(md, max(max(bits(a.Ma, ra + sc), bits(a.Ma, ra + sd)), max(bits(a.Ma, rb2 + sc), bits(a.Ma, rb2 + sd))));
-                if (a.Mb)
-                    md = max(md, max(max(bits(a.Mb, ra + sc), bits(a.Mb, ra + sd)), max(bits(a.Mb, rb2 + sc), bits(a.Mb, rb2 + sd))));
+                long long md = max(dab, bits(b.Mt2, so + sc + (long long)sd * ns));
+                md = max(md, max(max(bits(b.Ma, ra + sc), bits(b.Ma, ra + sd)), max(bits(b.Ma, rb2 + sc), bits(b.Ma, rb2 + sd))));
+                if (b.Mb)
+                    md = max(md, max(max(bits(b.Mb, ra + sc), bits(b.Mb, ra + sd)), max(bits(b.Mb, rb2 + sc), bits(b.Mb, rb2 + sd))));
                 if (md >= dthr)
                 {
                     bool lowp = false;
-                    if (a.mixed) // the FP32/FP64 split is this engine's own heuristic: evaluated in FP32
-                        lowp = Qfi * a.Qf2[j] * narrow_nonneg(md) < a.cutoff;
+                    if (b.mixed) // the FP32/FP64 split is this engine's own heuristic: evaluated in FP32
+                        lowp = Qfi * a.Qf2[j] * narrow_nonneg(md) < b.cutoff;
                     s32 = lowp;
                     s64 = !lowp;
                 }
@@ -449,7 +461,7 @@ __global__ void build_lists_kernel(BuildArgs a)
             const unsigned m64 = __ballot_sync(0xffffffffu, s64);
             const unsigned m32 = __ballot_sync(0xffffffffu, s32);
             const unsigned lt  = (1u << lane) - 1u;
-            if (a.pass)
+            if (b.pass)
             {
                 const Quartet qv {static_cast<uint32_t>(a.base1 + i), static_cast<uint32_t>(a.base2 + j)};
                 const unsigned long long w64 = o64 + c64 + __popc(m64 & lt), w32 = o32 + c32 + __popc(m32 & lt);
@@ -465,82 +477,86 @@ __global__ void build_lists_kernel(BuildArgs a)
             p32 += pp * __popc(m32);
         }
     }
-    if (a.pass == 0 && lane == 0)
+    if (b.pass == 0 && lane == 0)
     {
         a.bra_cnt[2 * i]     = c64;
         a.bra_cnt[2 * i + 1] = c32;
+        unsigned long long* prims = b.counts + 2 * kNumQuartetClasses + 2 * a.qc;
         if (p64)
-            atomicAdd(a.prim64, p64);
+            atomicAdd(prims, p64);
         if (p32)
-            atomicAdd(a.prim32, p32);
+            atomicAdd(prims + 1, p32);
     }
 }
 
-// Exclusive scan of the per-bra counts (two interleaved sequences, fp64 and fp32) in three steps:
-// per-block scan, scan of the block totals (one block), add the block offsets.  The grand totals land
-// in total[0..1] (the class kernels' list lengths).
-constexpr int kScanBlock = 1024;
-__global__ void scan_block_kernel(const unsigned* __restrict__ cnt, unsigned long long* __restrict__ off, int n,
-                                  unsigned long long* __restrict__ block_tot)
+// Exclusive scan of the per-bra counts (two interleaved sequences, fp64 and fp32), one block per class: the
+// block walks the class's bra pairs kScanBlock * kScanItems at a time with a running total, and leaves
+// the grand totals in counts[2 qc], counts[2 qc + 1] (the class kernels' list lengths).  One block is enough:
+// the longest class of (H2O)_64 (115k bra pairs) is 29 rounds.
+constexpr int kScanBlock = 1024, kScanItems = 4;
+__global__ void __launch_bounds__(kScanBlock) scan_lists_kernel(const __grid_constant__ BuildArgs b)
 {
+    const ClassBuild& a = b.cls[blockIdx.x];
     __shared__ unsigned long long warp_tot[2][32];
-    const int i = blockIdx.x * kScanBlock + threadIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int q = 0; q < 2; ++q)
+    unsigned long long run[2] = {0ull, 0ull};
+    for (int base = 0; base < a.n1; base += kScanBlock * kScanItems)
     {
-        unsigned long long v = i < n ? cnt[2 * i + q] : 0ull, x = v;
-        for (int o = 1; o < 32; o <<= 1)
+        const int i0 = base + static_cast<int>(threadIdx.x) * kScanItems;
+        uint2 c[kScanItems];
+        unsigned long long own[2] = {0ull, 0ull}, x[2];
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k)
         {
-            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o)
-                x += y;
+            c[k] = i0 + k < a.n1 ? reinterpret_cast<const uint2*>(a.bra_cnt)[i0 + k] : make_uint2(0u, 0u);
+            own[0] += c[k].x;
+            own[1] += c[k].y;
         }
-        if (lane == 31)
-            warp_tot[q][w] = x;
-        __syncthreads();
-        if (w == 0)
-        {
-            unsigned long long t = warp_tot[q][lane], tx = t;
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const unsigned long long y = __shfl_up_sync(0xffffffffu, tx, o);
-                if (lane >= o)
-                    tx += y;
-            }
-            warp_tot[q][lane] = tx - t; // exclusive warp offsets
-            if (lane == 31)
-                block_tot[2 * blockIdx.x + q] = tx;
-        }
-        __syncthreads();
-        if (i < n)
-            off[2 * i + q] = x - v + warp_tot[q][w];
-        __syncthreads();
-    }
-}
-
-__global__ void scan_tops_kernel(unsigned long long* __restrict__ block_tot, int nb, unsigned long long* __restrict__ total)
-{
-    if (threadIdx.x == 0)
+#pragma unroll
         for (int q = 0; q < 2; ++q)
         {
-            unsigned long long run = 0;
-            for (int b = 0; b < nb; ++b)
+            x[q] = own[q];
+            for (int o = 1; o < 32; o <<= 1)
             {
-                const unsigned long long t = block_tot[2 * b + q];
-                block_tot[2 * b + q] = run;
-                run += t;
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, x[q], o);
+                if (lane >= o)
+                    x[q] += y;
             }
-            total[q] = run;
+            if (lane == 31)
+                warp_tot[q][w] = x[q];
         }
-}
-
-__global__ void scan_add_kernel(unsigned long long* __restrict__ off, int n, const unsigned long long* __restrict__ block_tot)
-{
-    const int i = blockIdx.x * kScanBlock + threadIdx.x;
-    if (i < n)
+        __syncthreads();
+        if (w < 2) // warp w turns sequence w's warp totals into inclusive sums
+        {
+            unsigned long long t = warp_tot[w][lane];
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, t, o);
+                if (lane >= o)
+                    t += y;
+            }
+            warp_tot[w][lane] = t;
+        }
+        __syncthreads();
+        unsigned long long off[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) off[q] = run[q] + (w > 0 ? warp_tot[q][w - 1] : 0ull) + x[q] - own[q];
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k)
+        {
+            if (i0 + k < a.n1)
+                reinterpret_cast<ulonglong2*>(a.bra_off)[i0 + k] = make_ulonglong2(off[0], off[1]);
+            off[0] += c[k].x;
+            off[1] += c[k].y;
+        }
+        run[0] += warp_tot[0][31];
+        run[1] += warp_tot[1][31];
+        __syncthreads(); // the next round overwrites warp_tot
+    }
+    if (threadIdx.x == 0)
     {
-        off[2 * i] += block_tot[2 * blockIdx.x];
-        off[2 * i + 1] += block_tot[2 * blockIdx.x + 1];
+        b.counts[2 * a.qc]     = run[0];
+        b.counts[2 * a.qc + 1] = run[1];
     }
 }
 
@@ -1162,65 +1178,58 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
     const int ncnt = kNumQuartetClasses * 2;
     e->d_counts.alloc(2 * ncnt + 1);
     HFG_CUDA(cudaMemsetAsync(e->d_counts.p, 0, sizeof(unsigned long long) * (2 * ncnt + 1), s));
+    BuildArgs a {};
+    int blocks = 0;
+    // Heavy classes first, as the class kernels run them.
+    for (int qc = kNumQuartetClasses - 1; qc >= 0; --qc)
+    {
+        const int P1 = [&] { int p = 0; while ((p + 1) * (p + 2) / 2 <= qc) ++p; return p; }();
+        const int P2 = qc - P1 * (P1 + 1) / 2;
+        if (e->cap[qc] == 0 || e->cls_ids[P1].empty() || e->cls_ids[P2].empty())
+            continue;
+        ClassBuild& c = a.cls[a.ncls++];
+        c.qc          = qc;
+        c.ids1        = e->d_cls_ids[P1].p;
+        c.base1       = e->cls_base[P1];
+        c.base2       = e->cls_base[P2];
+        c.Q1          = e->d_cls_Q[P1].p;
+        c.n1          = static_cast<int>(e->cls_ids[P1].size());
+        c.Q2          = e->d_cls_Q[P2].p;
+        c.sh2         = e->d_cls_sh[P2].p;
+        c.seg2        = e->d_cls_seg[P2].p;
+        c.molseg2     = e->d_cls_molseg[P2].p;
+        c.same_class  = P1 == P2 ? 1 : 0;
+        c.Qf1         = e->d_cls_Qf[P1].p;
+        c.Qf2         = e->d_cls_Qf[P2].p;
+        c.bra_cnt     = e->d_bra_cnt[qc].p;
+        c.bra_off     = e->d_bra_off[qc].p;
+        c.out64       = e->d_list[qc][0].p;
+        c.out32       = mixed ? e->d_list[qc][1].p : nullptr;
+        c.cap         = e->cap[qc];
+        c.first_block = blocks;
+        blocks += (c.n1 + kBuildWarps - 1) / kBuildWarps;
+    }
+    a.pairs    = e->d_pairs.p;
+    a.Mt2      = e->d_smax2.p;
+    a.Ma       = e->d_smax[1].p;
+    a.Mb       = uhf ? e->d_smax[2].p : nullptr;
+    a.smax_off = e->d_smax_off.p;
+    a.nsh      = e->d_nsh.p;
+    a.sthr     = sthr;
+    a.dthr     = dthr;
+    a.cutoff   = static_cast<float>(cutoff);
+    a.mixed    = mixed ? 1 : 0;
+    a.counts   = e->d_counts.p;
     int launches = 0;
-    size_t max_blocks = 1;
-    for (int P1 = 0; P1 < kNumPairClasses; ++P1)
-        max_blocks = std::max(max_blocks, (e->cls_ids[P1].size() + kScanBlock - 1) / kScanBlock);
-    e->d_scan_tmp.alloc(2 * max_blocks);
-    for (int pass = 0; pass < 2; ++pass)
-        for (int P1 = 0; P1 < kNumPairClasses; ++P1)
-            for (int P2 = 0; P2 <= P1; ++P2)
-            {
-                const int qc = quartet_class(P1, P2);
-                if (e->cap[qc] == 0 || e->cls_ids[P1].empty() || e->cls_ids[P2].empty())
-                    continue;
-                BuildArgs a {};
-                a.ids1 = e->d_cls_ids[P1].p;
-                a.base1 = e->cls_base[P1];
-                a.base2 = e->cls_base[P2];
-                a.Q1   = e->d_cls_Q[P1].p;
-                a.n1   = static_cast<int>(e->cls_ids[P1].size());
-                a.Q2   = e->d_cls_Q[P2].p;
-                a.sh2  = e->d_cls_sh[P2].p;
-                a.seg2 = e->d_cls_seg[P2].p;
-                a.molseg2 = e->d_cls_molseg[P2].p;
-                a.same_class = P1 == P2;
-                a.pairs = e->d_pairs.p;
-                a.Mt = e->d_smax[0].p;
-                a.Mt2 = e->d_smax2.p;
-                a.Ma = e->d_smax[1].p;
-                a.Mb = uhf ? e->d_smax[2].p : nullptr;
-                a.Qf1 = e->d_cls_Qf[P1].p;
-                a.Qf2 = e->d_cls_Qf[P2].p;
-                a.smax_off = e->d_smax_off.p;
-                a.nsh = e->d_nsh.p;
-                a.sthr = sthr;
-                a.dthr = dthr;
-                a.cutoff = static_cast<float>(cutoff);
-                a.mixed = mixed ? 1 : 0;
-                a.pass = pass;
-                a.bra_cnt = e->d_bra_cnt[qc].p;
-                a.bra_off = e->d_bra_off[qc].p;
-                a.out64 = e->d_list[qc][0].p;
-                a.out32 = mixed ? e->d_list[qc][1].p : nullptr;
-                a.prim64 = e->d_counts.p + ncnt + 2 * qc;
-                a.prim32 = e->d_counts.p + ncnt + 2 * qc + 1;
-                a.cap = e->cap[qc];
-                const long long threads = static_cast<long long>(a.n1) * 32;
-                build_lists_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, s>>>(a);
-                HFG_CUDA(cudaGetLastError());
-                ++launches;
-                if (pass == 0)
-                {
-                    const int nb = (a.n1 + kScanBlock - 1) / kScanBlock;
-                    scan_block_kernel<<<nb, kScanBlock, 0, s>>>(e->d_bra_cnt[qc].p, e->d_bra_off[qc].p, a.n1,
-                                                                e->d_scan_tmp.p);
-                    scan_tops_kernel<<<1, 32, 0, s>>>(e->d_scan_tmp.p, nb, e->d_counts.p + 2 * qc);
-                    scan_add_kernel<<<nb, kScanBlock, 0, s>>>(e->d_bra_off[qc].p, a.n1, e->d_scan_tmp.p);
-                    HFG_CUDA(cudaGetLastError());
-                    launches += 3;
-                }
-            }
+    if (a.ncls > 0)
+    {
+        build_lists_kernel<<<static_cast<unsigned>(blocks), 32 * kBuildWarps, 0, s>>>(a);
+        scan_lists_kernel<<<static_cast<unsigned>(a.ncls), kScanBlock, 0, s>>>(a);
+        a.pass = 1;
+        build_lists_kernel<<<static_cast<unsigned>(blocks), 32 * kBuildWarps, 0, s>>>(a);
+        HFG_CUDA(cudaGetLastError());
+        launches = 3;
+    }
     if (graph)
         return launches + nspin;
     e->h_counts.assign(2 * ncnt + 1, 0);
