@@ -17,6 +17,18 @@
 //
 // Nearest-point expansion keeps |d| <= h/2, so the truncation error is below (h/2)^K / K! relative:
 // 1.2e-15 (FP64) and 2.6e-9 (FP32).
+//
+// The FP64 kernels that compute these scalars once per lane (the thread and chunk forms, the gradient) are
+// bound by the FP64 pipe, where a warp instruction takes 16 cycles of the SM, and use a third slice with
+// shorter polynomials (BoysFast below): Taylor polynomials of degree 13 economised by taking off their leading
+// Chebyshev polynomials one by one (Lanczos 1938), six coefficients for F_L and seven for e^d:
+//
+//   FP64     1/32     6         962 points    962 x 7 doubles = 53.9 KB    (h/2)^6 / (2^5 6!) = 6.3e-16
+//
+// F_L and e^{-T} together take 11 DFMA instead of 13, the grid point is found in FP32, and the downward
+// recursion runs on values that carry the prefactor already (scaled_boys); over T in [0, 30] its largest
+// relative error against a long-double series is 4.0e-16 / 1.2e-15 / 1.8e-15 for L = 1 / 4 / 9, that of
+// boys_eval times the prefactor powers 4.7e-16 / 1.2e-15 / 2.1e-15.  The other forms keep the smaller slice.
 #pragma once
 
 #include "hfg_common.cuh"
@@ -97,6 +109,92 @@ template <typename Real> constexpr int kRoundMagicLow = 0;
 template <> constexpr int kRoundMagicLow<double> = 0;          // low 32 bits of 1.5*2^52 are zero
 template <> constexpr int kRoundMagicLow<float>  = 0x400000;   // mantissa of 1.5*2^23
 
+// The grid of scaled_boys.
+struct BoysFast
+{
+    static constexpr double kStep    = 0.03125;
+    static constexpr double kInvStep = 32.0;
+    static constexpr int kTerms      = 6;
+    static constexpr int kPoints     = 962;
+    static constexpr int kRow        = kTerms + 1; // coefficients + e^{-T_i}; odd, so rows spread over the banks
+};
+
+// Economises a polynomial c[0..n) in x on |x| <= r to its first `keep` coefficients (constexpr: also the
+// coefficients of e^x below).  T_k(x/r) / 2^{k-1} scaled to leading coefficient 1 is subtracted from the top.
+constexpr void economise(double* c, int n, int keep, double r)
+{
+    using F = double;
+    for (int k = n - 1; k >= keep; --k)
+    {
+        // Chebyshev coefficients of T_k by T_{j+1} = 2 x T_j - T_{j-1}.
+        F a[24] {}, b[24] {};
+        a[0] = F(1);
+        b[1] = F(1);
+        for (int j = 1; j < k; ++j)
+        {
+            F t[24] {};
+            for (int i = 0; i <= j; ++i) t[i + 1] = F(2) * b[i];
+            for (int i = 0; i <= j; ++i) t[i] -= a[i];
+            for (int i = 0; i <= j + 1; ++i)
+            {
+                a[i] = b[i];
+                b[i] = t[i];
+            }
+        }
+        const F top = c[k];
+        F rk        = F(1); // r^(k - i)
+        for (int i = k; i >= 0; --i, rk *= r) c[i] -= top * rk * b[i] / b[k];
+    }
+}
+
+// Coefficient k of the economised e^x on |x| <= h/2; one more than F_L has, because e^x has
+// nothing like F_{L+6}/F_L <= 1/13 in its error term (6.3e-16 with six, 1e-18 with seven).
+constexpr int kExpTerms = BoysFast::kTerms + 1;
+constexpr double exp_coefficient(int k)
+{
+    double c[14] {};
+    for (int i = 0; i < 14; ++i) c[i] = inv_fact(i);
+    economise(c, 14, kExpTerms, BoysFast::kStep / 2);
+    return c[k];
+}
+template <int K> constexpr double kExpCoefficient = exp_coefficient(K);
+
+// Host: the BoysFast slice of total angular momentum L, row-major [point][kRow].
+inline std::vector<double> boys_fast_slice_host(int L)
+{
+    using G               = BoysFast;
+    constexpr int kTaylor = 14;
+    std::vector<double> out(static_cast<size_t>(G::kPoints) * G::kRow);
+    double eco[kTaylor][kTaylor] {}; // what economising moves from coefficient k to the lower ones
+    for (int k = G::kTerms; k < kTaylor; ++k)
+    {
+        eco[k][k] = 1.0;
+        economise(eco[k], kTaylor, G::kTerms, G::kStep / 2);
+    }
+    for (int i = 0; i < G::kPoints; ++i)
+    {
+        // The orders from the highest by the downward recursion, then the Taylor coefficients F_{L+k} / k!.
+        const long double Ti = i * static_cast<long double>(G::kStep), e = std::exp(-Ti);
+        long double c[kTaylor], kfact = 1.0L;
+        c[kTaylor - 1] = boys_series_host(L + kTaylor - 1, Ti);
+        for (int k = kTaylor - 1; k > 0; --k) c[k - 1] = (2 * Ti * c[k] + e) / (2 * (L + k) - 1);
+        for (int k = 2; k < kTaylor; ++k)
+        {
+            kfact *= k;
+            c[k] /= kfact;
+        }
+        double* row = &out[static_cast<size_t>(i) * G::kRow];
+        for (int j = 0; j < G::kTerms; ++j)
+        {
+            double moved = 0.0;
+            for (int k = kTaylor - 1; k >= G::kTerms; --k) moved += static_cast<double>(c[k]) * eco[k][j];
+            row[j] = static_cast<double>(c[j] + moved);
+        }
+        row[G::kTerms] = static_cast<double>(e);
+    }
+    return out;
+}
+
 #ifdef __CUDACC__
 __device__ __forceinline__ int bits_low(double y) { return __double2loint(y); }
 __device__ __forceinline__ int bits_low(float y) { return __float_as_int(y) & 0x7fffff; }
@@ -136,6 +234,95 @@ template <int L, typename Real> __device__ __forceinline__ void boys_eval(Real T
         const Real twoT = T + T;
 #pragma unroll
         for (int m = L; m >= 1; --m) F[m - 1] = (twoT * F[m] + e) * Real(1.0 / (2 * m - 1));
+    }
+}
+
+// Widening to double for the FP64 accumulators without the FP64 pipe (GB300 runs float -> double
+// conversions there, at 1/64 of the FP32 rate): the IEEE-754 fields are moved with integer operations.
+// Exact for normal numbers and zero; float subnormals (< 1.2e-38) become zero; infinities and NaNs keep
+// their class.
+__device__ __forceinline__ double widen(float x)
+{
+    const unsigned u                 = __float_as_uint(x);
+    const unsigned e                 = (u >> 23) & 0xffu;
+    const unsigned long long sign    = static_cast<unsigned long long>(u & 0x80000000u) << 32;
+    const unsigned long long de      = e == 0xffu ? 0x7ffull : static_cast<unsigned long long>(e + 896u);
+    const unsigned long long normal  = sign | (de << 52) | (static_cast<unsigned long long>(u & 0x7fffffu) << 29);
+    return __longlong_as_double(static_cast<long long>(e == 0u ? sign : normal));
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+
+// |x| as a float by integer operations, truncated (below FP32's normal range 0, above it +inf).
+__device__ __forceinline__ float narrow_abs(double x)
+{
+    const unsigned hi = static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu, lo = static_cast<unsigned>(__double2loint(x));
+    if (hi < 0x38100000u)
+        return 0.0f;
+    if (hi >= 0x47f00000u)
+        return __uint_as_float(0x7f800000u);
+    return __uint_as_float(((hi - 0x38000000u) << 3) | (lo >> 29));
+}
+
+// s^N.
+template <int N> __device__ __forceinline__ double power(double s)
+{
+    if constexpr (N == 1)
+        return s;
+    else if constexpr (N % 2 == 0)
+    {
+        const double h = power<N / 2>(s);
+        return h * h;
+    }
+    else
+        return s * power<N - 1>(s);
+}
+
+// f[m] = c s^m F_m(T), m = 0..L, with s = -2 rho and T = rho R2: what the R recursion starts from.  The
+// recursion runs on the scaled values, f_{m-1} = (c s^{m-1} e^{-T} - R2 f_m) / (2m - 1) (2T = -s R2), which
+// saves scaling each order, and the grid point is found in FP32 (an index off by one at a cell's edge only
+// lets |d| exceed h/2 by an ulp of FP32).
+template <int L> __device__ __forceinline__ void scaled_boys(double c, double s, double R2, const double* __restrict__ slice, double* f)
+{
+    using G          = BoysFast;
+    const double m2T = s * R2; // -2T
+    const float t2   = narrow_abs(m2T);
+    if (t2 > static_cast<float>(2.0 * kBoysAsymptotic))
+    {
+        const double r = hfg_rsqrt(-0.5 * m2T);
+        f[0]           = (c * kSqrtPiBy2) * r;
+        if constexpr (L > 0)
+        {
+            const double g = s * (r * r); // f_{m+1} = s (m + 1/2) f_m / T
+#pragma unroll
+            for (int m = 0; m < L; ++m) f[m + 1] = ((m + 0.5) * g) * f[m];
+        }
+        return;
+    }
+    const float y   = fmaf(t2, static_cast<float>(0.5 * G::kInvStep), static_cast<float>(kRoundMagic<float>));
+    const int pt    = max(0, min(__float_as_int(y) - __float_as_int(static_cast<float>(kRoundMagic<float>)), G::kPoints - 1));
+    const float ti  = (y - static_cast<float>(kRoundMagic<float>)) * static_cast<float>(G::kStep); // exact
+    const double x  = fma(0.5, m2T, widen(ti));                                                    // T_i - T
+    const double* g = slice + pt * G::kRow;
+    double F        = g[G::kTerms - 1];
+#pragma unroll
+    for (int k = G::kTerms - 2; k >= 0; --k) F = F * x + g[k];
+    if constexpr (L == 0)
+        f[0] = c * F;
+    else
+    {
+        double ex = kExpCoefficient<kExpTerms - 1>;
+        static_for<0, kExpTerms - 1>([&](auto K) { ex = ex * x + kExpCoefficient<kExpTerms - 2 - decltype(K)::value>; });
+        double u[L];
+        u[0] = c * (g[G::kTerms] * ex);
+#pragma unroll
+        for (int k = 1; k < L; ++k) u[k] = u[k - 1] * s;
+        f[L] = (c * power<L>(s)) * F;
+#pragma unroll
+        for (int m = L; m >= 1; --m)
+        {
+            const double t = fma(-R2, f[m], u[m - 1]);
+            f[m - 1]       = m == 1 ? t : t * (1.0 / (2 * m - 1));
+        }
     }
 }
 #endif

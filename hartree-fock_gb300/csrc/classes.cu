@@ -46,10 +46,12 @@ constexpr bool dual_form(bool fp32) { return fp32 && (QC == 11 || QC == 12 || QC
 // Ket-chunked thread form (FP32 d classes): ket components per thread, chosen so that R, G[HAB][CH] and
 // ERI[NAB][CH] stay in registers (HL + (HAB + NAB) * CH floats well below 255); 0 = not compiled.
 //   (dp|pp) (dp|ds): 3   (dp|dp): 2   (dd|ps) (dd|pp) (dd|ds) (dd|dp): 1
+// In FP64 (dp|pp) (dp|ds) (dp|dp): 3   (dd|ps): 1; what does not fit the registers spills to L1, whose traffic (two wavefronts per
+// warp and value) hides behind the FP64 pipe (16 SM cycles per warp instruction).
 constexpr int chunk_width(bool fp32)
 {
     if (!fp32)
-        return 0;
+        return (QC >= 12 && QC <= 14) ? 3 : QC == 16 ? 1 : 0;
     return (QC == 12 || QC == 13) ? 3 : QC == 14 ? 2 : (QC >= 16 && QC <= 19) ? 1 : 0;
 }
 // The form a launch with form 0 runs (before or without autotuning): the chunked form where the tuner
@@ -67,6 +69,22 @@ constexpr unsigned form_mask(bool fp32)
            (chunk_width(fp32) > 0 ? (1u << kFormChunk) : 0u);
 }
 
+// The split of a launch (SplitArgs): eight warps per SM fill it in FP64 (two per scheduler; the FP64 pipe takes a
+// warp instruction every 64 cycles of one).  FP32 lists are not split.
+template <typename Real> SplitArgs split_args(const ClassLaunch& c)
+{
+    SplitArgs s;
+    if (sizeof(Real) == 4)
+        return s;
+    s.lanes     = static_cast<unsigned>(c.num_sms) * 256u;
+    s.prims     = c.prims;
+    s.prims_dev = c.prims_dev;
+    unsigned long long m = c.prims / s.lanes;
+    m = m < 1 ? 1 : m;
+    while (s.smax < 128 && s.smax * m < static_cast<unsigned long long>(c.pmax)) s.smax <<= 1;
+    return s;
+}
+
 // Resident blocks per SM a grid may take: the occupancy limit times the share, at least one.
 inline unsigned long long resident(int per_sm, float share)
 {
@@ -74,15 +92,52 @@ inline unsigned long long resident(int per_sm, float share)
     return static_cast<unsigned long long>(r > 0 ? r : 1);
 }
 
+// Store mode: thread per quartet, or warp per quartet for the classes whose FP64 warp form is compiled.
+template <bool Warp> cudaError_t launch_store(const ClassLaunch& c)
+{
+    size_t smem = sizeof(double) * BoysGrid<double>::kPoints * BoysGrid<double>::kRow;
+    if constexpr (Warp)
+        smem += sizeof(double) * WarpLayout<LA, LB, LC, LD, double>::kPerWarp * kWarpKernelWarps;
+    auto kern = [] {
+        if constexpr (Warp)
+            return jk_class_warp_kernel<LA, LB, LC, LD, double, false>;
+        else
+            return jk_store_kernel<LA, LB, LC, LD>;
+    }();
+    constexpr unsigned threads = Warp ? 32 * kWarpKernelWarps : 128, per_block = Warp ? kWarpKernelWarps : 128;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess)
+        return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, static_cast<int>(threads), smem);
+    if (e != cudaSuccess)
+        return e;
+    const unsigned long long need = (c.count_host + per_block - 1) / per_block;
+    const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1);
+    const unsigned grid           = static_cast<unsigned>(need < cap ? need : cap);
+    const double* slice           = static_cast<const double*>(c.boys_slice);
+    if constexpr (Warp)
+        kern<<<grid, threads, smem, c.stream>>>(c.list, c.count_dev, c.view, slice, c.tables);
+    else
+        kern<<<grid, threads, smem, c.stream>>>(c.list, c.count_dev, c.view, slice);
+    return cudaGetLastError();
+}
+
 template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
 {
     constexpr bool kWarpForm = warp_form(sizeof(Real) == 4);
     if (c.count_host == 0)
         return cudaSuccess;
+    if constexpr (sizeof(Real) == 8 && !UHF)
+        if (c.view.store != nullptr)
+            return launch_store<warp_form(false)>(c);
     const int form = c.form == 0 ? default_form(sizeof(Real) == 4) : c.form;
     if (!((form_mask(sizeof(Real) == 4) >> form) & 1u))
         return cudaErrorInvalidValue;
+    // The thread and chunk forms stage the BoysFast slice in FP64, the others the BoysGrid slice.
     const size_t slice_bytes = sizeof(Real) * BoysGrid<Real>::kPoints * BoysGrid<Real>::kRow;
+    constexpr size_t kFastBytes = sizeof(Real) * boys_slice_size<Real>();
+    const Real* fast = static_cast<const Real*>(sizeof(Real) == 8 ? c.boys_fast : c.boys_slice);
     if constexpr (kGroup)
     {
         if (form == kFormGroup)
@@ -119,7 +174,8 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
                     if (err != cudaSuccess)
                         return;
                     auto kern         = jk_class_chunk_kernel<LA, LB, LC, LD, Real, UHF, k0, k1>;
-                    const size_t smem = slice_bytes;
+                    const SplitArgs sp = split_args<Real>(c);
+                    const size_t smem = kFastBytes + (sp.smax >= 32 ? sizeof(Real) * split_scratch<LA, LB, k0, k1>() : 0);
                     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
                     if (err != cudaSuccess)
                         return;
@@ -127,10 +183,10 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
                     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
                     if (err != cudaSuccess)
                         return;
-                    const unsigned long long need = (c.count_host + 127) / 128;
+                    const unsigned long long need = ((c.count_host + 31) / 32 * sp.smax + 3) / 4;
                     const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share);
                     kern<<<static_cast<unsigned>(need < cap ? need : cap), 128, smem, c.stream>>>(
-                        c.list, c.count_dev, c.view, static_cast<const Real*>(c.boys_slice));
+                        c.list, c.count_dev, c.view, fast, sp);
                     err = cudaGetLastError();
                 });
             return err;
@@ -165,7 +221,8 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
         if (form == kFormThread)
         {
             auto kern           = jk_class_kernel<LA, LB, LC, LD, Real, UHF>;
-            const size_t smem   = slice_bytes;
+            const SplitArgs sp  = split_args<Real>(c);
+            const size_t smem   = kFastBytes + (sp.smax >= 32 ? sizeof(Real) * split_scratch<LA, LB, 0, NCD>() : 0);
             cudaError_t e       = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
             if (e != cudaSuccess)
                 return e;
@@ -173,10 +230,10 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
             if (e != cudaSuccess)
                 return e;
-            const unsigned long long need = (c.count_host + 127) / 128;
+            const unsigned long long need = ((c.count_host + 31) / 32 * sp.smax + 3) / 4;
             const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share);
             const unsigned grid           = static_cast<unsigned>(need < cap ? need : cap);
-            kern<<<grid, 128, smem, c.stream>>>(c.list, c.count_dev, c.view, static_cast<const Real*>(c.boys_slice));
+            kern<<<grid, 128, smem, c.stream>>>(c.list, c.count_dev, c.view, fast, sp);
             return cudaGetLastError();
         }
     }

@@ -149,6 +149,9 @@ struct hfg_engine
     hfg::DevBuf<double> d_ksoa64[hfg::kNumPairClasses];
     hfg::DevBuf<float> d_ksoa32[hfg::kNumPairClasses];
     long long kfs[hfg::kNumPairClasses] {};
+    // ExponentTable (eri_jk.cuh) over the basis's nexp distinct exponents p; nexp = 0: too many, not tabulated.
+    hfg::DevBuf<double2> d_exptab;
+    int nexp = 0;
     // Host records in pack order: pair k's primitives start at record orig_off[k] of h_tab[class].
     std::vector<double> h_tab[hfg::kNumPairClasses];
     std::vector<int> orig_off;
@@ -158,6 +161,7 @@ struct hfg_engine
     double prim_thr = 1e-15;
     std::vector<double> h_qp[hfg::kNumPairClasses];
     std::vector<int> npp_full, keep_off, keep_idx;
+    int cls_npp[hfg::kNumPairClasses] {}; // largest kept count of any pair, per class
     // Unscreened records in pack order (the nuclear gradient's derivative integrals use every primitive).
     hfg::DevBuf<double> d_pptab64_full[hfg::kNumPairClasses];
     hfg::DevBuf<float> d_pptab32_full[hfg::kNumPairClasses];
@@ -169,6 +173,7 @@ struct hfg_engine
     hfg::DevBuf<int> d_shnao;          // per pair: Cartesian counts of sh1, sh2
     hfg::DevBuf<hfg::WarpTables> d_tables;
     hfg::DevBuf<double> d_boys64[hfg::kMaxLt + 2];
+    hfg::DevBuf<double> d_boysf[hfg::kMaxLt + 2]; // BoysFast slices
     hfg::DevBuf<float> d_boys32[hfg::kMaxLt + 2];
     hfg::DevBuf<double> d_gtab[hfg::kNumPairClasses]; // gradient records (built on first use)
     hfg::DevBuf<float> d_gtab32[hfg::kNumPairClasses]; // their FP32 copies (mixed-precision gradient)
@@ -824,18 +829,62 @@ static void screen_primitives(hfg_engine* e)
         e->keep_off[k + 1] = static_cast<int>(e->keep_idx.size());
         e->pairs[k].npp    = e->keep_off[k + 1] - e->keep_off[k];
     }
+    std::fill(std::begin(e->cls_npp), std::end(e->cls_npp), 0);
+    for (size_t k = 0; k < e->pairs.size(); ++k)
+    {
+        const int pc       = e->pair_class_of[k];
+        e->cls_npp[pc]      = std::max(e->cls_npp[pc], e->pairs[k].npp);
+    }
 }
 
 // Builds pairs, primitive-pair tables and sorted class lists skeleton (without Q).
 static void pack_molecules(hfg_engine* e)
 {
     using namespace hfg;
+    // Distinct primitive exponents of all molecules, and the distinct sums of two of them (record field 5).
+    std::vector<double> ex, sums;
+    for (const HostBasis& b : e->basis) ex.insert(ex.end(), b.alpha.begin(), b.alpha.end());
+    auto distinct = [](std::vector<double>& v) {
+        std::sort(v.begin(), v.end());
+        v.erase(std::unique(v.begin(), v.end()), v.end());
+    };
+    distinct(ex);
+    const size_t nex = ex.size();
+    const bool tabulate = nex * (nex + 1) / 2 <= 8 * static_cast<size_t>(kMaxExponents); // more have too many sums
+    std::vector<int> sum_at;
+    if (tabulate)
+    {
+        for (size_t i = 0; i < nex; ++i)
+            for (size_t j = 0; j <= i; ++j) sums.push_back(ex[i] + ex[j]);
+        distinct(sums);
+    }
+    e->nexp = tabulate && sums.size() <= static_cast<size_t>(kMaxExponents) ? static_cast<int>(sums.size()) : 0;
+    if (e->nexp > 0)
+    {
+        sum_at.resize(nex * nex);
+        for (size_t i = 0; i < nex; ++i)
+            for (size_t j = 0; j < nex; ++j)
+                sum_at[i * nex + j] =
+                    static_cast<int>(std::lower_bound(sums.begin(), sums.end(), ex[i] + ex[j]) - sums.begin());
+        std::vector<double2> t(sums.size() * sums.size());
+        for (size_t i = 0; i < sums.size(); ++i)
+            for (size_t j = 0; j < sums.size(); ++j)
+            {
+                const double p = sums[i], q = sums[j];
+                t[i * sums.size() + j] = make_double2(1.0 / std::sqrt(p + q), -2.0 * (p * q) / (p + q));
+            }
+        e->d_exptab.upload(t, e->stream);
+        HFG_CUDA(cudaStreamSynchronize(e->stream));
+    }
     std::vector<std::vector<double>> tab(kNumPairClasses);
     std::vector<int> class_npp(kNumPairClasses, 0);
     for (int m = 0; m < e->nmol; ++m)
     {
         const HostBasis& b = e->basis[m];
         const int ns       = e->mols[m].nshells;
+        std::vector<int> ex_at(e->nexp > 0 ? b.alpha.size() : 0);
+        for (size_t k = 0; k < ex_at.size(); ++k)
+            ex_at[k] = static_cast<int>(std::lower_bound(ex.begin(), ex.end(), b.alpha[k]) - ex.begin());
         for (int s1 = 0; s1 < ns; ++s1)
             for (int s2 = 0; s2 <= s1; ++s2)
             {
@@ -880,7 +929,8 @@ static void pack_molecules(hfg_engine* e)
                         rec[2] = P[1];
                         rec[3] = P[2];
                         rec[4] = std::sqrt(kTwoPi25) * ip * Kw;
-                        rec[5] = ip;
+                        rec[5] = kRoundMagic<double> +
+                                 (e->nexp > 0 ? sum_at[ex_at[b.prim_off[a] + pa] * nex + ex_at[b.prim_off[bb] + pb]] : 0);
                         double E[3][kMaxL + 1][kMaxL + 1][2 * kMaxL + 1];
                         for (int k = 0; k < 3; ++k) hermite_1d(l1, l2, p, PA[k], PB[k], E[k]);
                         int x = kPairHeader;
@@ -953,9 +1003,15 @@ static void pack_molecules(hfg_engine* e)
     for (int L = 0; L <= kMaxLt + 1; ++L)
     {
         e->d_boys64[L].upload(boys_slice_host<double>(L), e->stream);
+        e->d_boysf[L].upload(boys_fast_slice_host(L), e->stream);
         e->d_boys32[L].upload(boys_slice_host<float>(L), e->stream);
     }
     HFG_CUDA(cudaStreamSynchronize(e->stream));
+}
+
+static ExponentTable exponent_table(const hfg_engine* e)
+{
+    return ExponentTable {e->nexp > 0 ? e->d_exptab.p : nullptr, e->nexp};
 }
 
 static FockView base_view(hfg_engine* e, bool fp32)
@@ -970,7 +1026,15 @@ static FockView base_view(hfg_engine* e, bool fp32)
     }
     v.mat_off = e->d_mat_off.p;
     v.mat_ld  = e->d_mat_ld.p;
+    v.et      = exponent_table(e);
     return v;
+}
+
+// Most primitive quartets a quartet of class (P1|P2) has in the Fock build (after the primitive screening).
+static int max_prims(const hfg_engine* e, int P1, int P2)
+{
+    const long long p = static_cast<long long>(e->cls_npp[P1]) * e->cls_npp[P2];
+    return static_cast<int>(std::max(1ll, std::min(p, 1ll << 30)));
 }
 
 static int qclass_of(int pb, int pk) { return quartet_class(std::max(pb, pk), std::min(pb, pk)); }
@@ -1295,6 +1359,8 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
     t.list        = e->d_tune_list.p;
     t.count_dev   = e->d_tune_cnt.p;
     t.count_host  = m;
+    t.prims       = static_cast<unsigned long long>(static_cast<double>(base.prims) * (static_cast<double>(m) / static_cast<double>(n)));
+    t.prims_dev   = nullptr;
     t.view.X      = e->d_tune_acc[0].p;
     t.view.Ya     = e->d_tune_acc[1].p;
     t.view.Yb     = e->d_tune_acc[2].p;
@@ -1415,11 +1481,16 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
         cudaStream_t ps = (overlap && prec == 1) ? e->stream2 : s;
         if (!graph && !(persist && prec == 0))
             HFG_CUDA(cudaEventRecord(overlap && prec == 1 ? e->ev2[2] : e->ev[3 + prec], ps));
+        const unsigned long long* h_prims = e->h_counts.size() >= static_cast<size_t>(4 * kNumQuartetClasses)
+                                                ? e->h_counts.data() + 2 * kNumQuartetClasses : nullptr;
         for (int qc = kNumQuartetClasses - 1; qc >= 0; --qc)
         {
             const unsigned long long n = graph ? e->cap[qc] : e->h_counts[2 * qc + prec];
             if (n == 0 || in_queue(qc))
                 continue;
+            // In a graph the counts are those of the eager build before the capture: the kernels read the replay's
+            // own on the device, these only size the grids.
+            const unsigned long long prims = h_prims ? h_prims[2 * qc + prec] : n;
             const int P1 = [&] { int p = 0; while ((p + 1) * (p + 2) / 2 <= qc) ++p; return p; }();
             const int P2 = qc - P1 * (P1 + 1) / 2;
             const int L  = pair_class_l1(P1) + pair_class_l2(P1) + pair_class_l1(P2) + pair_class_l2(P2);
@@ -1438,12 +1509,16 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             c.view.ao_thr = r.schwartz_threshold;
             c.view.ao_thr_f = static_cast<float>(r.schwartz_threshold);
             c.boys_slice = prec == 1 ? static_cast<const void*>(e->d_boys32[L].p) : e->d_boys64[L].p;
+            c.boys_fast  = e->d_boysf[L].p;
             c.tables     = e->d_tables.p;
             c.fp32       = prec == 1;
             c.uhf        = uhf;
             c.stream     = ps;
             c.num_sms    = e->num_sms;
             c.share      = overlap ? (prec == 1 ? e->overlap_share32 : e->overlap_share) : 1.f;
+            c.pmax       = max_prims(e, P1, P2);
+            c.prims_dev  = e->d_counts.p + 2 * kNumQuartetClasses + 2 * qc + prec;
+            c.prims      = prims;
             if (graph)
             {
                 const int set  = e->form_set[qc][prec];

@@ -19,12 +19,19 @@ struct ClassLaunch
     unsigned long long count_host;
     FockView view;
     const void* boys_slice; // slice of the class's total L, Real of the precision
+    const void* boys_fast;  // FP64: its BoysFast slice (not used in store mode)
     const WarpTables* tables;
     bool fp32;
     bool uhf;
     cudaStream_t stream;
     int num_sms;
     int form; // 0: the class's default form, else one of kFormThread / kFormWarp / kFormGroup / kFormChunk
+    // For the split of short lists' primitive quartets over lanes (SplitArgs in eri_jk.cuh): the list's primitive
+    // quartets (an estimate where the list is not known yet), where the device keeps the exact number (may
+    // be null), and the most primitive quartets one quartet of the class can have.
+    unsigned long long prims = 0;
+    const unsigned long long* prims_dev = nullptr;
+    int pmax = 1;
     float share = 1.f; // fraction of the resident blocks per SM the grid may take (concurrent precisions)
 };
 // Kernel forms of a class kernel (eri_jk.cuh, eri_warp.cuh, eri_group.cuh).

@@ -33,6 +33,17 @@ namespace hfg
 {
 constexpr double kTwoPi25 = 34.98683665524972497; // 2 pi^{5/2}
 
+// 1/sqrt(p+q) and -2 pq/(p+q) for every two primitive-pair exponents of the basis: they depend on the
+// exponents alone, of which a molecule's pairs have few distinct ones (136 for water in 6-31G**), and cost ten
+// FP64 instructions per primitive quartet to compute against one 16-byte load.  Null where the basis has
+// more than kMaxExponents of them; the kernels compute the two numbers then.
+constexpr int kMaxExponents = 1024;
+struct ExponentTable
+{
+    const double2* t; // [n][n]
+    int n;
+};
+
 // Device view of everything a class kernel needs.
 struct FockView
 {
@@ -53,6 +64,7 @@ struct FockView
     double ao_thr;                      // AO-level skip threshold (SCHWARTZ_THRESH)
     float ao_thr_f;                     // the same threshold for the FP32 kernels
     double* store;                      // if set: write the quartets' integrals here instead of digesting
+    ExponentTable et;
 };
 
 __device__ constexpr double ang_norm(int l, int c)
@@ -136,14 +148,72 @@ template <typename Real, bool SoA> struct RecRef
     }
 };
 
+// The scalar part of one primitive quartet: P - Q and Fs[n] = pref (-2 rho)^n F_n, n = 0..L.  Fast (FP64
+// only): from a BoysFast slice and the exponent table; else from a BoysGrid<Real> slice.
+template <int L, typename Real, bool Fast, typename Bra, typename Ket>
+__device__ __forceinline__ void prim_scalars(const Bra& rb, const Ket& rk, const ExponentTable& et,
+                                             const Real* __restrict__ slice, Real& X, Real& Y, Real& Z, Real* Fs)
+{
+    if constexpr (Fast)
+    {
+        X = rb[1] - rk[1];
+        Y = rb[2] - rk[2];
+        Z = rb[3] - rk[3];
+        double rs, s;
+        if (et.t != nullptr)
+        {
+            const double2 v = __ldg(et.t + (__double2loint(rb[5]) * et.n + __double2loint(rk[5])));
+            rs              = v.x;
+            s               = v.y;
+        }
+        else
+        {
+            rs = rsqrt(rb[0] + rk[0]);
+            s  = (-2.0 * (rb[0] * rk[0])) * (rs * rs);
+        }
+        scaled_boys<L>((rb[4] * rk[4]) * rs, s, X * X + Y * Y + Z * Z, slice, Fs);
+    }
+    else
+    {
+        const Real p = rb[0], q = rk[0];
+        X = rb[1] - rk[1];
+        Y = rb[2] - rk[2];
+        Z = rb[3] - rk[3];
+        const Real rs   = hfg_rsqrt(p + q);
+        const Real rho  = (p * q) * (rs * rs);
+        const Real pref = (rb[4] * rk[4]) * rs;
+        const Real T    = rho * (X * X + Y * Y + Z * Z);
+        Real F[L + 1];
+        boys_eval<L, Real>(T, slice, F);
+        const Real m2r = Real(-2) * rho;
+        Real w         = pref;
+#pragma unroll
+        for (int n = 0; n <= L; ++n)
+        {
+            Fs[n] = w * F[n];
+            w *= m2r;
+        }
+    }
+}
+
+// The primitive quartets one lane of a group evaluates: bra primitives ib0, ib0 + ibs, ... and, for each,
+// ket primitives ik0, ik0 + iks, ... (all of them by default).
+struct PrimRange
+{
+    int ib0 = 0, ibs = 1, ik0 = 0, iks = 1;
+};
+
 // Contracted Cartesian integrals of one quartet (without the angular normalisation factors), for the ket
 // components kl in [KL0, KL1) (all of them by default): acc[ij * (KL1 - KL0) + kl - KL0].  KSoA: the ket
-// table tk is field-major with field stride kfs.
+// table tk is field-major with field stride kfs.  Fast (FP64, bound by the FP64 pipe): the scalars of
+// scaled_boys, and every Hermite term is one DFMA straight into its accumulator; a local sum added
+// afterwards costs HAB * NCD more FP64 instructions per primitive quartet.
 template <int LA, int LB, int LC, int LD, typename Real, bool KSoA = false, int KL0 = 0,
-          int KL1 = ncart(LC) * ncart(LD)>
+          int KL1 = ncart(LC) * ncart(LD), bool Fast = false>
 __device__ __forceinline__ void eval_quartet(const PairRec& bra, const PairRec& ket, const Real* __restrict__ tb,
                                              const Real* __restrict__ tk, const Real* __restrict__ slice,
-                                             Real* acc, long long kfs = 0)
+                                             Real* acc, long long kfs = 0, const ExponentTable et = ExponentTable {},
+                                             const PrimRange pr = PrimRange {})
 {
     constexpr int LAB = LA + LB, LCD = LC + LD, L = LAB + LCD;
     constexpr int NAB = ncart(LA) * ncart(LB), NCD = KL1 - KL0;
@@ -152,38 +222,20 @@ __device__ __forceinline__ void eval_quartet(const PairRec& bra, const PairRec& 
 #pragma unroll
     for (int x = 0; x < NAB * NCD; ++x) acc[x] = Real(0);
 
-    for (int ib = 0; ib < bra.npp; ++ib)
+    for (int ib = pr.ib0; ib < bra.npp; ib += pr.ibs)
     {
         const Real* __restrict__ rb = tb + static_cast<size_t>(bra.pp_off + ib) * SB;
-        const Real p = rb[0], Px = rb[1], Py = rb[2], Pz = rb[3], Wab = rb[4];
         Real G[HAB * NCD];
 #pragma unroll
         for (int x = 0; x < HAB * NCD; ++x) G[x] = Real(0);
 
-        for (int ik = 0; ik < ket.npp; ++ik)
+        for (int ik = pr.ik0; ik < ket.npp; ik += pr.iks)
         {
             const RecRef<Real, KSoA> rk {KSoA ? tk + (ket.kslot + static_cast<long long>(ik) * ket.kstep)
                                               : tk + static_cast<size_t>(ket.pp_off + ik) * SK,
                                          kfs};
-            const Real q = rk[0];
-            const Real X = Px - rk[1], Y = Py - rk[2], Z = Pz - rk[3];
-            const Real rs   = hfg_rsqrt(p + q);
-            const Real rho  = (p * q) * (rs * rs);
-            const Real pref = (Wab * rk[4]) * rs;
-            const Real T    = rho * (X * X + Y * Y + Z * Z);
-            Real F[L + 1];
-            boys_eval<L, Real>(T, slice, F);
-            Real Fs[L + 1];
-            {
-                const Real m2r = Real(-2) * rho;
-                Real w         = pref;
-#pragma unroll
-                for (int n = 0; n <= L; ++n)
-                {
-                    Fs[n] = w * F[n];
-                    w *= m2r;
-                }
-            }
+            Real X, Y, Z, Fs[L + 1];
+            prim_scalars<L, Real, Fast>(rb, rk, et, slice, X, Y, Z, Fs);
             Real R[HL];
             hermite_R<L, Real>(Fs, X, Y, Z, R);
 
@@ -198,7 +250,7 @@ __device__ __forceinline__ void eval_quartet(const PairRec& bra, const PairRec& 
                         {
                             constexpr int h = decltype(TUV)::value;
                             constexpr int t = htuv(h, LAB, 0), u = htuv(h, LAB, 1), v = htuv(h, LAB, 2);
-                            Real s          = Real(0);
+                            Real s          = Fast ? G[h * NCD + (kl - KL0)] : Real(0);
                             static_for<0, lx * ly * lz>(
                                 [&](auto EE)
                                 {
@@ -211,7 +263,10 @@ __device__ __forceinline__ void eval_quartet(const PairRec& bra, const PairRec& 
                                     else
                                         s += term;
                                 });
-                            G[h * NCD + (kl - KL0)] += s;
+                            if constexpr (Fast)
+                                G[h * NCD + (kl - KL0)] = s;
+                            else
+                                G[h * NCD + (kl - KL0)] += s;
                         });
                 });
         }
@@ -225,7 +280,7 @@ __device__ __forceinline__ void eval_quartet(const PairRec& bra, const PairRec& 
 #pragma unroll
                 for (int kl = 0; kl < NCD; ++kl)
                 {
-                    Real s = Real(0);
+                    Real s = Fast ? acc[ij * NCD + kl] : Real(0);
                     static_for<0, lx * ly * lz>(
                         [&](auto EE)
                         {
@@ -234,26 +289,14 @@ __device__ __forceinline__ void eval_quartet(const PairRec& bra, const PairRec& 
                             const Real gg = G[hidx(t, u, v, LAB) * NCD + kl];
                             s += (LA + LB == 0) ? gg : rb[eoff + e] * gg;
                         });
-                    acc[ij * NCD + kl] += s;
+                    if constexpr (Fast)
+                        acc[ij * NCD + kl] = s;
+                    else
+                        acc[ij * NCD + kl] += s;
                 }
             });
     }
 }
-
-// Widening to double for the FP64 accumulators without the FP64 pipe (GB300 runs float -> double
-// conversions there, at 1/64 of the FP32 rate): the IEEE-754 fields are moved with integer operations.
-// Exact for normal numbers and zero; float subnormals (< 1.2e-38) become zero; infinities and NaNs keep
-// their class.
-__device__ __forceinline__ double widen(float x)
-{
-    const unsigned u                 = __float_as_uint(x);
-    const unsigned e                 = (u >> 23) & 0xffu;
-    const unsigned long long sign    = static_cast<unsigned long long>(u & 0x80000000u) << 32;
-    const unsigned long long de      = e == 0xffu ? 0x7ffull : static_cast<unsigned long long>(e + 896u);
-    const unsigned long long normal  = sign | (de << 52) | (static_cast<unsigned long long>(u & 0x7fffffu) << 29);
-    return __longlong_as_double(static_cast<long long>(e == 0u ? sign : normal));
-}
-__device__ __forceinline__ double widen(double x) { return x; }
 
 template <typename Real> __device__ __forceinline__ Real ao_threshold(const FockView& v)
 {
@@ -490,73 +533,294 @@ __device__ __forceinline__ void digest_quartet(const PairRec& bra, const PairRec
     digest_loaded<LA, LB, LC, LD, Real, UHF>(bra, ket, same_pair, acc, v, d, true, false);
 }
 
-// Stage this class's Boys slice in shared memory.
-template <typename Real> __device__ __forceinline__ void stage_boys(const Real* __restrict__ g, Real* s)
+// Values of the Boys slice the thread, chunk and gradient kernels stage: BoysFast in FP64.
+template <typename Real> __host__ __device__ constexpr int boys_slice_size()
 {
-    constexpr int n = BoysGrid<Real>::kPoints * BoysGrid<Real>::kRow;
+    return sizeof(Real) == 8 ? BoysFast::kPoints * BoysFast::kRow : BoysGrid<Real>::kPoints * BoysGrid<Real>::kRow;
+}
+
+// Stage this class's Boys slice in shared memory.
+template <typename Real, int n = BoysGrid<Real>::kPoints * BoysGrid<Real>::kRow>
+__device__ __forceinline__ void stage_boys(const Real* __restrict__ g, Real* s)
+{
     for (int i = threadIdx.x; i < n; i += blockDim.x) s[i] = g[i];
     __syncthreads();
 }
 
-// One launch processes the whole surviving list of one class; the list length is read on the device
-// (written by the list builder), so a build needs no host round trip between kernels.
-template <int LA, int LB, int LC, int LD, typename Real, bool UHF>
-__global__ void __launch_bounds__(128) jk_class_kernel(const Quartet* __restrict__ list,
-                                                       const unsigned long long* __restrict__ count, FockView v,
-                                                       const Real* __restrict__ boys_slice)
+// How a launch splits its quartets' primitive quartets over lanes.  A quartet's primitive quartets are one
+// dependent FP64 chain per thread, and the contracted shells have hundreds to thousands of them ((8 8|8 8)
+// primitives in cc-pVDZ): a list too short to fill the GPU then takes as long as its longest quartet.  So
+// a window of 32 list entries is worked on by G warps, G a power of two up to `smax` (1 to 128): every
+// quartet gets G lanes, each with a strided share of the bra and ket primitives, and the lanes' integrals
+// are summed before one of them digests.  G grows with the window's primitive count P until each lane
+// has at most m = max(1, prims / lanes) primitive quartets, `prims` being the whole list's primitive
+// quartets and `lanes` what fills the GPU: a long list (m above any P) runs one lane per quartet, as
+// before, and pays nothing.
+struct SplitArgs
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Real* slice                = reinterpret_cast<Real*>(smem_raw);
-    const unsigned long long n = *count;
-    if (static_cast<unsigned long long>(blockIdx.x) * blockDim.x >= n)
-        return;
-    stage_boys<Real>(boys_slice, slice);
-    constexpr int N = ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD);
+    int smax = 1;                             // warps per window at most, a power of two; 1: no split
+    unsigned lanes = 1;                       // lanes that fill the GPU
+    unsigned long long prims = 0;             // the list's primitive quartets,
+    const unsigned long long* prims_dev = nullptr; // or where they stand (a captured graph's lists)
+};
+
+// Lanes per quartet for P primitive quartets at m a lane.
+__device__ __forceinline__ int split_lanes(int P, unsigned long long m, int smax)
+{
+    int g = 1;
+    while (g < smax && static_cast<unsigned long long>(g) * m < static_cast<unsigned long long>(P)) g <<= 1;
+    return g;
+}
+
+// Share of lane r of g: the g lanes as a gb x gk grid over the bra and ket primitives, powers of two with
+// the fewest rounds.
+__device__ __forceinline__ PrimRange split_range(int npb, int npk, int r, int g)
+{
+    int best = 1 << 30, bk = 1;
+    for (int gk = 1; gk <= g; gk <<= 1)
+    {
+        const int gb = g / gk, rounds = ((npb + gb - 1) / gb) * ((npk + gk - 1) / gk);
+        if (rounds < best)
+        {
+            best = rounds;
+            bk   = gk;
+        }
+    }
+    return PrimRange {r / bk, g / bk, r % bk, bk};
+}
+
+// Digestion of one quartet by a whole warp: w[ij * (KL1 - KL0) + kl - KL0] in shared memory holds the
+// contracted integrals with their angular factors; each lane owns output elements of J and K.  (One lane
+// digesting for the warp would run NAB * NCD * 6 dependent FP64 instructions on its own.)
+template <int LA, int LB, int LC, int LD, typename Real, bool UHF, int KL0, int KL1>
+__device__ __forceinline__ void digest_shared(const PairRec& bra, const PairRec& ket, bool same_pair, Real* w,
+                                              const FockView& v)
+{
+    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
+    constexpr int NAB = NA * NB, CH = KL1 - KL0;
+    const int lane = threadIdx.x & 31;
+    const long long off = v.mat_off[bra.mol];
+    const int n         = v.mat_ld[bra.mol];
+    const int a0 = bra.ao1, b0 = bra.ao2, c0 = ket.ao1, d0 = ket.ao2;
+    auto at = [&](int r, int c) -> long long { return off + r + static_cast<long long>(c) * n; };
+    const Real s   = (bra.same ? Real(0.5) : Real(1)) * (ket.same ? Real(0.5) : Real(1)) * (same_pair ? Real(0.5) : Real(1));
+    const Real thr = ao_threshold<Real>(v);
+    for (int x = lane; x < NAB * CH; x += 32) w[x] = (fabs(w[x]) < thr) ? Real(0) : s * w[x];
+    __syncwarp();
+    constexpr int nJ = NAB + CH, nK = (NA + NB) * (NC + ND), nspin = UHF ? 2 : 1;
+    for (int o = lane; o < nJ + nspin * nK; o += 32)
+    {
+        Real sum = Real(0);
+        if (o < NAB)
+        {
+            for (int x = 0; x < CH; ++x) sum += w[o * CH + x] * ldD<Real>(v.Dt, at(c0 + (KL0 + x) / ND, d0 + (KL0 + x) % ND));
+            atomicAdd(v.X + at(a0 + o / NB, b0 + o % NB), widen(Real(2) * sum));
+        }
+        else if (o < nJ)
+        {
+            const int x = o - NAB;
+            for (int ij = 0; ij < NAB; ++ij) sum += w[ij * CH + x] * ldD<Real>(v.Dt, at(a0 + ij / NB, b0 + ij % NB));
+            atomicAdd(v.X + at(c0 + (KL0 + x) / ND, d0 + (KL0 + x) % ND), widen(Real(2) * sum));
+        }
+        else
+        {
+            // K(row AO of a or b, column AO of c or d), contracted with D(the other bra AO, the other ket AO).
+            const int k = (o - nJ) % nK, spin = (o - nJ) / nK;
+            const int row = k / (NC + ND), col = k % (NC + ND);
+            const bool ra = row < NA, cc = col < NC;
+            const int i0 = ra ? row : row - NA, k0 = cc ? col : col - NC;
+            const void* Ds = spin == 0 ? v.Da : v.Db;
+            for (int x = 0; x < CH; ++x)
+            {
+                const int kk = (KL0 + x) / ND, ll = (KL0 + x) % ND;
+                if ((cc ? kk : ll) != k0)
+                    continue;
+                const int dcol = cc ? d0 + ll : c0 + kk;
+                if (ra)
+                    for (int j = 0; j < NB; ++j) sum += w[(i0 * NB + j) * CH + x] * ldD<Real>(Ds, at(b0 + j, dcol));
+                else
+                    for (int i = 0; i < NA; ++i) sum += w[(i * NB + i0) * CH + x] * ldD<Real>(Ds, at(a0 + i, dcol));
+            }
+            bool reached = false;
+            for (int x = 0; x < CH; ++x) reached = reached || (cc ? (KL0 + x) / ND : (KL0 + x) % ND) == k0;
+            if (reached)
+                atomicAdd((spin == 0 ? v.Ya : v.Yb) + at((ra ? a0 : b0) + i0, (cc ? c0 : d0) + k0), widen(sum));
+        }
+    }
+    __syncwarp(); // the next quartet reuses w
+}
+
+// Values of the block's shared scratch of a split launch (per warp one quartet's integrals).
+template <int LA, int LB, int KL0, int KL1> __host__ __device__ constexpr int split_scratch()
+{
+    return 4 * ncart(LA) * ncart(LB) * (KL1 - KL0);
+}
+
+// The quartets of one list for the ket components [KL0, KL1): thread per quartet, or G lanes per quartet
+// (SplitArgs).  `scratch`: split_scratch() values of shared memory, used by split launches only.
+template <int LA, int LB, int LC, int LD, typename Real, bool UHF, int KL0, int KL1>
+__device__ __forceinline__ void class_body(const Quartet* __restrict__ list, unsigned long long n, const FockView& v,
+                                           const Real* __restrict__ slice, Real* scratch, const SplitArgs& sp)
+{
+    constexpr int NB = ncart(LB), ND = ncart(LD);
+    constexpr int NAB = ncart(LA) * NB, NCD = ncart(LC) * ND, CH = KL1 - KL0, N = NAB * CH;
     const Real* tb      = static_cast<const Real*>(v.pptab[pair_class(LA, LB)]);
     const Real* tk      = static_cast<const Real*>(v.ksoa[pair_class(LC, LD)]);
     const long long kfs = v.kfs[pair_class(LC, LD)];
-    using DD   = DigestD<LA, LB, LC, LD, Real, UHF>;
-    const int lane = threadIdx.x & 31;
-    // Warp-uniform iteration (every lane runs the same trip count, inactive lanes past the end), so that
-    // the digestion may sum the bra block over the warp.
-    for (unsigned long long base = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u);
-         base < n; base += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
+    using DD            = DigestD<LA, LB, LC, LD, Real, UHF>;
+    constexpr bool kEarly = DD::kEarly && CH == NCD;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    // FP32 lists are never split: their chains are short, and their integrals keep one order of summation.
+    constexpr bool kFP64 = sizeof(Real) == 8, kSplit = kFP64;
+    const int S          = kSplit ? sp.smax : 1;
+    const unsigned long long items = ((n + 31) >> 5) * static_cast<unsigned long long>(S);
+    unsigned long long m = 0;
+    if (kSplit && S > 1)
     {
-        const unsigned long long q = base + lane;
-        const bool active          = q < n;
-        const Quartet qt           = list[active ? q : base];
-        const PairRec bra          = v.pairs[qt.bra];
-        const PairRec ket          = v.pairs[qt.ket];
+        m = (sp.prims_dev ? *sp.prims_dev : sp.prims) / sp.lanes;
+        m = m < 1 ? 1 : m;
+    }
+    // Warp-uniform iteration (every lane runs the same trip count, inactive lanes past the end), so that
+    // the digestion may sum the bra block over the warp.  With S >= 4 the four warps of a block are slices of
+    // one window, so that they may share a quartet (G = 64, 128): their branches on G are block-uniform.
+    for (unsigned long long it = static_cast<unsigned long long>(blockIdx.x) * 4 + wib; it < items;
+         it += static_cast<unsigned long long>(gridDim.x) * 4)
+    {
+        unsigned long long base = it * 32, q = base + lane;
+        int g = 1, r = 0;
+        PrimRange pr;
+        if (kSplit && S > 1)
+        {
+            const int ls    = __ffs(S) - 1;
+            base            = (it >> ls) * 32;
+            const int slc   = static_cast<int>(it) & (S - 1);
+            q               = base + lane;
+            const Quartet w = list[q < n ? q : base];
+            g = split_lanes(__reduce_max_sync(0xffffffffu, v.pairs[w.bra].npp * v.pairs[w.ket].npp), m, S);
+            if (slc >= g)
+                continue;
+            q = base + (g <= 32 ? slc * (32 / g) + lane / g : slc / (g / 32));
+            r = g <= 32 ? lane % g : (slc % (g / 32)) * 32 + lane;
+        }
+        const bool active = q < n;
+        const Quartet qt  = list[active ? q : base];
+        const PairRec bra = v.pairs[qt.bra];
+        const PairRec ket = v.pairs[qt.ket];
+        if (g > 1)
+            pr = split_range(bra.npp, ket.npp, r, g);
         DD d;
-        if (v.store == nullptr && DD::kEarly)
+        if (kEarly)
             load_digest_d<LA, LB, LC, LD, Real, UHF>(bra, ket, v, d);
         Real acc[N];
         if (active)
-            eval_quartet<LA, LB, LC, LD, Real, true>(bra, ket, tb, tk, slice, acc, kfs);
+            eval_quartet<LA, LB, LC, LD, Real, true, KL0, KL1, kFP64>(bra, ket, tb, tk, slice, acc, kfs, v.et, pr);
         else
         {
 #pragma unroll
             for (int x = 0; x < N; ++x) acc[x] = Real(0);
         }
-        if (v.store != nullptr)
+        bool leader = active;
+        if (kSplit && g > 1)
         {
-            if (active)
-                static_for<0, N>(
-                    [&](auto E)
-                    {
-                        constexpr int e  = decltype(E)::value;
-                        constexpr int NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
-                        constexpr double an = ang_norm(LA, e / NCD / NB) * ang_norm(LB, (e / NCD) % NB)
-                                            * ang_norm(LC, (e % NCD) / ND) * ang_norm(LD, e % ND);
-                        v.store[q * N + e] = double(acc[e]) * an;
-                    });
-            continue;
+            for (int o = min(g, 32) >> 1; o > 0; o >>= 1)
+#pragma unroll
+                for (int x = 0; x < N; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
+            if (g >= 32)
+            {
+                // One quartet per warp or group of warps: its integrals through shared memory.
+                Real* w = scratch + wib * N;
+                if (lane == 0)
+                    static_for<0, N>(
+                        [&](auto E)
+                        {
+                            constexpr int e = decltype(E)::value;
+                            constexpr Real an = Real(ang_norm(LA, e / CH / NB) * ang_norm(LB, (e / CH) % NB) *
+                                                     ang_norm(LC, (KL0 + e % CH) / ND) * ang_norm(LD, (KL0 + e % CH) % ND));
+                            w[e] = acc[e] * an;
+                        });
+                const int nw = g / 32;
+                if (nw > 1)
+                    __syncthreads();
+                else
+                    __syncwarp();
+                if (wib % nw == 0 && active)
+                {
+                    for (int k = 1; k < nw; ++k)
+                        for (int x = lane; x < N; x += 32) w[x] += w[k * N + x];
+                    __syncwarp();
+                    digest_shared<LA, LB, LC, LD, Real, UHF, KL0, KL1>(bra, ket, qt.bra == qt.ket, w, v);
+                }
+                if (nw > 1)
+                    __syncthreads(); // the leading warp has read the others' integrals
+                continue;
+            }
+            leader = active && r == 0;
+            if (!leader)
+            {
+#pragma unroll
+                for (int x = 0; x < N; ++x) acc[x] = Real(0);
+            }
         }
-        if (!DD::kEarly)
-            load_digest_d<LA, LB, LC, LD, Real, UHF>(bra, ket, v, d);
+        if (!kEarly)
+            load_digest_d<LA, LB, LC, LD, Real, UHF>(bra, ket, v, d); // values the chunk does not read are never loaded
         const unsigned bra0 = __shfl_sync(0xffffffffu, qt.bra, 0);
         const bool bra_warp = __all_sync(0xffffffffu, qt.bra == bra0);
-        digest_loaded<LA, LB, LC, LD, Real, UHF>(bra, ket, qt.bra == qt.ket, acc, v, d, active, bra_warp);
+        digest_loaded<LA, LB, LC, LD, Real, UHF, KL0, KL1>(bra, ket, qt.bra == qt.ket, acc, v, d, leader, bra_warp);
+    }
+}
+
+// Thread form: one launch processes the whole surviving list of one class; the list length is read on
+// the device (written by the list builder), so a build needs no host round trip between kernels.
+template <int LA, int LB, int LC, int LD, typename Real, bool UHF>
+__global__ void __launch_bounds__(128) jk_class_kernel(const Quartet* __restrict__ list,
+                                                       const unsigned long long* __restrict__ count, FockView v,
+                                                       const Real* __restrict__ boys_slice, SplitArgs sp)
+{
+    constexpr int NCD = ncart(LC) * ncart(LD);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Real* slice                = reinterpret_cast<Real*>(smem_raw);
+    const unsigned long long n = *count;
+    if (static_cast<unsigned long long>(blockIdx.x) * 4 >= ((n + 31) >> 5) * static_cast<unsigned long long>(sp.smax))
+        return;
+    stage_boys<Real, boys_slice_size<Real>()>(boys_slice, slice);
+    class_body<LA, LB, LC, LD, Real, UHF, 0, NCD>(list, n, v, slice, slice + boys_slice_size<Real>(), sp);
+}
+
+// Store mode of the thread classes: one thread per quartet writes its contracted integrals (the Schwartz
+// bounds, stored integrals and single blocks).  It stays on the BoysGrid slice and one lane per quartet: the
+// kets of a list are sorted by Q, copies of one molecule have Q equal up to the last bits, and which of
+// them share a warp decides the rounding of the FP32 sums of a mixed build; the Q of one basis and
+// geometry is therefore kept bit for bit.
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(128) jk_store_kernel(const Quartet* __restrict__ list,
+                                                       const unsigned long long* __restrict__ count, FockView v,
+                                                       const double* __restrict__ boys_slice)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* slice              = reinterpret_cast<double*>(smem_raw);
+    const unsigned long long n = *count;
+    if (static_cast<unsigned long long>(blockIdx.x) * blockDim.x >= n)
+        return;
+    stage_boys<double>(boys_slice, slice);
+    constexpr int N = ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD);
+    const double* tb = static_cast<const double*>(v.pptab[pair_class(LA, LB)]);
+    const double* tk = static_cast<const double*>(v.ksoa[pair_class(LC, LD)]);
+    for (unsigned long long q = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; q < n;
+         q += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
+    {
+        const Quartet qt = list[q];
+        double acc[N];
+        eval_quartet<LA, LB, LC, LD, double, true>(v.pairs[qt.bra], v.pairs[qt.ket], tb, tk, slice, acc,
+                                                   v.kfs[pair_class(LC, LD)]);
+        static_for<0, N>(
+            [&](auto E)
+            {
+                constexpr int e  = decltype(E)::value;
+                constexpr int NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
+                constexpr double an = ang_norm(LA, e / NCD / NB) * ang_norm(LB, (e / NCD) % NB)
+                                    * ang_norm(LC, (e % NCD) / ND) * ang_norm(LD, e % ND);
+                v.store[q * N + e] = acc[e] * an;
+            });
     }
 }
 
@@ -568,61 +832,8 @@ __global__ void __launch_bounds__(128) jk_class_kernel(const Quartet* __restrict
 // is its own launch over the whole list (jk_class_chunk_kernel<..., KL0, KL1>), so that every SM runs one
 // chunk's unrolled code at a time: with the chunks of a quartet in neighbouring blocks of one launch the
 // resident blocks of an SM ran different chunk bodies and stalled on instruction fetch (ncu: 30 cycles
-// per issued instruction).  Each chunk recomputes the Boys values and R of its quartet: for FP32, where
-// these are cheap next to the two Hermite transforms, that buys full lanes and no shared-memory round
-// trips; the list and the records are re-read per chunk from L2.
-template <int LA, int LB, int LC, int LD, typename Real, bool UHF, int KL0, int KL1>
-__device__ __forceinline__ void chunk_body(const Quartet* __restrict__ list, unsigned long long n, const FockView& v,
-                                           const Real* __restrict__ slice, unsigned qb, unsigned nqb)
-{
-    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    constexpr int NAB = NA * NB, NCD = NC * ND, CH = KL1 - KL0;
-    const Real* tb      = static_cast<const Real*>(v.pptab[pair_class(LA, LB)]);
-    const Real* tk      = static_cast<const Real*>(v.ksoa[pair_class(LC, LD)]);
-    const long long kfs = v.kfs[pair_class(LC, LD)];
-    using DD       = DigestD<LA, LB, LC, LD, Real, UHF>;
-    const int lane = threadIdx.x & 31;
-    for (unsigned long long base = static_cast<unsigned long long>(qb) * blockDim.x + (threadIdx.x & ~31u); base < n;
-         base += static_cast<unsigned long long>(nqb) * blockDim.x)
-    {
-        const unsigned long long q = base + lane;
-        const bool active          = q < n;
-        const Quartet qt           = list[active ? q : base];
-        const PairRec bra          = v.pairs[qt.bra];
-        const PairRec ket          = v.pairs[qt.ket];
-        Real acc[NAB * CH];
-        if (active)
-            eval_quartet<LA, LB, LC, LD, Real, true, KL0, KL1>(bra, ket, tb, tk, slice, acc, kfs);
-        else
-        {
-#pragma unroll
-            for (int x = 0; x < NAB * CH; ++x) acc[x] = Real(0);
-        }
-        if (v.store != nullptr)
-        {
-            if (active)
-                static_for<0, NAB>(
-                    [&](auto IJ)
-                    {
-                        constexpr int ij = decltype(IJ)::value;
-                        static_for<KL0, KL1>(
-                            [&](auto KLx)
-                            {
-                                constexpr int kl = decltype(KLx)::value;
-                                constexpr double an = ang_norm(LA, ij / NB) * ang_norm(LB, ij % NB) *
-                                                      ang_norm(LC, kl / ND) * ang_norm(LD, kl % ND);
-                                v.store[q * (NAB * NCD) + ij * NCD + kl] = double(acc[ij * CH + (kl - KL0)]) * an;
-                            });
-                    });
-            continue;
-        }
-        DD d;
-        load_digest_d<LA, LB, LC, LD, Real, UHF>(bra, ket, v, d); // values the chunk does not read are never loaded
-        const unsigned bra0 = __shfl_sync(0xffffffffu, qt.bra, 0);
-        const bool bra_warp = __all_sync(0xffffffffu, qt.bra == bra0);
-        digest_loaded<LA, LB, LC, LD, Real, UHF, KL0, KL1>(bra, ket, qt.bra == qt.ket, acc, v, d, active, bra_warp);
-    }
-}
+// per issued instruction).  Each chunk recomputes the Boys values and R of its quartet, which buys full
+// lanes and no shared-memory round trips; the list and the records are re-read per chunk from L2.
 
 // Chunks of CH ket components of a (LC LD) ket.
 template <int LC, int LD, int CH> __host__ __device__ constexpr int num_chunks()
@@ -634,15 +845,15 @@ template <int LC, int LD, int CH> __host__ __device__ constexpr int num_chunks()
 template <int LA, int LB, int LC, int LD, typename Real, bool UHF, int KL0, int KL1>
 __global__ void __launch_bounds__(128) jk_class_chunk_kernel(const Quartet* __restrict__ list,
                                                              const unsigned long long* __restrict__ count, FockView v,
-                                                             const Real* __restrict__ boys_slice)
+                                                             const Real* __restrict__ boys_slice, SplitArgs sp)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Real* slice                = reinterpret_cast<Real*>(smem_raw);
     const unsigned long long n = *count;
-    if (static_cast<unsigned long long>(blockIdx.x) * blockDim.x >= n)
+    if (static_cast<unsigned long long>(blockIdx.x) * 4 >= ((n + 31) >> 5) * static_cast<unsigned long long>(sp.smax))
         return;
-    stage_boys<Real>(boys_slice, slice);
-    chunk_body<LA, LB, LC, LD, Real, UHF, KL0, KL1>(list, n, v, slice, blockIdx.x, gridDim.x);
+    stage_boys<Real, boys_slice_size<Real>()>(boys_slice, slice);
+    class_body<LA, LB, LC, LD, Real, UHF, KL0, KL1>(list, n, v, slice, slice + boys_slice_size<Real>(), sp);
 }
 
 // Digestion of stored integrals (the stored-integral SCF): integral blocks written once in store mode

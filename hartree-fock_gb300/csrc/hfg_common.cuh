@@ -100,7 +100,8 @@ __host__ __device__ constexpr int e3_total(int l1, int l2) { return e3_offset(l1
 
 // Per-primitive-pair record: [0] p, [1..3] P, [4] W = sqrt(2 pi^{5/2}) / p * exp(-ab/p |A-B|^2) * c_a c_b *
 // radial normalisation of both primitives (so that W_ab W_cd / sqrt(p+q) is the whole primitive
-// prefactor of an ERI), [5] 1/p, then e3_total(l1,l2) Hermite coefficients; padded to even.
+// prefactor of an ERI), [5] the index of p among the basis's distinct exponents in the low 32 bits of
+// 1.5 * 2^52 + index (no conversion on the FP64 pipe), then e3_total(l1,l2) Hermite coefficients; padded to even.
 constexpr int kPairHeader = 6;
 __host__ __device__ constexpr int pp_stride(int l1, int l2)
 {
