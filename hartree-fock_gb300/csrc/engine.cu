@@ -124,6 +124,11 @@ struct hfg_engine
     // ev2: fork, join, FP32 start, FP32 end.
     cudaStream_t stream2 = nullptr;
     cudaEvent_t ev2[4] {};
+    // Short lists (a class kernel that cannot fill the GPU by itself) run side by side on side[precision][0..3],
+    // forked from and joined to the precision's own stream: a small molecule has up to 21 of them per
+    // precision, each as long as its longest quartet.
+    cudaStream_t side[2][4] {};
+    cudaEvent_t ev_side[2][5] {}; // fork, then the end of each side stream
     bool overlap = true;
     float overlap_share = 1.0f;   // FP64 class kernels' grids
     float overlap_share32 = 1.0f; // FP32 class kernels' grids
@@ -1387,6 +1392,36 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
     return pick;
 }
 
+// The side streams of one precision, forked from its own stream at construction and joined to it by join().
+// Lists are short below 64 primitive quartets for each lane of a full GPU (eight warps an SM).
+struct SideStreams
+{
+    hfg_engine* e;
+    int prec;
+    cudaStream_t own;
+    int used = 0;
+    SideStreams(hfg_engine* e_, int prec_, cudaStream_t own_) : e(e_), prec(prec_), own(own_)
+    {
+        HFG_CUDA(cudaEventRecord(e->ev_side[prec][0], own));
+    }
+    bool is_short(unsigned long long prims) const { return prims < static_cast<unsigned long long>(e->num_sms) * 256 * 64; }
+    cudaStream_t next()
+    {
+        const int k = used++ % 4;
+        if (used <= 4)
+            HFG_CUDA(cudaStreamWaitEvent(e->side[prec][k], e->ev_side[prec][0], 0));
+        return e->side[prec][k];
+    }
+    void join()
+    {
+        for (int k = 0; k < std::min(used, 4); ++k)
+        {
+            HFG_CUDA(cudaEventRecord(e->ev_side[prec][1 + k], e->side[prec][k]));
+            HFG_CUDA(cudaStreamWaitEvent(own, e->ev_side[prec][1 + k], 0));
+        }
+    }
+};
+
 // Enqueues one build on the engine stream.  Eager (graph == false): timing events, list lengths read
 // back after the list build, only non-empty classes launched, forms tuned on first use.  Graph: nothing
 // that needs the host (no read-back, no tuning): every class with a non-empty capacity is launched
@@ -1481,16 +1516,24 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
         cudaStream_t ps = (overlap && prec == 1) ? e->stream2 : s;
         if (!graph && !(persist && prec == 0))
             HFG_CUDA(cudaEventRecord(overlap && prec == 1 ? e->ev2[2] : e->ev[3 + prec], ps));
+        // The long lists first, one after the other on the precision's stream (each fills the GPU; kernel forms
+        // are timed here on first use), then the short ones spread over the side streams, where they also
+        // fill the tails of the long ones.
+        SideStreams side(e, prec, ps);
         const unsigned long long* h_prims = e->h_counts.size() >= static_cast<size_t>(4 * kNumQuartetClasses)
                                                 ? e->h_counts.data() + 2 * kNumQuartetClasses : nullptr;
-        for (int qc = kNumQuartetClasses - 1; qc >= 0; --qc)
+        for (int pq = 0; pq < 2 * kNumQuartetClasses; ++pq)
         {
+            const int pass = pq / kNumQuartetClasses, qc = kNumQuartetClasses - 1 - pq % kNumQuartetClasses;
             const unsigned long long n = graph ? e->cap[qc] : e->h_counts[2 * qc + prec];
             if (n == 0 || in_queue(qc))
                 continue;
             // In a graph the counts are those of the eager build before the capture: the kernels read the replay's
-            // own on the device, these only size the grids.
+            // own on the device, these only size the grids and choose the streams.
             const unsigned long long prims = h_prims ? h_prims[2 * qc + prec] : n;
+            const bool is_short = side.is_short(prims) && n < kTuneMin;
+            if (is_short != (pass == 1))
+                continue;
             const int P1 = [&] { int p = 0; while ((p + 1) * (p + 2) / 2 <= qc) ++p; return p; }();
             const int P2 = qc - P1 * (P1 + 1) / 2;
             const int L  = pair_class_l1(P1) + pair_class_l2(P1) + pair_class_l1(P2) + pair_class_l2(P2);
@@ -1513,7 +1556,7 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             c.tables     = e->d_tables.p;
             c.fp32       = prec == 1;
             c.uhf        = uhf;
-            c.stream     = ps;
+            c.stream     = is_short ? side.next() : ps;
             c.num_sms    = e->num_sms;
             c.share      = overlap ? (prec == 1 ? e->overlap_share32 : e->overlap_share) : 1.f;
             c.pmax       = max_prims(e, P1, P2);
@@ -1531,6 +1574,7 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             form_ran[qc][prec] = c.form != 0 ? c.form : class_default_form(qc, prec == 1);
             launches += class_launches(qc, prec == 1, c.form);
         }
+        side.join();
         if (!graph && overlap && prec == 1)
             HFG_CUDA(cudaEventRecord(e->ev2[3], ps));
         if (!graph && overlap && prec == 0)
@@ -2299,6 +2343,25 @@ extern "C" {
 
 const char* hfg_version(void) { return "hfgpu 0.1 (sm_103a)"; }
 
+static void destroy_side(hfg_engine* e)
+{
+    for (auto& streams : e->side)
+        for (auto& st : streams)
+            if (st)
+            {
+                cudaStreamSynchronize(st);
+                cudaStreamDestroy(st);
+                st = nullptr;
+            }
+    for (auto& evs : e->ev_side)
+        for (auto& ev : evs)
+            if (ev)
+            {
+                cudaEventDestroy(ev);
+                ev = nullptr;
+            }
+}
+
 int hfg_create_batch(const hfg_basis* bases, int nmol, int device, hfg_engine** out)
 {
     if (!out || !bases || nmol <= 0)
@@ -2320,6 +2383,10 @@ int hfg_create_batch(const hfg_basis* bases, int nmol, int device, hfg_engine** 
         HFG_CUDA(cudaStreamCreateWithFlags(&e->stream2, cudaStreamNonBlocking));
         for (auto& ev : e->ev) HFG_CUDA(cudaEventCreate(&ev));
         for (auto& ev : e->ev2) HFG_CUDA(cudaEventCreate(&ev));
+        for (auto& streams : e->side)
+            for (auto& st : streams) HFG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        for (auto& evs : e->ev_side)
+            for (auto& ev : evs) HFG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         e->nmol = nmol;
         e->basis.resize(nmol);
         long long mat = 0, smax = 0;
@@ -2355,6 +2422,7 @@ int hfg_create_batch(const hfg_basis* bases, int nmol, int device, hfg_engine** 
             cudaStreamDestroy(e->stream2);
             e->stream2 = nullptr;
         }
+        destroy_side(e.get());
         return rc;
     }
     *out = e.release();
@@ -2382,6 +2450,7 @@ void hfg_destroy(hfg_engine* e)
     for (auto& ev : e->ev2)
         if (ev)
             cudaEventDestroy(ev);
+    destroy_side(e);
     if (e->stream2)
     {
         cudaStreamSynchronize(e->stream2);
