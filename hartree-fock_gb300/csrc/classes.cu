@@ -288,12 +288,26 @@ namespace
 //   FP64: (ss|ss) (ps|ss) (ps|ps) (pp|ss) (ds|ss);  FP32: also (pp|ps) (ds|ps) (dp|ss).
 template <typename Real> constexpr bool grad_thread_form()
 {
-    return GradThread<LA, LB, LC, LD>::kValues <= (sizeof(Real) == 8 ? 72 : 160);
+    return GradThread<LA, LB, LC, LD>::kValues <= (sizeof(Real) == 8 ? 300 : 160);
+}
+
+// The split of a gradient launch: `width` lanes work on one slice together.
+template <typename Real> SplitArgs grad_split(const GradLaunch& c, int width)
+{
+    SplitArgs s;
+    if (sizeof(Real) == 4)
+        return s;
+    s.lanes = static_cast<unsigned>(c.num_sms) * 256u / width;
+    s.prims = c.prims;
+    unsigned long long m = c.prims / s.lanes;
+    m = m < 1 ? 1 : m;
+    while (s.smax < 128 && s.smax * m < static_cast<unsigned long long>(c.pmax)) s.smax <<= 1;
+    return s;
 }
 
 template <typename Real> cudaError_t launch_grad_thread(const GradLaunch& c)
 {
-    const size_t smem = sizeof(Real) * BoysGrid<Real>::kPoints * BoysGrid<Real>::kRow;
+    const size_t smem = sizeof(Real) * boys_slice_size<Real>();
     auto kern         = grad_thread_kernel<LA, LB, LC, LD, Real>;
     cudaError_t e     = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess)
@@ -302,10 +316,11 @@ template <typename Real> cudaError_t launch_grad_thread(const GradLaunch& c)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
     if (e != cudaSuccess)
         return e;
-    const unsigned long long need = (c.count + 127) / 128;
+    const SplitArgs sp            = grad_split<Real>(c, 1);
+    const unsigned long long need = ((c.count + 31) / 32 * sp.smax + 3) / 4;
     const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1);
-    kern<<<static_cast<unsigned>(need < cap ? need : cap), 128, smem, c.stream>>>(c.list, c.count, c.view,
-                                                                                static_cast<const Real*>(c.boys_slice));
+    kern<<<static_cast<unsigned>(need < cap ? need : cap), 128, smem, c.stream>>>(
+        c.list, c.count, c.view, static_cast<const Real*>(c.boys_slice), sp);
     return cudaGetLastError();
 }
 
@@ -315,7 +330,7 @@ template <typename Real> cudaError_t launch_grad_t(const GradLaunch& c)
         if (!c.group_form)
             return launch_grad_thread<Real>(c);
     using W           = GradLayout<LA, LB, LC, LD>;
-    const size_t smem = sizeof(Real) * (BoysGrid<Real>::kPoints * BoysGrid<Real>::kRow + W::kPerWarp * kGradWarps);
+    const size_t smem = sizeof(Real) * (boys_slice_size<Real>() + W::kPerWarp * kGradWarps);
     auto kern         = grad_class_kernel<LA, LB, LC, LD, Real>;
     cudaError_t e     = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess)
@@ -325,10 +340,11 @@ template <typename Real> cudaError_t launch_grad_t(const GradLaunch& c)
     if (e != cudaSuccess)
         return e;
     constexpr unsigned long long per_block = kGradWarps * (32 / W::kGroup); // quartets in flight per block
-    const unsigned long long need = (c.count + per_block - 1) / per_block;
+    const SplitArgs sp            = grad_split<Real>(c, W::kGroup);
+    const unsigned long long need = (c.count * sp.smax + per_block - 1) / per_block;
     const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1);
     kern<<<static_cast<unsigned>(need < cap ? need : cap), 32 * kGradWarps, smem, c.stream>>>(
-        c.list, c.count, c.view, static_cast<const Real*>(c.boys_slice), c.tables);
+        c.list, c.count, c.view, static_cast<const Real*>(c.boys_slice), c.tables, sp);
     return cudaGetLastError();
 }
 } // namespace

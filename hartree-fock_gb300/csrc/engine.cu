@@ -166,7 +166,7 @@ struct hfg_engine
     double prim_thr = 1e-15;
     std::vector<double> h_qp[hfg::kNumPairClasses];
     std::vector<int> npp_full, keep_off, keep_idx;
-    int cls_npp[hfg::kNumPairClasses] {}; // largest kept count of any pair, per class
+    int cls_npp[hfg::kNumPairClasses] {}, cls_npp_full[hfg::kNumPairClasses] {}; // largest of any pair: kept, all
     // Unscreened records in pack order (the nuclear gradient's derivative integrals use every primitive).
     hfg::DevBuf<double> d_pptab64_full[hfg::kNumPairClasses];
     hfg::DevBuf<float> d_pptab32_full[hfg::kNumPairClasses];
@@ -835,10 +835,12 @@ static void screen_primitives(hfg_engine* e)
         e->pairs[k].npp    = e->keep_off[k + 1] - e->keep_off[k];
     }
     std::fill(std::begin(e->cls_npp), std::end(e->cls_npp), 0);
+    std::fill(std::begin(e->cls_npp_full), std::end(e->cls_npp_full), 0);
     for (size_t k = 0; k < e->pairs.size(); ++k)
     {
         const int pc       = e->pair_class_of[k];
         e->cls_npp[pc]      = std::max(e->cls_npp[pc], e->pairs[k].npp);
+        e->cls_npp_full[pc] = std::max(e->cls_npp_full[pc], e->npp_full[k]);
     }
 }
 
@@ -1035,10 +1037,12 @@ static FockView base_view(hfg_engine* e, bool fp32)
     return v;
 }
 
-// Most primitive quartets a quartet of class (P1|P2) has in the Fock build (after the primitive screening).
-static int max_prims(const hfg_engine* e, int P1, int P2)
+// Most primitive quartets a quartet of class (P1|P2) has in the Fock build (after the primitive screening), or
+// in the gradient (`all`).
+static int max_prims(const hfg_engine* e, int P1, int P2, bool all = false)
 {
-    const long long p = static_cast<long long>(e->cls_npp[P1]) * e->cls_npp[P2];
+    const int* most   = all ? e->cls_npp_full : e->cls_npp;
+    const long long p = static_cast<long long>(most[P1]) * most[P2];
     return static_cast<int>(std::max(1ll, std::min(p, 1ll << 30)));
 }
 
@@ -2136,24 +2140,44 @@ static double gradient_two_electron(hfg_engine* e, const std::vector<int>& shell
         g.Dt = prec ? static_cast<const void*>(e->d_dDf[0].p) : e->d_dD[0].p;
         g.Da = prec ? static_cast<const void*>(e->d_dDf[1].p) : e->d_dD[1].p;
         g.Db = uhf ? (prec ? static_cast<const void*>(e->d_dDf[2].p) : e->d_dD[2].p) : g.Da;
+        g.et         = exponent_table(e);
         g.n          = e->mols[0].nao;
         g.shell_atom = e->d_shell_atom.p;
         g.grad       = e->d_grad.p;
     }
     HFG_CUDA(cudaEventRecord(e->ev[6], s));
+    // Streams as in a Fock build: the FP32 kernels beside the FP64 ones, the long lists of a precision one after
+    // the other, its short ones side by side.
+    const bool overlap = mixed && e->overlap;
+    if (overlap)
+    {
+        HFG_CUDA(cudaEventRecord(e->ev2[0], s));
+        HFG_CUDA(cudaStreamWaitEvent(e->stream2, e->ev2[0], 0));
+    }
     for (int prec = 0; prec < (mixed ? 2 : 1); ++prec)
-        for (int qc = kNumQuartetClasses - 1; qc >= 0; --qc)
+    {
+        SideStreams side(e, prec, overlap && prec == 1 ? e->stream2 : s);
+        for (int pq = 0; pq < 2 * kNumQuartetClasses; ++pq)
         {
-            const unsigned long long n = e->h_counts[2 * qc + prec];
-            if (n == 0)
+            const int pass = pq / kNumQuartetClasses, qc = kNumQuartetClasses - 1 - pq % kNumQuartetClasses;
+            const unsigned long long n = e->h_counts[2 * qc + prec], prims = e->h_counts[2 * kNumQuartetClasses + 2 * qc + prec];
+            if (n == 0 || side.is_short(prims) != (pass == 1))
                 continue;
             const int P1 = [&] { int p = 0; while ((p + 1) * (p + 2) / 2 <= qc) ++p; return p; }();
             const int P2 = qc - P1 * (P1 + 1) / 2;
             const int L  = pair_class_l1(P1) + pair_class_l2(P1) + pair_class_l1(P2) + pair_class_l2(P2);
-            const void* slice = prec ? static_cast<const void*>(e->d_boys32[L + 1].p) : e->d_boys64[L + 1].p;
-            GradLaunch g {e->d_list[qc][prec].p, n, v[prec], slice, e->d_tables.p, s, e->num_sms, prec == 1, e->grad_group_only};
+            const void* slice = prec ? static_cast<const void*>(e->d_boys32[L + 1].p) : e->d_boysf[L + 1].p;
+            GradLaunch g {e->d_list[qc][prec].p, n, v[prec], slice, e->d_tables.p, pass == 1 ? side.next() : side.own,
+                          e->num_sms, prec == 1, e->grad_group_only, prims, max_prims(e, P1, P2, true)};
             HFG_CUDA(launch_grad(qc, g));
         }
+        side.join();
+    }
+    if (overlap)
+    {
+        HFG_CUDA(cudaEventRecord(e->ev2[1], e->stream2));
+        HFG_CUDA(cudaStreamWaitEvent(s, e->ev2[1], 0));
+    }
     HFG_CUDA(cudaEventRecord(e->ev[7], s));
     std::vector<double> g(static_cast<size_t>(3) * natom);
     HFG_CUDA(cudaMemcpyAsync(g.data(), e->d_grad.p, sizeof(double) * g.size(), cudaMemcpyDeviceToHost, s));

@@ -72,6 +72,8 @@ struct GradLaunch
     int num_sms;
     bool fp32;
     bool group_form; // the lane-group kernel for every class (else the thread form where it is compiled)
+    unsigned long long prims; // as in ClassLaunch, for the split of short lists
+    int pmax;
 };
 cudaError_t launch_grad(int qclass, const GradLaunch& L);
 

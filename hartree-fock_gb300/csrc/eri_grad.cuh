@@ -45,6 +45,7 @@ struct GradView
     const void* Dt;                     // densities, Real of the kernel
     const void* Da;
     const void* Db;
+    ExponentTable et;
     int n;                  // nao
     const int* shell_atom;  // per shell
     double* grad;           // [natom][3]
@@ -89,7 +90,7 @@ template <typename Real> __device__ __forceinline__ Real e1(const Real* T, int l
 template <int LA, int LB, int LC, int LD, typename Real>
 __global__ void __launch_bounds__(32 * kGradWarps)
     grad_class_kernel(const Quartet* __restrict__ list, unsigned long long n, GradView v,
-                      const Real* __restrict__ boys_slice, const WarpTables* __restrict__ tabs)
+                      const Real* __restrict__ boys_slice, const WarpTables* __restrict__ tabs, SplitArgs sp)
 {
     using W = GradLayout<LA, LB, LC, LD>;
     constexpr int NB = W::NB, ND = W::ND, NAB = W::NAB, NCD = W::NCD;
@@ -106,10 +107,15 @@ __global__ void __launch_bounds__(32 * kGradWarps)
     const int wl = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int lane = wl % GS, grp = wl / GS; // lane within the quartet's group, group within the warp
     const unsigned gmask = (GS == 32) ? 0xffffffffu : (((1u << GS) - 1u) << (grp * GS));
-    if (static_cast<unsigned long long>(blockIdx.x) * kGradWarps * NG >= n)
+    // Items: S slices of every quartet's primitive quartets (SplitArgs with a lane group in the place of a
+    // lane), each worked on by one lane group, whose gradient terms simply add up.
+    constexpr bool kSplit = sizeof(Real) == 8; // FP32 lists are never split, as in the Fock build
+    const int S1 = kSplit ? sp.smax : 1, ls = __ffs(S1) - 1;
+    const unsigned long long items = n * static_cast<unsigned long long>(S1);
+    if (static_cast<unsigned long long>(blockIdx.x) * kGradWarps * NG >= items)
         return;
-    stage_boys<Real>(boys_slice, slice);
-    Real* wbase = slice + BoysGrid<Real>::kPoints * BoysGrid<Real>::kRow + wib * W::kPerWarp + grp * W::kPerGroup;
+    stage_boys<Real, boys_slice_size<Real>()>(boys_slice, slice);
+    Real* wbase = slice + boys_slice_size<Real>() + wib * W::kPerWarp + grp * W::kPerGroup;
     Real* Rbuf0 = wbase;
     Real* Rbuf1 = wbase + HL;
     Real* Gs    = wbase + 2 * HL;
@@ -121,12 +127,22 @@ __global__ void __launch_bounds__(32 * kGradWarps)
     const Real* Da = static_cast<const Real*>(v.Da);
     const Real* Db = static_cast<const Real*>(v.Db);
 
-    for (unsigned long long q = (static_cast<unsigned long long>(blockIdx.x) * kGradWarps + wib) * NG + grp; q < n;
-         q += static_cast<unsigned long long>(gridDim.x) * kGradWarps * NG)
+    unsigned long long m = sp.prims / sp.lanes;
+    m = m < 1 ? 1 : m;
+    for (unsigned long long it = (static_cast<unsigned long long>(blockIdx.x) * kGradWarps + wib) * NG + grp; it < items;
+         it += static_cast<unsigned long long>(gridDim.x) * kGradWarps * NG)
     {
-        const Quartet qt  = list[q];
+        const Quartet qt  = list[it >> ls];
         const PairRec bra = v.pairs[qt.bra];
         const PairRec ket = v.pairs[qt.ket];
+        PrimRange pr;
+        if (kSplit && S1 > 1)
+        {
+            const int slc = static_cast<int>(it) & (S1 - 1), g = split_lanes(bra.npp * ket.npp, m, S1);
+            if (slc >= g)
+                continue;
+            pr = split_range(bra.npp, ket.npp, slc, g);
+        }
         const int a0 = bra.ao1, b0 = bra.ao2, c0 = ket.ao1, d0 = ket.ao2;
         const int n = v.n;
         const Real sdeg = Real(4) * (bra.same ? Real(0.5) : Real(1)) * (ket.same ? Real(0.5) : Real(1)) * (qt.bra == qt.ket ? Real(0.5) : Real(1));
@@ -147,27 +163,15 @@ __global__ void __launch_bounds__(32 * kGradWarps)
 
         // The scalars of one primitive quartet into a row of the group's buffer: P - Q, then
         // Fs[n] = pref (-2 rho)^n F_n.  Each lane fills its own row, for a different primitive quartet.
-        auto prim_scalars = [&](const Real* rb, const Real* rk, Real* row)
+        auto scalars_row = [&](const Real* rb, const Real* rk, Real* row)
         {
-            const Real p = rb[0], qq = rk[0];
-            const Real X = rb[1] - rk[1], Y = rb[2] - rk[2], Z = rb[3] - rk[3];
-            const Real rs   = hfg_rsqrt(p + qq);
-            const Real rho  = (p * qq) * (rs * rs);
-            const Real pref = (rb[4] * rk[4]) * rs;
-            const Real T    = rho * (X * X + Y * Y + Z * Z);
-            Real F[L + 1];
-            boys_eval<L, Real>(T, slice, F);
+            Real X, Y, Z, Fs[L + 1];
+            prim_scalars<L, Real, sizeof(Real) == 8>(rb, rk, v.et, slice, X, Y, Z, Fs);
             row[0] = X;
             row[1] = Y;
             row[2] = Z;
-            const Real m2r = Real(-2) * rho;
-            Real w         = pref;
 #pragma unroll
-            for (int k = 0; k <= L; ++k)
-            {
-                row[3 + k] = w * F[k];
-                w *= m2r;
-            }
+            for (int k = 0; k <= L; ++k) row[3 + k] = Fs[k];
         };
         // R^0_{tuv} of one buffered primitive quartet into one of the group's two R buffers (levels in
         // parallel over the group's lanes); returns the buffer that holds it.
@@ -212,21 +216,21 @@ __global__ void __launch_bounds__(32 * kGradWarps)
         // Bra-outer pass (centres A, B): G[tuv][kl] (t+u+v <= LAB+1) summed over the ket primitives of one
         // bra primitive pair, then contracted with Gamma and the bra's derivative coefficients once per bra
         // primitive pair.
-        for (int ib = 0; ib < bra.npp; ++ib)
+        for (int ib = pr.ib0; ib < bra.npp; ib += pr.ibs)
         {
             const Real* __restrict__ rb = static_cast<const Real*>(v.pptab[PCB]) + static_cast<size_t>(bra.pp_off + ib) * SB;
             const Real* __restrict__ gb = static_cast<const Real*>(v.gtab[PCB]) + static_cast<size_t>(bra.pp_off + ib) * GB;
             const Real aexp = gb[0], bexp = gb[1];
             for (int e = lane; e < HAB1 * NCD; e += GS) Gs[e] = Real(0);
-            for (int ik = 0; ik < ket.npp; ++ik)
+            for (int ik = pr.ik0, j = 0; ik < ket.npp; ik += pr.iks, j = (j + 1) % GS)
             {
-                const int j = ik % GS;
                 if (j == 0)
                 {
                     // The next GS ket primitives' scalars, one per lane.
-                    if (ik + lane < ket.npp)
-                        prim_scalars(rb, static_cast<const Real*>(v.pptab[PCK]) + static_cast<size_t>(ket.pp_off + ik + lane) * SK,
-                                     Sb + lane * kScal);
+                    const int il = ik + lane * pr.iks;
+                    if (il < ket.npp)
+                        scalars_row(rb, static_cast<const Real*>(v.pptab[PCK]) + static_cast<size_t>(ket.pp_off + il) * SK,
+                                    Sb + lane * kScal);
                     __syncwarp(gmask);
                 }
                 // The ket's 3-D Hermite coefficients E^{kl}_{tau nu phi} from its forward record (one DFMA per
@@ -289,21 +293,21 @@ __global__ void __launch_bounds__(32 * kGradWarps)
 
         // Ket-outer pass (centre C): X[ij][tuv'] (tau+nu+phi <= LCD+1) summed over the bra primitives of one
         // ket primitive pair, then contracted once per ket primitive pair.
-        for (int ik = 0; ik < ket.npp; ++ik)
+        for (int ik = pr.ik0; ik < ket.npp; ik += pr.iks)
         {
             const Real* __restrict__ rk = static_cast<const Real*>(v.pptab[PCK]) + static_cast<size_t>(ket.pp_off + ik) * SK;
             const Real* __restrict__ gk = static_cast<const Real*>(v.gtab[PCK]) + static_cast<size_t>(ket.pp_off + ik) * GK;
             const Real cexp = gk[0];
             for (int e = lane; e < NAB * HCD1; e += GS) Xs[e] = Real(0);
-            for (int ib = 0; ib < bra.npp; ++ib)
+            for (int ib = pr.ib0, j = 0; ib < bra.npp; ib += pr.ibs, j = (j + 1) % GS)
             {
-                const int j = ib % GS;
                 if (j == 0)
                 {
                     // The next GS bra primitives' scalars, one per lane.
-                    if (ib + lane < bra.npp)
-                        prim_scalars(static_cast<const Real*>(v.pptab[PCB]) + static_cast<size_t>(bra.pp_off + ib + lane) * SB, rk,
-                                     Sb + lane * kScal);
+                    const int il = ib + lane * pr.ibs;
+                    if (il < bra.npp)
+                        scalars_row(static_cast<const Real*>(v.pptab[PCB]) + static_cast<size_t>(bra.pp_off + il) * SB, rk,
+                                    Sb + lane * kScal);
                     __syncwarp(gmask);
                 }
                 // The bra's 3-D Hermite coefficients from its forward record, as for the ket in the first pass.
@@ -405,7 +409,8 @@ template <int LA, int LB, int LC, int LD> struct GradThread
 
 template <int LA, int LB, int LC, int LD, typename Real>
 __global__ void __launch_bounds__(128)
-    grad_thread_kernel(const Quartet* __restrict__ list, unsigned long long n, GradView v, const Real* __restrict__ boys_slice)
+    grad_thread_kernel(const Quartet* __restrict__ list, unsigned long long n, GradView v, const Real* __restrict__ boys_slice,
+                       SplitArgs sp)
 {
     using W = GradThread<LA, LB, LC, LD>;
     constexpr int NB = ncart(LB), ND = ncart(LD), NAB = W::NAB, NCD = W::NCD;
@@ -419,9 +424,15 @@ __global__ void __launch_bounds__(128)
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Real* slice = reinterpret_cast<Real*>(smem_raw);
-    if (static_cast<unsigned long long>(blockIdx.x) * blockDim.x >= n)
+    // Windows of 32 quartets, each worked on by G warps (SplitArgs); the lanes' gradient terms add up.
+    constexpr bool kSplit = sizeof(Real) == 8; // FP32 lists are never split, as in the Fock build
+    const int S = kSplit ? sp.smax : 1, ls = __ffs(S) - 1;
+    const unsigned long long items = ((n + 31) >> 5) * static_cast<unsigned long long>(S);
+    if (static_cast<unsigned long long>(blockIdx.x) * 4 >= items)
         return;
-    stage_boys<Real>(boys_slice, slice);
+    unsigned long long m = sp.prims / sp.lanes;
+    m = m < 1 ? 1 : m;
+    stage_boys<Real, boys_slice_size<Real>()>(boys_slice, slice);
     const Real* __restrict__ tbf = static_cast<const Real*>(v.pptab[PCB]);
     const Real* __restrict__ tkf = static_cast<const Real*>(v.pptab[PCK]);
     const Real* __restrict__ tbg = static_cast<const Real*>(v.gtab[PCB]);
@@ -431,14 +442,27 @@ __global__ void __launch_bounds__(128)
     const Real* Db = static_cast<const Real*>(v.Db);
     const int lane = threadIdx.x & 31;
 
-    for (unsigned long long base = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u);
-         base < n; base += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
+    for (unsigned long long it = static_cast<unsigned long long>(blockIdx.x) * 4 + (threadIdx.x >> 5); it < items;
+         it += static_cast<unsigned long long>(gridDim.x) * 4)
     {
-        const unsigned long long q = base + lane;
-        const bool active          = q < n;
-        const Quartet qt           = list[active ? q : base];
-        const PairRec bra          = v.pairs[qt.bra];
-        const PairRec ket          = v.pairs[qt.ket];
+        const unsigned long long base = (it >> ls) * 32;
+        unsigned long long q          = base + lane;
+        int g = 1, r = 0;
+        if (kSplit && S > 1)
+        {
+            const int slc   = static_cast<int>(it) & (S - 1);
+            const Quartet w = list[q < n ? q : base];
+            g = split_lanes(__reduce_max_sync(0xffffffffu, v.pairs[w.bra].npp * v.pairs[w.ket].npp), m, S);
+            if (slc >= g)
+                continue;
+            q = base + (g <= 32 ? slc * (32 / g) + lane / g : slc / (g / 32));
+            r = g <= 32 ? lane % g : (slc % (g / 32)) * 32 + lane;
+        }
+        bool active       = q < n;
+        const Quartet qt  = list[active ? q : base];
+        const PairRec bra = v.pairs[qt.bra];
+        const PairRec ket = v.pairs[qt.ket];
+        const PrimRange pr = kSplit && g > 1 ? split_range(bra.npp, ket.npp, r, g) : PrimRange {};
         Real gA[3] = {0, 0, 0}, gP[3] = {0, 0, 0}, gC[3] = {0, 0, 0};
         if (active)
         {
@@ -465,34 +489,19 @@ __global__ void __launch_bounds__(128)
             // R^0_{tuv}, t+u+v <= L, of one primitive quartet.
             auto prim_R = [&](const Real* rb, const Real* rk, Real* R)
             {
-                const Real p = rb[0], qq = rk[0];
-                const Real X = rb[1] - rk[1], Y = rb[2] - rk[2], Z = rb[3] - rk[3];
-                const Real rs   = hfg_rsqrt(p + qq);
-                const Real rho  = (p * qq) * (rs * rs);
-                const Real pref = (rb[4] * rk[4]) * rs;
-                const Real T    = rho * (X * X + Y * Y + Z * Z);
-                Real F[L + 1];
-                boys_eval<L, Real>(T, slice, F);
-                Real Fs[L + 1];
-                const Real m2r = Real(-2) * rho;
-                Real w         = pref;
-#pragma unroll
-                for (int m = 0; m <= L; ++m)
-                {
-                    Fs[m] = w * F[m];
-                    w *= m2r;
-                }
+                Real X, Y, Z, Fs[L + 1];
+                prim_scalars<L, Real, sizeof(Real) == 8>(rb, rk, v.et, slice, X, Y, Z, Fs);
                 hermite_R<L, Real>(Fs, X, Y, Z, R);
             };
 
             // Bra-outer pass: centres A and P.
-            for (int ib = 0; ib < bra.npp; ++ib)
+            for (int ib = pr.ib0; ib < bra.npp; ib += pr.ibs)
             {
                 const Real* __restrict__ rb = tbf + static_cast<size_t>(bra.pp_off + ib) * SB;
                 Real Gs[HAB1 * NCD];
 #pragma unroll
                 for (int x = 0; x < HAB1 * NCD; ++x) Gs[x] = Real(0);
-                for (int ik = 0; ik < ket.npp; ++ik)
+                for (int ik = pr.ik0; ik < ket.npp; ik += pr.iks)
                 {
                     const Real* __restrict__ rk = tkf + static_cast<size_t>(ket.pp_off + ik) * SK;
                     Real R[nherm(L)];
@@ -589,13 +598,13 @@ __global__ void __launch_bounds__(128)
             }
 
             // Ket-outer pass: centre C.
-            for (int ik = 0; ik < ket.npp; ++ik)
+            for (int ik = pr.ik0; ik < ket.npp; ik += pr.iks)
             {
                 const Real* __restrict__ rk = tkf + static_cast<size_t>(ket.pp_off + ik) * SK;
                 Real Hs[HCD1 * NAB];
 #pragma unroll
                 for (int x = 0; x < HCD1 * NAB; ++x) Hs[x] = Real(0);
-                for (int ib = 0; ib < bra.npp; ++ib)
+                for (int ib = pr.ib0; ib < bra.npp; ib += pr.ibs)
                 {
                     const Real* __restrict__ rb = tbf + static_cast<size_t>(bra.pp_off + ib) * SB;
                     Real R[nherm(L)];
@@ -672,6 +681,22 @@ __global__ void __launch_bounds__(128)
                             });
                     });
             }
+        }
+        if (kSplit && g > 1)
+        {
+            // Sum the lanes of each quartet; its first lane goes on with the sum.
+            for (int o = min(g, 32) >> 1; o > 0; o >>= 1)
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+                {
+                    gA[x] += __shfl_xor_sync(0xffffffffu, gA[x], o);
+                    gP[x] += __shfl_xor_sync(0xffffffffu, gP[x], o);
+                    gC[x] += __shfl_xor_sync(0xffffffffu, gC[x], o);
+                }
+            active = active && lane % min(g, 32) == 0;
+            if (!active)
+#pragma unroll
+                for (int x = 0; x < 3; ++x) gA[x] = gP[x] = gC[x] = Real(0);
         }
         // g_B = g_P - g_A, g_D = -(g_P + g_C); the bra atoms' terms summed over the warp when it shares the bra.
         const unsigned bra0 = __shfl_sync(0xffffffffu, qt.bra, 0);
