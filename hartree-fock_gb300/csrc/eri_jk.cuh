@@ -382,13 +382,69 @@ template <int ND, int KL0, int KL1> __host__ __device__ constexpr bool chunk_has
     return false;
 }
 
+// 2x and |x| < thr without the FP64 pipe in FP64 (thr >= 0; IEEE bit patterns of non-negative numbers order
+// like the numbers, a NaN is above any thr).  Doubling drops subnormals.
+__device__ __forceinline__ double twice(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return (b & 0x7ff0000000000000ll) == 0 ? 0.0 : __longlong_as_double(b + 0x0010000000000000ll);
+}
+__device__ __forceinline__ float twice(float x) { return 2.0f * x; }
+__device__ __forceinline__ bool below(double x, double thr)
+{
+    return (__double_as_longlong(x) & 0x7fffffffffffffffll) < __double_as_longlong(thr);
+}
+__device__ __forceinline__ bool below(float x, float thr) { return fabsf(x) < thr; }
+
+// Sums x[0..N) over the warp, handing half of the values to the other half of the lanes at every step: some
+// N + 5 additions a lane in the place of 5 N.  Returns this lane's value and its index (-1: another lane
+// adds it).  N <= 64; values beyond 32 leave two per lane, in `second`.
+template <int N> __device__ __forceinline__ void warp_sum_spread(double* x, int lane, double& first, int& at1, double& second, int& at2)
+{
+    int base = 0, len = N; // this lane's values are base .. base + len of the original
+    bool mine = true;
+    static_for<0, 5>(
+        [&](auto S)
+        {
+            constexpr int o = 16 >> decltype(S)::value;
+            // Values held at this step: ceil(N / 2^S).
+            constexpr int M = (N + (1 << decltype(S)::value) - 1) >> decltype(S)::value, H = (M + 1) / 2;
+            const bool up = (lane & o) != 0;
+            if constexpr (M == 1)
+            {
+                x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+                mine = mine && !up;
+            }
+            else
+            {
+#pragma unroll
+                for (int k = 0; k < H; ++k)
+                {
+                    const double lo = x[k], hi = H + k < M ? x[H + k] : 0.0;
+                    const double other = __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
+                    x[k]               = (up ? hi : lo) + other;
+                }
+                base += up ? H : 0;
+                len = up ? max(0, len - H) : min(len, H);
+            }
+        });
+    constexpr int last = (N + 31) >> 5;
+    first  = x[0];
+    at1    = mine && len > 0 ? base : -1;
+    second = last > 1 ? x[1] : 0.0;
+    at2    = mine && len > 1 ? base + 1 : -1;
+}
+
 // Digestion of one evaluated quartet into X, Ya (, Yb), with its density values already loaded; acc holds
 // the integrals of the ket components kl in [KL0, KL1) (all of them by default), and only the output
 // elements those components reach are added.
+// Normalised: acc carries the angular factors already.  The skip and the degeneracy factor (a power of two,
+// 1 for most quartets) are applied before the contraction, without the FP64 pipe where nothing is to scale.
 // bra_warp: every lane of the warp calls this together and all active lanes hold the same bra pair;
 // the bra's Coulomb block X_ab is then summed over the warp and added once (inactive lanes pass
 // active = false and acc = 0).  Otherwise each active lane adds its own.
-template <int LA, int LB, int LC, int LD, typename Real, bool UHF, int KL0 = 0, int KL1 = ncart(LC) * ncart(LD)>
+template <int LA, int LB, int LC, int LD, typename Real, bool UHF, int KL0 = 0, int KL1 = ncart(LC) * ncart(LD),
+          bool Normalised = false>
 __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec& ket, bool same_pair, const Real* acc,
                                               const FockView& v, const DigestD<LA, LB, LC, LD, Real, UHF>& d,
                                               bool active, bool bra_warp)
@@ -401,6 +457,20 @@ __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec&
     const Real thr = ao_threshold<Real>(v);
     const int a0 = bra.ao1, b0 = bra.ao2, c0 = ket.ao1, d0 = ket.ao2;
     auto at = [&](int r, int c) -> long long { return off + r + static_cast<long long>(c) * n; };
+
+    Real w[NAB * CH];
+    static_for<0, NAB * CH>(
+        [&](auto E)
+        {
+            constexpr int x   = decltype(E)::value;
+            constexpr Real an = Real(ang_norm(LA, x / CH / NB) * ang_norm(LB, (x / CH) % NB) *
+                                     ang_norm(LC, (KL0 + x % CH) / ND) * ang_norm(LD, (KL0 + x % CH) % ND));
+            const Real eri = Normalised ? acc[x] : acc[x] * an;
+            w[x]           = below(eri, thr) ? Real(0) : eri;
+        });
+    if (__any_sync(__activemask(), s != Real(1)))
+#pragma unroll
+        for (int x = 0; x < NAB * CH; ++x) w[x] *= s;
 
     Real Jab[NAB], Jcd[CH];
 #pragma unroll
@@ -435,19 +505,16 @@ __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec&
                             {
                                 constexpr int kl = decltype(KLx)::value;
                                 constexpr int k = kl / ND, l = kl % ND;
-                                constexpr Real an = Real(ang_norm(LA, i) * ang_norm(LB, j) * ang_norm(LC, k)
-                                                         * ang_norm(LD, l));
-                                const Real eri = acc[(i * NB + j) * CH + (kl - KL0)] * an;
-                                const Real w   = (fabs(eri) < thr) ? Real(0) : s * eri;
+                                const Real g = w[(i * NB + j) * CH + (kl - KL0)];
                                 if (spin == 0)
                                 {
-                                    Jab[i * NB + j] += w * d.Dcd[k * ND + l];
-                                    Jcd[kl - KL0] += w * d.Dab[i * NB + j];
+                                    Jab[i * NB + j] += g * d.Dcd[k * ND + l];
+                                    Jcd[kl - KL0] += g * d.Dab[i * NB + j];
                                 }
-                                Kac[i * NC + k] += w * d.Dbd[spin][j * ND + l];
-                                Kad[i * ND + l] += w * d.Dbc[spin][j * NC + k];
-                                Kbc[j * NC + k] += w * d.Dad[spin][i * ND + l];
-                                Kbd[j * ND + l] += w * d.Dac[spin][i * NC + k];
+                                Kac[i * NC + k] += g * d.Dbd[spin][j * ND + l];
+                                Kad[i * ND + l] += g * d.Dbc[spin][j * NC + k];
+                                Kbc[j * NC + k] += g * d.Dad[spin][i * ND + l];
+                                Kbd[j * ND + l] += g * d.Dac[spin][i * NC + k];
                             });
                     });
             });
@@ -498,14 +565,27 @@ __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec&
     {
         // Warp sum of the bra block, then one atomic per element from lane 0.
         const int lane = threadIdx.x & 31;
-#pragma unroll
-        for (int x = 0; x < NAB; ++x)
+        if constexpr (sizeof(Real) == 8)
         {
-            Real t = Jab[x];
+            double t1, t2;
+            int x1, x2;
+            warp_sum_spread<NAB>(Jab, lane, t1, x1, t2, x2);
+            if (x1 >= 0)
+                atomicAdd(v.X + at(a0 + x1 / NB, b0 + x1 % NB), twice(t1));
+            if (NAB > 32 && x2 >= 0)
+                atomicAdd(v.X + at(a0 + x2 / NB, b0 + x2 % NB), twice(t2));
+        }
+        else
+        {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (lane == 0)
-                atomicAdd(v.X + at(a0 + x / NB, b0 + x % NB), widen(Real(2) * t));
+            for (int x = 0; x < NAB; ++x)
+            {
+                Real t = Jab[x];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (lane == 0)
+                    atomicAdd(v.X + at(a0 + x / NB, b0 + x % NB), widen(twice(t)));
+            }
         }
     }
     else if (active)
@@ -513,13 +593,13 @@ __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec&
 #pragma unroll
         for (int i = 0; i < NA; ++i)
 #pragma unroll
-            for (int j = 0; j < NB; ++j) atomicAdd(v.X + at(a0 + i, b0 + j), widen(Real(2) * Jab[i * NB + j]));
+            for (int j = 0; j < NB; ++j) atomicAdd(v.X + at(a0 + i, b0 + j), widen(twice(Jab[i * NB + j])));
     }
     if (active)
     {
 #pragma unroll
         for (int x = 0; x < CH; ++x)
-            atomicAdd(v.X + at(c0 + (KL0 + x) / ND, d0 + (KL0 + x) % ND), widen(Real(2) * Jcd[x]));
+            atomicAdd(v.X + at(c0 + (KL0 + x) / ND, d0 + (KL0 + x) % ND), widen(twice(Jcd[x])));
     }
 }
 
@@ -605,7 +685,7 @@ __device__ __forceinline__ void digest_shared(const PairRec& bra, const PairRec&
     auto at = [&](int r, int c) -> long long { return off + r + static_cast<long long>(c) * n; };
     const Real s   = (bra.same ? Real(0.5) : Real(1)) * (ket.same ? Real(0.5) : Real(1)) * (same_pair ? Real(0.5) : Real(1));
     const Real thr = ao_threshold<Real>(v);
-    for (int x = lane; x < NAB * CH; x += 32) w[x] = (fabs(w[x]) < thr) ? Real(0) : s * w[x];
+    for (int x = lane; x < NAB * CH; x += 32) w[x] = below(w[x], thr) ? Real(0) : s * w[x];
     __syncwarp();
     constexpr int nJ = NAB + CH, nK = (NA + NB) * (NC + ND), nspin = UHF ? 2 : 1;
     for (int o = lane; o < nJ + nspin * nK; o += 32)
@@ -614,13 +694,13 @@ __device__ __forceinline__ void digest_shared(const PairRec& bra, const PairRec&
         if (o < NAB)
         {
             for (int x = 0; x < CH; ++x) sum += w[o * CH + x] * ldD<Real>(v.Dt, at(c0 + (KL0 + x) / ND, d0 + (KL0 + x) % ND));
-            atomicAdd(v.X + at(a0 + o / NB, b0 + o % NB), widen(Real(2) * sum));
+            atomicAdd(v.X + at(a0 + o / NB, b0 + o % NB), widen(twice(sum)));
         }
         else if (o < nJ)
         {
             const int x = o - NAB;
             for (int ij = 0; ij < NAB; ++ij) sum += w[ij * CH + x] * ldD<Real>(v.Dt, at(a0 + ij / NB, b0 + ij % NB));
-            atomicAdd(v.X + at(c0 + (KL0 + x) / ND, d0 + (KL0 + x) % ND), widen(Real(2) * sum));
+            atomicAdd(v.X + at(c0 + (KL0 + x) / ND, d0 + (KL0 + x) % ND), widen(twice(sum)));
         }
         else
         {
@@ -886,17 +966,14 @@ __device__ __forceinline__ void stored_body(const Quartet* __restrict__ list, un
                     [&](auto KLx)
                     {
                         constexpr int kl = decltype(KLx)::value;
-                        // The digestion multiplies by the angular factors again.
-                        constexpr double inv_an = 1.0 / (ang_norm(LA, ij / NB) * ang_norm(LB, ij % NB) *
-                                                         ang_norm(LC, kl / ND) * ang_norm(LD, kl % ND));
-                        acc[ij * CH + (kl - KL0)] = active ? blk[ij * NCD + kl] * inv_an : 0.0;
+                        acc[ij * CH + (kl - KL0)] = active ? blk[ij * NCD + kl] : 0.0;
                     });
             });
         DD d;
         load_digest_d<LA, LB, LC, LD, double, UHF>(bra, ket, v, d);
         const unsigned bra0 = __shfl_sync(0xffffffffu, qt.bra, 0);
         const bool bra_warp = __all_sync(0xffffffffu, qt.bra == bra0);
-        digest_loaded<LA, LB, LC, LD, double, UHF, KL0, KL1>(bra, ket, qt.bra == qt.ket, acc, v, d, active, bra_warp);
+        digest_loaded<LA, LB, LC, LD, double, UHF, KL0, KL1, true>(bra, ket, qt.bra == qt.ket, acc, v, d, active, bra_warp);
     }
 }
 
