@@ -46,21 +46,24 @@ constexpr bool dual_form(bool fp32) { return fp32 && (QC == 11 || QC == 12 || QC
 // Ket-chunked thread form (FP32 d classes): ket components per thread, chosen so that R, G[HAB][CH] and
 // ERI[NAB][CH] stay in registers (HL + (HAB + NAB) * CH floats well below 255); 0 = not compiled.
 //   (dp|pp) (dp|ds): 3   (dp|dp): 2   (dd|ps) (dd|pp) (dd|ds) (dd|dp): 1
-// In FP64 (dp|pp) (dp|ds) (dp|dp): 3   (dd|ps): 1; what does not fit the registers spills to L1, whose traffic (two wavefronts per
-// warp and value) hides behind the FP64 pipe (16 SM cycles per warp instruction).
+// In FP64 (dp|pp) (dp|ds) (dp|dp): 3   (dd|ps) (dd|pp) (dd|ds): 1; what does not fit the registers spills to
+// L1, whose traffic (two wavefronts per warp and value) hides behind the FP64 pipe (16 SM cycles per warp
+// instruction).
 constexpr int chunk_width(bool fp32)
 {
     if (!fp32)
-        return (QC >= 12 && QC <= 14) ? 3 : QC == 16 ? 1 : 0;
+        return (QC >= 12 && QC <= 14) ? 3 : (QC >= 16 && QC <= 18) ? 1 : 0;
     return (QC == 12 || QC == 13) ? 3 : QC == 14 ? 2 : (QC >= 16 && QC <= 19) ? 1 : 0;
 }
 // The form a launch with form 0 runs (before or without autotuning): the chunked form where the tuner
-// keeps it at full size ((H2O)_64/6-31G**: (dp|pp), (dp|ds), (dp|dp), (dd|pp), (dd|ds), (dd|dp) in FP32),
-// else warp or thread.
+// keeps it at full size ((H2O)_64/6-31G**: (dp|pp), (dp|ds), (dp|dp), (dd|pp), (dd|ds), (dd|dp) in FP32; in FP64
+// wherever it is compiled, at every size: an FP64 build of (H2O)_27/6-31G** takes 346 ms with the warp form and
+// 35 / 29 / 18 / 12 ms less with (dp|pp) / (dp|ds) / (dp|dp) / (dd|ps) chunked, whose lanes are all busy), else
+// warp or thread.
 constexpr int default_form(bool fp32)
 {
-    return (fp32 && (QC == 12 || QC == 13 || QC == 14 || (QC >= 17 && QC <= 19))) ? kFormChunk
-                                                                                   : (warp_form(fp32) ? kFormWarp : kFormThread);
+    const bool chunk = fp32 ? (QC == 12 || QC == 13 || QC == 14 || (QC >= 17 && QC <= 19)) : chunk_width(false) > 0;
+    return chunk ? kFormChunk : (warp_form(fp32) ? kFormWarp : kFormThread);
 }
 constexpr unsigned form_mask(bool fp32)
 {

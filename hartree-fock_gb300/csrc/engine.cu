@@ -1344,8 +1344,11 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
                 pick = f;
         return pick;
     }
+    // The FP64 group form is not tried: the thread form splits short lists itself, and on long ones the group form
+    // loses in every class (12 to 53 ms of a 346 ms FP64 build of (H2O)_27/6-31G**).
+    const unsigned tried       = prec == 0 ? mask & ~(1u << kFormGroup) : mask;
     const unsigned long long n = base.count_host;
-    if (n < kTuneMin || !e->autotune)
+    if (n < kTuneMin || !e->autotune || (tried & (tried - 1)) == 0)
         return 0; // too small to time, or tuning off: the default form runs and the class stays untuned
     const auto t0 = std::chrono::steady_clock::now();
     const unsigned long long nch   = n <= kTuneSample ? 1 : kTuneChunks;
@@ -1376,7 +1379,7 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
     float best    = 0.f;
     for (int f = 1; f < 32; ++f)
     {
-        if (!((mask >> f) & 1u))
+        if (!((tried >> f) & 1u))
             continue;
         t.form = f;
         HFG_CUDA(launch_class(qc, t));
