@@ -77,15 +77,34 @@ constexpr unsigned form_mask(bool fp32)
 template <typename Real> SplitArgs split_args(const ClassLaunch& c)
 {
     SplitArgs s;
+    // FP32 windows are short (some 10 us): four at a time, which also keep their bra's rows in L1.
     if (sizeof(Real) == 4)
+    {
+        s.run = 4;
         return s;
+    }
     s.lanes     = static_cast<unsigned>(c.num_sms) * 256u;
     s.prims     = c.prims;
     s.prims_dev = c.prims_dev;
     unsigned long long m = c.prims / s.lanes;
     m = m < 1 ? 1 : m;
     while (s.smax < 128 && s.smax * m < static_cast<unsigned long long>(c.pmax)) s.smax <<= 1;
+    // Blocks take pieces of four slices when split: a quarter of a window at a time at most, since the slices
+    // beyond a window's own G are empty.
+    s.run = s.smax >= 32 ? s.smax / 16 : 1;
     return s;
+}
+
+// Sets the launch's counter where its items make more than one wave of blocks.
+inline cudaError_t queue_items(SplitArgs& s, unsigned long long* next, unsigned long long need, unsigned long long cap, cudaStream_t stream)
+{
+    if (next == nullptr || need <= cap)
+    {
+        s.run = 1;
+        return cudaSuccess;
+    }
+    s.next = next;
+    return cudaMemsetAsync(next, 0, sizeof(unsigned long long), stream);
 }
 
 // Resident blocks per SM a grid may take: the occupancy limit times the share, at least one.
@@ -177,7 +196,7 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
                     if (err != cudaSuccess)
                         return;
                     auto kern         = jk_class_chunk_kernel<LA, LB, LC, LD, Real, UHF, k0, k1>;
-                    const SplitArgs sp = split_args<Real>(c);
+                    SplitArgs sp = split_args<Real>(c);
                     const size_t smem = kFastBytes + (sp.smax >= 32 ? sizeof(Real) * split_scratch<LA, LB, k0, k1>() : 0);
                     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
                     if (err != cudaSuccess)
@@ -188,6 +207,9 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
                         return;
                     const unsigned long long need = ((c.count_host + 31) / 32 * sp.smax + 3) / 4;
                     const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share);
+                    err = queue_items(sp, c.next ? c.next + decltype(C)::value : nullptr, need, cap, c.stream);
+                    if (err != cudaSuccess)
+                        return;
                     kern<<<static_cast<unsigned>(need < cap ? need : cap), 128, smem, c.stream>>>(
                         c.list, c.count_dev, c.view, fast, sp);
                     err = cudaGetLastError();
@@ -224,7 +246,7 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
         if (form == kFormThread)
         {
             auto kern           = jk_class_kernel<LA, LB, LC, LD, Real, UHF>;
-            const SplitArgs sp  = split_args<Real>(c);
+            SplitArgs sp        = split_args<Real>(c);
             const size_t smem   = kFastBytes + (sp.smax >= 32 ? sizeof(Real) * split_scratch<LA, LB, 0, NCD>() : 0);
             cudaError_t e       = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
             if (e != cudaSuccess)
@@ -236,6 +258,9 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
             const unsigned long long need = ((c.count_host + 31) / 32 * sp.smax + 3) / 4;
             const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share);
             const unsigned grid           = static_cast<unsigned>(need < cap ? need : cap);
+            e = queue_items(sp, c.next, need, cap, c.stream);
+            if (e != cudaSuccess)
+                return e;
             kern<<<grid, 128, smem, c.stream>>>(c.list, c.count_dev, c.view, fast, sp);
             return cudaGetLastError();
         }
@@ -298,6 +323,7 @@ template <typename Real> constexpr bool grad_thread_form()
 template <typename Real> SplitArgs grad_split(const GradLaunch& c, int width)
 {
     SplitArgs s;
+    s.run = width == 1 ? 1 : 4;
     if (sizeof(Real) == 4)
         return s;
     s.lanes = static_cast<unsigned>(c.num_sms) * 256u / width;
@@ -305,6 +331,8 @@ template <typename Real> SplitArgs grad_split(const GradLaunch& c, int width)
     unsigned long long m = c.prims / s.lanes;
     m = m < 1 ? 1 : m;
     while (s.smax < 128 && s.smax * m < static_cast<unsigned long long>(c.pmax)) s.smax <<= 1;
+    if (s.smax >= 8)
+        s.run = s.smax / 4; // the slices beyond a window's own G are empty
     return s;
 }
 
@@ -319,9 +347,12 @@ template <typename Real> cudaError_t launch_grad_thread(const GradLaunch& c)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
     if (e != cudaSuccess)
         return e;
-    const SplitArgs sp            = grad_split<Real>(c, 1);
+    SplitArgs sp                  = grad_split<Real>(c, 1);
     const unsigned long long need = ((c.count + 31) / 32 * sp.smax + 3) / 4;
     const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1);
+    e = queue_items(sp, c.next, need, cap, c.stream);
+    if (e != cudaSuccess)
+        return e;
     kern<<<static_cast<unsigned>(need < cap ? need : cap), 128, smem, c.stream>>>(
         c.list, c.count, c.view, static_cast<const Real*>(c.boys_slice), sp);
     return cudaGetLastError();
@@ -343,9 +374,12 @@ template <typename Real> cudaError_t launch_grad_t(const GradLaunch& c)
     if (e != cudaSuccess)
         return e;
     constexpr unsigned long long per_block = kGradWarps * (32 / W::kGroup); // quartets in flight per block
-    const SplitArgs sp            = grad_split<Real>(c, W::kGroup);
+    SplitArgs sp                  = grad_split<Real>(c, W::kGroup);
     const unsigned long long need = (c.count * sp.smax + per_block - 1) / per_block;
     const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1);
+    e = queue_items(sp, c.next, need, cap, c.stream);
+    if (e != cudaSuccess)
+        return e;
     kern<<<static_cast<unsigned>(need < cap ? need : cap), 32 * kGradWarps, smem, c.stream>>>(
         c.list, c.count, c.view, static_cast<const Real*>(c.boys_slice), c.tables, sp);
     return cudaGetLastError();

@@ -222,12 +222,14 @@ struct hfg_engine
     unsigned long long cap[hfg::kNumQuartetClasses] {};
     bool cap_mixed = false;
     hfg::DevBuf<hfg::Quartet> d_list[hfg::kNumQuartetClasses][2];
+    hfg::DevBuf<unsigned long long> d_next;   // item counters [prec][qclass][kMaxChunks] of the class launches
     hfg::DevBuf<unsigned long long> d_counts; // [qclass][prec] quartets, then [qclass][prec] prim quartets, then overflow
     std::vector<unsigned long long> h_counts;
 
     // Work matrices.
     hfg::DevBuf<double> d_dD[3];   // tot, alpha, beta (FP64)
-    hfg::DevBuf<float> d_dDf[3];   // FP32 copies for the FP32 kernels
+    hfg::DevBuf<float> d_dDf[3];   // FP32 copies for the FP32 kernels (alpha, beta transposed in a Fock build)
+    hfg::DevBuf<double> d_dDT[3];  // alpha, beta transposed for the FP64 kernels of a Fock build
     hfg::DevBuf<double> d_acc[3];  // X, Ya, Yb
     hfg::DevBuf<double> d_out[3];  // J, Ka, Kb
     hfg::DevBuf<double> d_smax[3]; // shell-pair maxima of |dD|
@@ -292,6 +294,31 @@ __global__ void to_float_kernel(const double* __restrict__ a, float* __restrict_
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         b[i] = static_cast<float>(a[i]);
+}
+
+// The transposed copies of the molecule blocks of a: t64, t32 (either may be null).
+__global__ void transpose_kernel(const double* __restrict__ a, double* __restrict__ t64, float* __restrict__ t32,
+                                 const long long* __restrict__ mat_off, const int* __restrict__ mat_ld, int nmol, long long total)
+{
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x)
+    {
+        int lo = 0, hi = nmol - 1;
+        while (lo < hi)
+        {
+            const int mid = (lo + hi + 1) >> 1;
+            if (mat_off[mid] <= e)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        const long long off = mat_off[lo], loc = e - off;
+        const int n = mat_ld[lo], r = static_cast<int>(loc % n), c = static_cast<int>(loc / n);
+        const double x = a[off + c + (long long)r * n];
+        if (t64)
+            t64[e] = x;
+        if (t32)
+            t32[e] = static_cast<float>(x);
+    }
 }
 
 // nch contiguous chunks of `chunk` entries, chunk c starting at entry c * (n / nch) of list[0, n)
@@ -1006,6 +1033,7 @@ static void pack_molecules(hfg_engine* e)
     auto tables = std::make_unique<WarpTables>();
     build_warp_tables(*tables);
     e->d_tables.alloc(1);
+    e->d_next.alloc(2 * kNumQuartetClasses * kMaxChunks);
     HFG_CUDA(cudaMemcpyAsync(e->d_tables.p, tables.get(), sizeof(WarpTables), cudaMemcpyHostToDevice, e->stream));
     for (int L = 0; L <= kMaxLt + 1; ++L)
     {
@@ -1449,16 +1477,18 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
         HFG_CUDA(cudaMemcpyAsync(e->d_dD[k].p, src[k], sizeof(double) * N2,
                                  r.device_pointers ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
         HFG_CUDA(cudaMemsetAsync(e->d_acc[k].p, 0, sizeof(double) * N2, s));
-        if (mixed)
-        {
+        if (k > 0)
+            transpose_kernel<<<grid_for(N2, 256, e->num_sms), 256, 0, s>>>(e->d_dD[k].p, e->d_dDT[k].p,
+                                                                          mixed ? e->d_dDf[k].p : nullptr, e->d_mat_off.p,
+                                                                          e->d_mat_ld.p, e->nmol, N2);
+        else if (mixed)
             to_float_kernel<<<grid_for(N2, 256, e->num_sms), 256, 0, s>>>(e->d_dD[k].p, e->d_dDf[k].p, N2);
-            HFG_CUDA(cudaGetLastError());
-        }
+        HFG_CUDA(cudaGetLastError());
     }
     if (!graph)
         HFG_CUDA(cudaEventRecord(e->ev[1], s));
 
-    int launches = nspin * (mixed ? 2 : 1) +
+    int launches = nspin - 1 + (mixed ? 1 : 0) +
                    build_lists(e, uhf, mixed, r.schwartz_threshold, r.density_threshold, r.fp32_cutoff, graph);
 
     // Class kernels: FP64 lists on `s`; FP32 lists on stream2 concurrently when overlapping, else after.
@@ -1472,8 +1502,8 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
         FockView v  = base_view(e, prec == 1);
         v.pairs     = e->d_spairs.p;
         v.Dt        = prec == 1 ? static_cast<const void*>(e->d_dDf[0].p) : e->d_dD[0].p;
-        v.Da        = prec == 1 ? static_cast<const void*>(e->d_dDf[1].p) : e->d_dD[1].p;
-        v.Db        = prec == 1 ? static_cast<const void*>(e->d_dDf[2].p) : e->d_dD[2].p;
+        v.Da        = prec == 1 ? static_cast<const void*>(e->d_dDf[1].p) : e->d_dDT[1].p;
+        v.Db        = prec == 1 ? static_cast<const void*>(e->d_dDf[2].p) : e->d_dDT[2].p;
         v.X         = e->d_acc[0].p;
         v.Ya        = e->d_acc[1].p;
         v.Yb        = e->d_acc[2].p;
@@ -1551,8 +1581,8 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             c.view       = base_view(e, prec == 1);
             c.view.pairs = e->d_spairs.p;
             c.view.Dt    = prec == 1 ? static_cast<const void*>(e->d_dDf[0].p) : e->d_dD[0].p;
-            c.view.Da    = prec == 1 ? static_cast<const void*>(e->d_dDf[1].p) : e->d_dD[1].p;
-            c.view.Db    = prec == 1 ? static_cast<const void*>(e->d_dDf[2].p) : e->d_dD[2].p;
+            c.view.Da    = prec == 1 ? static_cast<const void*>(e->d_dDf[1].p) : e->d_dDT[1].p;
+            c.view.Db    = prec == 1 ? static_cast<const void*>(e->d_dDf[2].p) : e->d_dDT[2].p;
             c.view.X     = e->d_acc[0].p;
             c.view.Ya    = e->d_acc[1].p;
             c.view.Yb    = e->d_acc[2].p;
@@ -1569,6 +1599,7 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             c.pmax       = max_prims(e, P1, P2);
             c.prims_dev  = e->d_counts.p + 2 * kNumQuartetClasses + 2 * qc + prec;
             c.prims      = prims;
+            c.next       = e->d_next.p + (prec * kNumQuartetClasses + qc) * kMaxChunks;
             if (graph)
             {
                 const int set  = e->form_set[qc][prec];
@@ -1656,6 +1687,8 @@ static void fock_direct(hfg_engine* e, const hfg_fock_request& r, hfg_fock_stats
     for (int k = 0; k < 3; ++k)
     {
         e->d_dD[k].alloc(N2);
+        if (k > 0)
+            e->d_dDT[k].alloc(N2);
         e->d_acc[k].alloc(N2);
         e->d_out[k].alloc(N2);
         e->d_smax[k].alloc(e->smax_total);
@@ -1779,6 +1812,8 @@ static void store_integrals(hfg_engine* e, double sthr, size_t* bytes_out)
     for (int k = 0; k < 3; ++k)
     {
         e->d_dD[k].alloc(N2);
+        if (k > 0)
+            e->d_dDT[k].alloc(N2);
         e->d_acc[k].alloc(N2);
         e->d_out[k].alloc(N2);
         e->d_smax[k].alloc(e->smax_total);
@@ -1855,8 +1890,14 @@ static void fock_conventional(hfg_engine* e, const hfg_fock_request& r, hfg_fock
         HFG_CUDA(cudaMemcpyAsync(e->d_dD[k].p, src[k], sizeof(double) * N2,
                                  r.device_pointers ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
         HFG_CUDA(cudaMemsetAsync(e->d_acc[k].p, 0, sizeof(double) * N2, s));
+        if (k > 0)
+        {
+            transpose_kernel<<<grid_for(N2, 256, e->num_sms), 256, 0, s>>>(e->d_dD[k].p, e->d_dDT[k].p, nullptr, e->d_mat_off.p,
+                                                                          e->d_mat_ld.p, e->nmol, N2);
+            HFG_CUDA(cudaGetLastError());
+        }
     }
-    int launches = 0;
+    int launches = nspin - 1;
     for (int qc = kNumQuartetClasses - 1; qc >= 0; --qc)
     {
         if (e->conv_n[qc] == 0)
@@ -1868,8 +1909,8 @@ static void fock_conventional(hfg_engine* e, const hfg_fock_request& r, hfg_fock
         L.view        = base_view(e, false);
         L.view.pairs  = e->d_spairs.p;
         L.view.Dt     = e->d_dD[0].p;
-        L.view.Da     = e->d_dD[1].p;
-        L.view.Db     = e->d_dD[2].p;
+        L.view.Da     = e->d_dDT[1].p;
+        L.view.Db     = e->d_dDT[2].p;
         L.view.X      = e->d_acc[0].p;
         L.view.Ya     = e->d_acc[1].p;
         L.view.Yb     = e->d_acc[2].p;
@@ -2171,7 +2212,8 @@ static double gradient_two_electron(hfg_engine* e, const std::vector<int>& shell
             const int L  = pair_class_l1(P1) + pair_class_l2(P1) + pair_class_l1(P2) + pair_class_l2(P2);
             const void* slice = prec ? static_cast<const void*>(e->d_boys32[L + 1].p) : e->d_boysf[L + 1].p;
             GradLaunch g {e->d_list[qc][prec].p, n, v[prec], slice, e->d_tables.p, pass == 1 ? side.next() : side.own,
-                          e->num_sms, prec == 1, e->grad_group_only, prims, max_prims(e, P1, P2, true)};
+                          e->num_sms, prec == 1, e->grad_group_only, prims, max_prims(e, P1, P2, true),
+                          e->d_next.p + (prec * kNumQuartetClasses + qc) * kMaxChunks};
             HFG_CUDA(launch_grad(qc, g));
         }
         side.join();

@@ -11,6 +11,8 @@
 
 namespace hfg
 {
+constexpr int kMaxChunks = 18; // launches of one class in the chunk form at most
+
 // Launches the class kernel of one quartet class for one list.
 struct ClassLaunch
 {
@@ -32,6 +34,7 @@ struct ClassLaunch
     unsigned long long prims = 0;
     const unsigned long long* prims_dev = nullptr;
     int pmax = 1;
+    unsigned long long* next = nullptr; // kMaxChunks item counters (SplitArgs::next), or null: static order
     float share = 1.f; // fraction of the resident blocks per SM the grid may take (concurrent precisions)
 };
 // Kernel forms of a class kernel (eri_jk.cuh, eri_warp.cuh, eri_group.cuh).
@@ -74,6 +77,7 @@ struct GradLaunch
     bool group_form; // the lane-group kernel for every class (else the thread form where it is compiled)
     unsigned long long prims; // as in ClassLaunch, for the split of short lists
     int pmax;
+    unsigned long long* next; // one item counter, as in ClassLaunch
 };
 cudaError_t launch_grad(int qclass, const GradLaunch& L);
 

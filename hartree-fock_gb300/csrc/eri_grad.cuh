@@ -129,8 +129,10 @@ __global__ void __launch_bounds__(32 * kGradWarps)
 
     unsigned long long m = sp.prims / sp.lanes;
     m = m < 1 ? 1 : m;
-    for (unsigned long long it = (static_cast<unsigned long long>(blockIdx.x) * kGradWarps + wib) * NG + grp; it < items;
-         it += static_cast<unsigned long long>(gridDim.x) * kGradWarps * NG)
+    unsigned long long round = 0, it = 0, end = 0;
+    while (take_items(sp, items, (static_cast<unsigned long long>(blockIdx.x) * kGradWarps + wib) * NG + grp,
+                      static_cast<unsigned long long>(gridDim.x) * kGradWarps * NG, false, gmask, grp * GS, nullptr, round, it, end))
+    for (; it < end; ++it)
     {
         const Quartet qt  = list[it >> ls];
         const PairRec bra = v.pairs[qt.bra];
@@ -442,8 +444,10 @@ __global__ void __launch_bounds__(128)
     const Real* Db = static_cast<const Real*>(v.Db);
     const int lane = threadIdx.x & 31;
 
-    for (unsigned long long it = static_cast<unsigned long long>(blockIdx.x) * 4 + (threadIdx.x >> 5); it < items;
-         it += static_cast<unsigned long long>(gridDim.x) * 4)
+    unsigned long long round = 0, it = 0, end = 0;
+    while (take_items(sp, items, blockIdx.x * 4ull + (threadIdx.x >> 5), gridDim.x * 4ull, false, 0xffffffffu, 0, nullptr, round,
+                      it, end))
+    for (; it < end; ++it)
     {
         const unsigned long long base = (it >> ls) * 32;
         unsigned long long q          = base + lane;

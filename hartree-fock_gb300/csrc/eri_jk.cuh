@@ -54,10 +54,13 @@ struct FockView
     const void* ksoa[kNumPairClasses];
     long long kfs[kNumPairClasses];
     const void* Dt;                     // dD_tot   (double for FP64 kernels, float for FP32 kernels)
-    const void* Da;                     // dD_alpha
-    const void* Db;                     // dD_beta (UHF)
+    // The exchange matrices are transposed, element (r, c) at c + r * n: the exchange terms pair an AO of the
+    // bra, which the lanes of a warp share, with one of the ket, which differs; along the ket index the
+    // components of a shell and neighbouring shells now share sectors and lines.
+    const void* Da;                     // dD_alpha, transposed
+    const void* Db;                     // dD_beta (UHF), transposed
     double* X;                          // J accumulator (J = X + X^T)
-    double* Ya;                         // K_alpha accumulator
+    double* Ya;                         // K_alpha accumulator, transposed or not (K = Y + Y^T)
     double* Yb;                         // K_beta accumulator (UHF)
     const long long* mat_off;           // per molecule: offset of its n x n block in the packed matrices
     const int* mat_ld;                  // per molecule: n
@@ -335,6 +338,7 @@ __device__ __forceinline__ void load_digest_d(const PairRec& bra, const PairRec&
     const int n         = v.mat_ld[bra.mol];
     const int a0 = bra.ao1, b0 = bra.ao2, c0 = ket.ao1, d0 = ket.ao2;
     auto at = [&](int r, int c) -> long long { return off + r + static_cast<long long>(c) * n; };
+    auto tr = [&](int r, int c) -> long long { return off + c + static_cast<long long>(r) * n; };
 #pragma unroll
     for (int k = 0; k < NC; ++k)
 #pragma unroll
@@ -351,17 +355,17 @@ __device__ __forceinline__ void load_digest_d(const PairRec& bra, const PairRec&
         for (int j = 0; j < NB; ++j)
         {
 #pragma unroll
-            for (int l = 0; l < ND; ++l) d.Dbd[spin][j * ND + l] = ldD<Real>(Ds, at(b0 + j, d0 + l));
+            for (int l = 0; l < ND; ++l) d.Dbd[spin][j * ND + l] = ldD<Real>(Ds, tr(b0 + j, d0 + l));
 #pragma unroll
-            for (int k = 0; k < NC; ++k) d.Dbc[spin][j * NC + k] = ldD<Real>(Ds, at(b0 + j, c0 + k));
+            for (int k = 0; k < NC; ++k) d.Dbc[spin][j * NC + k] = ldD<Real>(Ds, tr(b0 + j, c0 + k));
         }
 #pragma unroll
         for (int i = 0; i < NA; ++i)
         {
 #pragma unroll
-            for (int l = 0; l < ND; ++l) d.Dad[spin][i * ND + l] = ldD<Real>(Ds, at(a0 + i, d0 + l));
+            for (int l = 0; l < ND; ++l) d.Dad[spin][i * ND + l] = ldD<Real>(Ds, tr(a0 + i, d0 + l));
 #pragma unroll
-            for (int k = 0; k < NC; ++k) d.Dac[spin][i * NC + k] = ldD<Real>(Ds, at(a0 + i, c0 + k));
+            for (int k = 0; k < NC; ++k) d.Dac[spin][i * NC + k] = ldD<Real>(Ds, tr(a0 + i, c0 + k));
         }
     }
 }
@@ -457,6 +461,7 @@ __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec&
     const Real thr = ao_threshold<Real>(v);
     const int a0 = bra.ao1, b0 = bra.ao2, c0 = ket.ao1, d0 = ket.ao2;
     auto at = [&](int r, int c) -> long long { return off + r + static_cast<long long>(c) * n; };
+    auto tr = [&](int r, int c) -> long long { return off + c + static_cast<long long>(r) * n; };
 
     Real w[NAB * CH];
     static_for<0, NAB * CH>(
@@ -530,14 +535,14 @@ __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec&
                         {
                             constexpr int k = decltype(Kx)::value;
                             if constexpr (chunk_has_k<ND, KL0, KL1>(k))
-                                atomicAdd(Y + at(a0 + i, c0 + k), widen(Kac[i * NC + k]));
+                                atomicAdd(Y + tr(a0 + i, c0 + k), widen(Kac[i * NC + k]));
                         });
                     static_for<0, ND>(
                         [&](auto Lx)
                         {
                             constexpr int l = decltype(Lx)::value;
                             if constexpr (chunk_has_l<ND, KL0, KL1>(l))
-                                atomicAdd(Y + at(a0 + i, d0 + l), widen(Kad[i * ND + l]));
+                                atomicAdd(Y + tr(a0 + i, d0 + l), widen(Kad[i * ND + l]));
                         });
                 });
             static_for<0, NB>(
@@ -549,14 +554,14 @@ __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec&
                         {
                             constexpr int k = decltype(Kx)::value;
                             if constexpr (chunk_has_k<ND, KL0, KL1>(k))
-                                atomicAdd(Y + at(b0 + j, c0 + k), widen(Kbc[j * NC + k]));
+                                atomicAdd(Y + tr(b0 + j, c0 + k), widen(Kbc[j * NC + k]));
                         });
                     static_for<0, ND>(
                         [&](auto Lx)
                         {
                             constexpr int l = decltype(Lx)::value;
                             if constexpr (chunk_has_l<ND, KL0, KL1>(l))
-                                atomicAdd(Y + at(b0 + j, d0 + l), widen(Kbd[j * ND + l]));
+                                atomicAdd(Y + tr(b0 + j, d0 + l), widen(Kbd[j * ND + l]));
                         });
                 });
         }
@@ -639,6 +644,11 @@ __device__ __forceinline__ void stage_boys(const Real* __restrict__ g, Real* s)
 struct SplitArgs
 {
     int smax = 1;                             // warps per window at most, a power of two; 1: no split
+    int run  = 1;                             // consecutive items taken at a time
+    // Items taken so far by the whole launch (zeroed before it), or null: items go round robin.  The windows of a
+    // list differ a hundredfold in primitive quartets, and with some hundred windows a warp round robin left
+    // the SMs idle for a fifth of the FP64 (ps|ss) kernel of (H2O)_16 (ncu: 16.4 M of 21.2 M cycles active).
+    unsigned long long* next = nullptr;
     unsigned lanes = 1;                       // lanes that fill the GPU
     unsigned long long prims = 0;             // the list's primitive quartets,
     const unsigned long long* prims_dev = nullptr; // or where they stand (a captured graph's lists)
@@ -650,6 +660,34 @@ __device__ __forceinline__ int split_lanes(int P, unsigned long long m, int smax
     int g = 1;
     while (g < smax && static_cast<unsigned long long>(g) * m < static_cast<unsigned long long>(P)) g <<= 1;
     return g;
+}
+
+// Takes the next run of items [at, end) of `units`; false at the end of the list.  `who`: this taker's number
+// of `takers` (static order); `lead`: the lane that asks the counter, whose answer the mask's lanes share.
+// by_block: the whole block takes one run (through `box` in shared memory), else every mask's lanes theirs.
+__device__ __forceinline__ bool take_items(const SplitArgs& sp, unsigned long long units, unsigned long long who,
+                                           unsigned long long takers, bool by_block, unsigned mask, int lead,
+                                           unsigned long long* box, unsigned long long& round, unsigned long long& at,
+                                           unsigned long long& end)
+{
+    if (sp.next == nullptr)
+        at = (round++ * takers + who) * sp.run;
+    else if (by_block)
+    {
+        __syncthreads(); // every warp has read the last answer
+        if (threadIdx.x == 0)
+            *box = atomicAdd(sp.next, static_cast<unsigned long long>(sp.run));
+        __syncthreads();
+        at = *box;
+    }
+    else
+    {
+        if ((threadIdx.x & 31) == lead)
+            at = atomicAdd(sp.next, static_cast<unsigned long long>(sp.run));
+        at = __shfl_sync(mask, at, lead);
+    }
+    end = at + sp.run < units ? at + sp.run : units;
+    return at < units;
 }
 
 // Share of lane r of g: the g lanes as a gb x gk grid over the bra and ket primitives, powers of two with
@@ -683,6 +721,7 @@ __device__ __forceinline__ void digest_shared(const PairRec& bra, const PairRec&
     const int n         = v.mat_ld[bra.mol];
     const int a0 = bra.ao1, b0 = bra.ao2, c0 = ket.ao1, d0 = ket.ao2;
     auto at = [&](int r, int c) -> long long { return off + r + static_cast<long long>(c) * n; };
+    auto tr = [&](int r, int c) -> long long { return off + c + static_cast<long long>(r) * n; };
     const Real s   = (bra.same ? Real(0.5) : Real(1)) * (ket.same ? Real(0.5) : Real(1)) * (same_pair ? Real(0.5) : Real(1));
     const Real thr = ao_threshold<Real>(v);
     for (int x = lane; x < NAB * CH; x += 32) w[x] = below(w[x], thr) ? Real(0) : s * w[x];
@@ -717,14 +756,14 @@ __device__ __forceinline__ void digest_shared(const PairRec& bra, const PairRec&
                     continue;
                 const int dcol = cc ? d0 + ll : c0 + kk;
                 if (ra)
-                    for (int j = 0; j < NB; ++j) sum += w[(i0 * NB + j) * CH + x] * ldD<Real>(Ds, at(b0 + j, dcol));
+                    for (int j = 0; j < NB; ++j) sum += w[(i0 * NB + j) * CH + x] * ldD<Real>(Ds, tr(b0 + j, dcol));
                 else
-                    for (int i = 0; i < NA; ++i) sum += w[(i * NB + i0) * CH + x] * ldD<Real>(Ds, at(a0 + i, dcol));
+                    for (int i = 0; i < NA; ++i) sum += w[(i * NB + i0) * CH + x] * ldD<Real>(Ds, tr(a0 + i, dcol));
             }
             bool reached = false;
             for (int x = 0; x < CH; ++x) reached = reached || (cc ? (KL0 + x) / ND : (KL0 + x) % ND) == k0;
             if (reached)
-                atomicAdd((spin == 0 ? v.Ya : v.Yb) + at((ra ? a0 : b0) + i0, (cc ? c0 : d0) + k0), widen(sum));
+                atomicAdd((spin == 0 ? v.Ya : v.Yb) + tr((ra ? a0 : b0) + i0, (cc ? c0 : d0) + k0), widen(sum));
         }
     }
     __syncwarp(); // the next quartet reuses w
@@ -763,9 +802,15 @@ __device__ __forceinline__ void class_body(const Quartet* __restrict__ list, uns
     // Warp-uniform iteration (every lane runs the same trip count, inactive lanes past the end), so that
     // the digestion may sum the bra block over the warp.  With S >= 4 the four warps of a block are slices of
     // one window, so that they may share a quartet (G = 64, 128): their branches on G are block-uniform.
-    for (unsigned long long it = static_cast<unsigned long long>(blockIdx.x) * 4 + wib; it < items;
-         it += static_cast<unsigned long long>(gridDim.x) * 4)
+    // Runs keep the windows of one bra pair together, whose rows of D and records are then found in L1.
+    __shared__ unsigned long long box;
+    const bool by_block = S >= 4;
+    unsigned long long round = 0, at = 0, end = 0;
+    while (take_items(sp, by_block ? items / 4 : items, by_block ? blockIdx.x : blockIdx.x * 4ull + wib,
+                      by_block ? gridDim.x : gridDim.x * 4ull, by_block, 0xffffffffu, 0, &box, round, at, end))
+    for (; at < end; ++at)
     {
+        const unsigned long long it = by_block ? at * 4 + wib : at;
         unsigned long long base = it * 32, q = base + lane;
         int g = 1, r = 0;
         PrimRange pr;

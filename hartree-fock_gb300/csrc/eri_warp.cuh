@@ -333,7 +333,8 @@ __global__ void __launch_bounds__(32 * kWarpKernelWarps)
                 atomicAdd(v.X + at(c0 + kl / ND, d0 + kl % ND), widen(Real(2) * s));
             }
         }
-        // K blocks: ac, ad, bc, bd.
+        // K blocks: ac, ad, bc, bd (the exchange densities are transposed).
+        auto tr = [&](int r, int c) -> long long { return off + c + static_cast<long long>(r) * nld; };
         constexpr int nspin = UHF ? 2 : 1;
         for (int spin = 0; spin < nspin; ++spin)
         {
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(32 * kWarpKernelWarps)
                     const int i = o / NC, k = o % NC;
                     for (int j = 0; j < NB; ++j)
                         for (int l = 0; l < ND; ++l)
-                            s += Es[(i * NB + j) * NCD + k * ND + l] * ldD<Real>(Ds, at(b0 + j, d0 + l));
+                            s += Es[(i * NB + j) * NCD + k * ND + l] * ldD<Real>(Ds, tr(b0 + j, d0 + l));
                     atomicAdd(Yo + at(a0 + i, c0 + k), widen(s));
                 }
                 else if (o < NA * NC + NA * ND)
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(32 * kWarpKernelWarps)
                     const int r = o - NA * NC, i = r / ND, l = r % ND;
                     for (int j = 0; j < NB; ++j)
                         for (int k = 0; k < NC; ++k)
-                            s += Es[(i * NB + j) * NCD + k * ND + l] * ldD<Real>(Ds, at(b0 + j, c0 + k));
+                            s += Es[(i * NB + j) * NCD + k * ND + l] * ldD<Real>(Ds, tr(b0 + j, c0 + k));
                     atomicAdd(Yo + at(a0 + i, d0 + l), widen(s));
                 }
                 else if (o < NA * NC + NA * ND + NB * NC)
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(32 * kWarpKernelWarps)
                     const int r = o - NA * NC - NA * ND, j = r / NC, k = r % NC;
                     for (int i = 0; i < NA; ++i)
                         for (int l = 0; l < ND; ++l)
-                            s += Es[(i * NB + j) * NCD + k * ND + l] * ldD<Real>(Ds, at(a0 + i, d0 + l));
+                            s += Es[(i * NB + j) * NCD + k * ND + l] * ldD<Real>(Ds, tr(a0 + i, d0 + l));
                     atomicAdd(Yo + at(b0 + j, c0 + k), widen(s));
                 }
                 else
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(32 * kWarpKernelWarps)
                     const int r = o - NA * NC - NA * ND - NB * NC, j = r / ND, l = r % ND;
                     for (int i = 0; i < NA; ++i)
                         for (int k = 0; k < NC; ++k)
-                            s += Es[(i * NB + j) * NCD + k * ND + l] * ldD<Real>(Ds, at(a0 + i, c0 + k));
+                            s += Es[(i * NB + j) * NCD + k * ND + l] * ldD<Real>(Ds, tr(a0 + i, c0 + k));
                     atomicAdd(Yo + at(b0 + j, d0 + l), widen(s));
                 }
             }
