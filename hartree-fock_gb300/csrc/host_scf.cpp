@@ -333,6 +333,8 @@ class Scf
     int lwork_ = 0;
     int* info_ = nullptr;
     std::deque<Hist> hist_;
+    std::deque<std::vector<double>> dots_; // e_i . e_j, j <= i, of the history
+    DMat Cprev_;                           // last orbitals, where the level shift needs them
 
     void up(DMat& d, const std::vector<double>& h)
     {
@@ -499,12 +501,19 @@ class Scf
         }
     }
     // e = F_a D_a S - S D_a F_a + (beta), history of at most diis_size entries (DIIS.cpp:12-26).
+    // A full history gives its oldest buffers to the new entry (no allocation, whose cudaFree stalls the device).
     void diis_update()
     {
-        Hist h;
-        h.Fa.alloc(static_cast<size_t>(n_) * n_);
-        h.Fb.alloc(static_cast<size_t>(n_) * n_);
-        h.e.alloc(static_cast<size_t>(n_) * n_);
+        const bool full = static_cast<int>(hist_.size()) >= o_.diis_size;
+        Hist h          = full ? std::move(hist_.front()) : Hist {};
+        if (full)
+        {
+            hist_.pop_front();
+            dots_.pop_front();
+            for (auto& row : dots_) row.erase(row.begin());
+        }
+        else
+            for (DMat* m : {&h.Fa, &h.Fb, &h.e}) m->alloc(static_cast<size_t>(n_) * n_);
         auto comm = [&](const DMat& F, const DMat& D, double beta) {
             gemm(CUBLAS_OP_N, CUBLAS_OP_N, n_, n_, n_, 1.0, F.p, D.p, 0.0, T1_.p);
             gemm(CUBLAS_OP_N, CUBLAS_OP_N, n_, n_, n_, 1.0, T1_.p, S_.p, 0.0, T2_.p);
@@ -520,9 +529,11 @@ class Scf
         comm(Fb_, Db_, 1.0);
         copy(h.Fa, Fa_);
         copy(h.Fb, Fb_);
-        if (static_cast<int>(hist_.size()) >= o_.diis_size)
-            hist_.pop_front();
         hist_.push_back(std::move(h));
+        // The new row of B; the older dot products are kept (each is one host round trip).
+        std::vector<double> row;
+        for (const Hist& old : hist_) row.push_back(dot(hist_.back().e, old.e));
+        dots_.push_back(std::move(row));
     }
     // Bordered B c = (0, .., 0, -1), F = sum c_i F_i (DIIS.cpp:28-72).
     void diis_extrapolate()
@@ -533,7 +544,7 @@ class Scf
         std::vector<double> B(static_cast<size_t>(m + 1) * (m + 1), 0.0), rhs(m + 1, 0.0);
         for (int i = 0; i < m; ++i)
             for (int j = 0; j <= i; ++j)
-                B[i + j * (m + 1)] = B[j + i * (m + 1)] = dot(hist_[i].e, hist_[j].e);
+                B[i + j * (m + 1)] = B[j + i * (m + 1)] = dots_[i][j];
         for (int i = 0; i < m; ++i) B[m + i * (m + 1)] = B[i + m * (m + 1)] = -1.0;
         B[m + m * (m + 1)] = 0.0;
         rhs[m]            = -1.0;
@@ -591,6 +602,14 @@ class Scf
         for (int k = 0; k < n; ++k) x[perm[k]] = y[k];
         return x;
     }
+    // A copy of the orbitals C for the level shift.
+    const DMat& keep(const DMat& C)
+    {
+        if (!Cprev_.p)
+            Cprev_.alloc(static_cast<size_t>(n_) * n_);
+        copy(Cprev_, C);
+        return Cprev_;
+    }
     // SCF.cpp:747-835.
     void diagonalize_update(int it)
     {
@@ -609,18 +628,14 @@ class Scf
         }
         // alpha
         {
-            DMat Cprev(static_cast<size_t>(n_) * n_);
-            copy(Cprev, Ca_);
-            eig_orth(Fa_, Ca_, wa_, ls_a_, &Cprev, nocc_a_);
+            eig_orth(Fa_, Ca_, wa_, ls_a_, ls_a_ ? &keep(Ca_) : nullptr, nocc_a_);
         }
         copy(Dap_, Da_);
         density(Ca_, nocc_a_, Da_, damp_);
         copy(Dbp_, Db_);
         if (uhf_)
         {
-            DMat Cprev(static_cast<size_t>(n_) * n_);
-            copy(Cprev, Cb_);
-            eig_orth(Fb_, Cb_, wb_, ls_b_, &Cprev, nocc_b_);
+            eig_orth(Fb_, Cb_, wb_, ls_b_, ls_b_ ? &keep(Cb_) : nullptr, nocc_b_);
             density(Cb_, nocc_b_, Db_, damp_);
         }
         else
