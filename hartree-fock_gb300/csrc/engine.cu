@@ -214,7 +214,9 @@ struct hfg_engine
     hfg::DevBuf<int4> d_cls_seg[hfg::kNumPairClasses];
     hfg::DevBuf<int2> d_cls_sh[hfg::kNumPairClasses]; // (sh1, sh2) of each sorted position
     hfg::DevBuf<int2> d_cls_molseg[hfg::kNumPairClasses];
+    hfg::DevBuf<float4> d_cls_diff[hfg::kNumPairClasses]; // most diffuse primitive pair of each sorted position: P, p
     hfg::DevBuf<unsigned> d_bra_cnt[hfg::kNumQuartetClasses];            // per bra pair: survivors (fp64, fp32)
+    hfg::DevBuf<unsigned> d_bra_near[hfg::kNumQuartetClasses];           // per bra pair: near FP64 survivors
     hfg::DevBuf<unsigned long long> d_bra_off[hfg::kNumQuartetClasses];  // per bra pair: list offsets
 
     // Quartet lists (capacity for the Schwartz threshold they were sized for).
@@ -389,7 +391,10 @@ struct ClassBuild
     const int2* sh2;     // (sh1, sh2) per ket position
     const int4* seg2;    // ket class segments (equal primitive-pair count, Q descending inside)
     const int2* molseg2; // per molecule: ket segment range
+    const float4* diff1; // per position: centre and exponent p of the pair's most diffuse primitive pair
+    const float4* diff2;
     unsigned* bra_cnt;             // [n1][2]
+    unsigned* bra_near;            // [n1] FP64 survivors that are not far (below)
     unsigned long long* bra_off;   // [n1][2] exclusive offsets (pass 1)
     Quartet* out64;
     Quartet* out32;
@@ -428,6 +433,11 @@ struct BuildArgs
 // bra pair and precision, pass 1 writes them at scanned offsets in candidate order, so the list is
 // ordered by bra pair and, inside a bra pair, by ket primitive count: a warp of the class kernels sees
 // quartets of equal primitive counts.  FP32 / FP64 split by the quartet bound Q_i Q_j max|dD|.
+// The FP64 survivors of a bra pair are written in two parts, near and far: far is where the most diffuse
+// primitive quartet (and so, but for the shift between primitive centres, every one) has T > 30, the
+// asymptotic branch of the Boys function.  A warp with both kinds runs both branches, each with part of
+// its lanes: (ps|ss) of (H2O)_16 ran its FP64 instructions with 20.9 of 32 lanes.  FP32 survivors keep one
+// part, whose order their FP32 sums follow.
 __global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __grid_constant__ BuildArgs b)
 {
     int ci = 0;
@@ -453,7 +463,9 @@ __global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __g
     const long long dthr = __double_as_longlong(b.dthr);
     const long long ra = so + (long long)sa * ns, rb2 = so + (long long)sb * ns;
     const float Qfi = a.Qf1[i];
-    unsigned c64 = 0, c32 = 0;
+    const float4 di = a.diff1[i];
+    unsigned c64 = 0, c32 = 0, cfar = 0; // c64: near survivors in pass 1
+    const unsigned near64 = b.pass ? a.bra_near[i] : 0u;
     unsigned long long p64 = 0, p32 = 0;
     const unsigned long long o64 = b.pass ? a.bra_off[2 * i] : 0ull;
     const unsigned long long o32 = b.pass ? a.bra_off[2 * i + 1] : 0ull;
@@ -495,28 +507,39 @@ __global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __g
                     s64 = !lowp;
                 }
             }
-            const unsigned m64 = __ballot_sync(0xffffffffu, s64);
-            const unsigned m32 = __ballot_sync(0xffffffffu, s32);
-            const unsigned lt  = (1u << lane) - 1u;
+            bool far = false;
+            if (s64)
+            {
+                const float4 dj = a.diff2[j];
+                const float x = di.x - dj.x, y = di.y - dj.y, z = di.z - dj.z;
+                far = di.w * dj.w * (x * x + y * y + z * z) > static_cast<float>(kBoysAsymptotic) * (di.w + dj.w);
+            }
+            const unsigned mfar = __ballot_sync(0xffffffffu, far);
+            const unsigned m64  = __ballot_sync(0xffffffffu, s64 && !far);
+            const unsigned m32  = __ballot_sync(0xffffffffu, s32);
+            const unsigned lt   = (1u << lane) - 1u;
             if (b.pass)
             {
                 const Quartet qv {static_cast<uint32_t>(a.base1 + i), static_cast<uint32_t>(a.base2 + j)};
-                const unsigned long long w64 = o64 + c64 + __popc(m64 & lt), w32 = o32 + c32 + __popc(m32 & lt);
+                const unsigned long long w64 = o64 + (far ? near64 + cfar + __popc(mfar & lt) : c64 + __popc(m64 & lt)),
+                                         w32 = o32 + c32 + __popc(m32 & lt);
                 if (s64 && w64 < a.cap)
                     a.out64[w64] = qv;
                 if (s32 && w32 < a.cap)
                     a.out32[w32] = qv;
             }
             c64 += __popc(m64);
+            cfar += __popc(mfar);
             c32 += __popc(m32);
             const unsigned long long pp = (unsigned long long)pi.npp * seg.z;
-            p64 += pp * __popc(m64);
+            p64 += pp * (__popc(m64) + __popc(mfar));
             p32 += pp * __popc(m32);
         }
     }
     if (b.pass == 0 && lane == 0)
     {
-        a.bra_cnt[2 * i]     = c64;
+        a.bra_near[i]        = c64;
+        a.bra_cnt[2 * i]     = c64 + cfar;
         a.bra_cnt[2 * i + 1] = c32;
         unsigned long long* prims = b.counts + 2 * kNumQuartetClasses + 2 * a.qc;
         if (p64)
@@ -1168,6 +1191,20 @@ static void sort_classes(hfg_engine* e)
         std::vector<int2> sh(ids.size());
         for (size_t k2 = 0; k2 < ids.size(); ++k2) sh[k2] = make_int2(e->pairs[ids[k2]].sh1, e->pairs[ids[k2]].sh2);
         e->d_cls_sh[pc].upload(sh, e->stream);
+        const int stride = pp_stride(pair_class_l1(pc), pair_class_l2(pc));
+        std::vector<float4> diff(ids.size());
+        for (size_t k2 = 0; k2 < ids.size(); ++k2)
+        {
+            const double* rec = &e->h_tab[pc][static_cast<size_t>(e->orig_off[ids[k2]]) * stride];
+            const double* low = rec;
+            for (int i = 1; i < e->npp_full[ids[k2]]; ++i)
+                if (rec[static_cast<size_t>(i) * stride] < low[0])
+                    low = rec + static_cast<size_t>(i) * stride;
+            diff[k2] = make_float4(static_cast<float>(low[1]), static_cast<float>(low[2]), static_cast<float>(low[3]),
+                                   static_cast<float>(low[0]));
+        }
+        e->d_cls_diff[pc].upload(diff, e->stream);
+        HFG_CUDA(cudaStreamSynchronize(e->stream)); // diff dies here
         e->d_cls_ids[pc].upload(ids, e->stream);
         e->d_cls_Q[pc].upload(e->cls_Q[pc], e->stream);
         {
@@ -1251,6 +1288,7 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
             if (mixed)
                 e->d_list[qc][1].alloc(std::max<unsigned long long>(c, 1));
             e->d_bra_cnt[qc].alloc(2 * std::max<size_t>(e->cls_ids[P1].size(), 1));
+            e->d_bra_near[qc].alloc(std::max<size_t>(e->cls_ids[P1].size(), 1));
             e->d_bra_off[qc].alloc(2 * std::max<size_t>(e->cls_ids[P1].size(), 1));
         }
     e->cap_thr   = sthr;
@@ -1303,6 +1341,9 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
         c.Qf1         = e->d_cls_Qf[P1].p;
         c.Qf2         = e->d_cls_Qf[P2].p;
         c.bra_cnt     = e->d_bra_cnt[qc].p;
+        c.bra_near    = e->d_bra_near[qc].p;
+        c.diff1       = e->d_cls_diff[P1].p;
+        c.diff2       = e->d_cls_diff[P2].p;
         c.bra_off     = e->d_bra_off[qc].p;
         c.out64       = e->d_list[qc][0].p;
         c.out32       = mixed ? e->d_list[qc][1].p : nullptr;
@@ -1898,6 +1939,8 @@ static void fock_conventional(hfg_engine* e, const hfg_fock_request& r, hfg_fock
         }
     }
     int launches = nspin - 1;
+    // The classes side by side: each streams its own blocks, and the small ones fill the tails of the large.
+    SideStreams side(e, 0, s);
     for (int qc = kNumQuartetClasses - 1; qc >= 0; --qc)
     {
         if (e->conv_n[qc] == 0)
@@ -1916,11 +1959,12 @@ static void fock_conventional(hfg_engine* e, const hfg_fock_request& r, hfg_fock
         L.view.Yb     = e->d_acc[2].p;
         L.view.ao_thr = r.schwartz_threshold;
         L.uhf         = uhf;
-        L.stream      = s;
+        L.stream      = side.next();
         L.num_sms     = e->num_sms;
         HFG_CUDA(launch_stored(qc, L));
         ++launches;
     }
+    side.join();
     double* outs[3] = {r.J, r.K_alpha, r.K_beta};
     for (int k = 0; k < nspin; ++k)
     {
