@@ -86,25 +86,37 @@ template <typename Real> SplitArgs split_args(const ClassLaunch& c)
     s.lanes     = static_cast<unsigned>(c.num_sms) * 256u;
     s.prims     = c.prims;
     s.prims_dev = c.prims_dev;
-    unsigned long long m = c.prims / s.lanes;
-    m = m < 1 ? 1 : m;
-    while (s.smax < 128 && s.smax * m < static_cast<unsigned long long>(c.pmax)) s.smax <<= 1;
-    // Blocks take pieces of four slices when split: a quarter of a window at a time at most, since the slices
-    // beyond a window's own G are empty.
-    s.run = s.smax >= 32 ? s.smax / 16 : 1;
     return s;
 }
 
-// Sets the launch's counter where its items make more than one wave of blocks.
-inline cudaError_t queue_items(SplitArgs& s, unsigned long long* next, unsigned long long need, unsigned long long cap, cudaStream_t stream)
+// Sets the split for the list's longest quartet (pmax) and the order its items are taken in, for `cap` resident
+// blocks of `warps` warps (each `per` windows or groups wide) and `windows` of them; returns the blocks to launch.
+// Up to four waves of blocks go round robin, more through the counter `next`.
+inline unsigned long long plan_items(SplitArgs& s, bool split, unsigned long long pmax, unsigned long long windows,
+                                     unsigned per_block, unsigned long long cap, unsigned long long* next, cudaStream_t stream,
+                                     cudaError_t& err)
 {
-    if (next == nullptr || need <= cap)
+    err             = cudaSuccess;
+    auto warps_for = [&](bool queued, int most) {
+        int w = 1;
+        if (split)
+            while (w < most && w * split_share(s.prims, s.lanes, queued) < pmax) w <<= 1;
+        return w;
+    };
+    s.smax                  = warps_for(false, 128);
+    unsigned long long need = (windows * s.smax + per_block - 1) / per_block;
+    if (next == nullptr || need <= 4 * cap)
     {
         s.run = 1;
-        return cudaSuccess;
+        return need < cap ? need : cap;
     }
+    // Eight takers a window at most: the slices beyond a window's own G are empty.
+    s.smax = warps_for(true, 32);
+    s.run  = s.smax >= 8 ? s.smax / 8 : s.run;
     s.next = next;
-    return cudaMemsetAsync(next, 0, sizeof(unsigned long long), stream);
+    need   = (windows * s.smax + per_block - 1) / per_block;
+    err    = cudaMemsetAsync(next, 0, sizeof(unsigned long long), stream);
+    return need < cap ? need : cap;
 }
 
 // Resident blocks per SM a grid may take: the occupancy limit times the share, at least one.
@@ -197,7 +209,7 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
                         return;
                     auto kern         = jk_class_chunk_kernel<LA, LB, LC, LD, Real, UHF, k0, k1>;
                     SplitArgs sp = split_args<Real>(c);
-                    const size_t smem = kFastBytes + (sp.smax >= 32 ? sizeof(Real) * split_scratch<LA, LB, k0, k1>() : 0);
+                    const size_t smem = kFastBytes + (sizeof(Real) == 8 ? sizeof(Real) * split_scratch<LA, LB, k0, k1>() : 0);
                     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
                     if (err != cudaSuccess)
                         return;
@@ -205,12 +217,13 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
                     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
                     if (err != cudaSuccess)
                         return;
-                    const unsigned long long need = ((c.count_host + 31) / 32 * sp.smax + 3) / 4;
-                    const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share);
-                    err = queue_items(sp, c.next ? c.next + decltype(C)::value : nullptr, need, cap, c.stream);
+                    const unsigned long long grid =
+                        plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count_host + 31) / 32, 4,
+                                   static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share),
+                                   c.next ? c.next + decltype(C)::value : nullptr, c.stream, err);
                     if (err != cudaSuccess)
                         return;
-                    kern<<<static_cast<unsigned>(need < cap ? need : cap), 128, smem, c.stream>>>(
+                    kern<<<static_cast<unsigned>(grid), 128, smem, c.stream>>>(
                         c.list, c.count_dev, c.view, fast, sp);
                     err = cudaGetLastError();
                 });
@@ -247,7 +260,7 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
         {
             auto kern           = jk_class_kernel<LA, LB, LC, LD, Real, UHF>;
             SplitArgs sp        = split_args<Real>(c);
-            const size_t smem   = kFastBytes + (sp.smax >= 32 ? sizeof(Real) * split_scratch<LA, LB, 0, NCD>() : 0);
+            const size_t smem   = kFastBytes + (sizeof(Real) == 8 ? sizeof(Real) * split_scratch<LA, LB, 0, NCD>() : 0);
             cudaError_t e       = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
             if (e != cudaSuccess)
                 return e;
@@ -255,13 +268,12 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
             if (e != cudaSuccess)
                 return e;
-            const unsigned long long need = ((c.count_host + 31) / 32 * sp.smax + 3) / 4;
-            const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share);
-            const unsigned grid           = static_cast<unsigned>(need < cap ? need : cap);
-            e = queue_items(sp, c.next, need, cap, c.stream);
+            const unsigned long long grid =
+                plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count_host + 31) / 32, 4,
+                           static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share), c.next, c.stream, e);
             if (e != cudaSuccess)
                 return e;
-            kern<<<grid, 128, smem, c.stream>>>(c.list, c.count_dev, c.view, fast, sp);
+            kern<<<static_cast<unsigned>(grid), 128, smem, c.stream>>>(c.list, c.count_dev, c.view, fast, sp);
             return cudaGetLastError();
         }
     }
@@ -328,11 +340,6 @@ template <typename Real> SplitArgs grad_split(const GradLaunch& c, int width)
         return s;
     s.lanes = static_cast<unsigned>(c.num_sms) * 256u / width;
     s.prims = c.prims;
-    unsigned long long m = c.prims / s.lanes;
-    m = m < 1 ? 1 : m;
-    while (s.smax < 128 && s.smax * m < static_cast<unsigned long long>(c.pmax)) s.smax <<= 1;
-    if (s.smax >= 8)
-        s.run = s.smax / 4; // the slices beyond a window's own G are empty
     return s;
 }
 
@@ -348,12 +355,12 @@ template <typename Real> cudaError_t launch_grad_thread(const GradLaunch& c)
     if (e != cudaSuccess)
         return e;
     SplitArgs sp                  = grad_split<Real>(c, 1);
-    const unsigned long long need = ((c.count + 31) / 32 * sp.smax + 3) / 4;
-    const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1);
-    e = queue_items(sp, c.next, need, cap, c.stream);
+    const unsigned long long grid = plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count + 31) / 32, 4,
+                                               static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1), c.next,
+                                               c.stream, e);
     if (e != cudaSuccess)
         return e;
-    kern<<<static_cast<unsigned>(need < cap ? need : cap), 128, smem, c.stream>>>(
+    kern<<<static_cast<unsigned>(grid), 128, smem, c.stream>>>(
         c.list, c.count, c.view, static_cast<const Real*>(c.boys_slice), sp);
     return cudaGetLastError();
 }
@@ -373,14 +380,14 @@ template <typename Real> cudaError_t launch_grad_t(const GradLaunch& c)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kGradWarps, smem);
     if (e != cudaSuccess)
         return e;
-    constexpr unsigned long long per_block = kGradWarps * (32 / W::kGroup); // quartets in flight per block
+    constexpr unsigned per_block = kGradWarps * (32 / W::kGroup); // quartets in flight per block
     SplitArgs sp                  = grad_split<Real>(c, W::kGroup);
-    const unsigned long long need = (c.count * sp.smax + per_block - 1) / per_block;
-    const unsigned long long cap  = static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1);
-    e = queue_items(sp, c.next, need, cap, c.stream);
+    const unsigned long long grid = plan_items(sp, sizeof(Real) == 8, c.pmax, c.count, per_block,
+                                               static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1), c.next,
+                                               c.stream, e);
     if (e != cudaSuccess)
         return e;
-    kern<<<static_cast<unsigned>(need < cap ? need : cap), 32 * kGradWarps, smem, c.stream>>>(
+    kern<<<static_cast<unsigned>(grid), 32 * kGradWarps, smem, c.stream>>>(
         c.list, c.count, c.view, static_cast<const Real*>(c.boys_slice), c.tables, sp);
     return cudaGetLastError();
 }

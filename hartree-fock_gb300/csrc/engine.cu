@@ -2199,8 +2199,11 @@ static double gradient_two_electron(hfg_engine* e, const std::vector<int>& shell
     cudaStream_t s = e->stream;
     build_grad_tables(e);
     e->d_shell_atom.upload(shell_atom, s);
-    e->d_grad.alloc(static_cast<size_t>(3) * natom);
-    HFG_CUDA(cudaMemsetAsync(e->d_grad.p, 0, sizeof(double) * 3 * natom, s));
+    // Copies of the gradient the kernels' blocks add into, summed on the host.
+    const int copies = natom <= 4096 ? 32 : 1;
+    const size_t ng  = static_cast<size_t>(3) * natom;
+    e->d_grad.alloc(ng * copies);
+    HFG_CUDA(cudaMemsetAsync(e->d_grad.p, 0, sizeof(double) * ng * copies, s));
     const long long N2 = e->mat_total;
     if (mixed)
         for (int k = 0; k < 3; ++k)
@@ -2232,6 +2235,8 @@ static double gradient_two_electron(hfg_engine* e, const std::vector<int>& shell
         g.n          = e->mols[0].nao;
         g.shell_atom = e->d_shell_atom.p;
         g.grad       = e->d_grad.p;
+        g.copies     = copies;
+        g.natom      = natom;
     }
     HFG_CUDA(cudaEventRecord(e->ev[6], s));
     // Streams as in a Fock build: the FP32 kernels beside the FP64 ones, the long lists of a precision one after
@@ -2268,10 +2273,10 @@ static double gradient_two_electron(hfg_engine* e, const std::vector<int>& shell
         HFG_CUDA(cudaStreamWaitEvent(s, e->ev2[1], 0));
     }
     HFG_CUDA(cudaEventRecord(e->ev[7], s));
-    std::vector<double> g(static_cast<size_t>(3) * natom);
+    std::vector<double> g(ng * copies);
     HFG_CUDA(cudaMemcpyAsync(g.data(), e->d_grad.p, sizeof(double) * g.size(), cudaMemcpyDeviceToHost, s));
     HFG_CUDA(cudaStreamSynchronize(s));
-    for (size_t k = 0; k < g.size(); ++k) grad[k] += g[k];
+    for (size_t k = 0; k < g.size(); ++k) grad[k % ng] += g[k];
     float ms = 0.f;
     HFG_CUDA(cudaEventElapsedTime(&ms, e->ev[6], e->ev[7]));
     return ms;

@@ -48,7 +48,8 @@ struct GradView
     ExponentTable et;
     int n;                  // nao
     const int* shell_atom;  // per shell
-    double* grad;           // [natom][3]
+    double* grad;           // [copies][natom][3], summed by the caller: block b adds into copy b % copies, since
+    int copies, natom;      // all quartets of a small molecule would add to a few hundred addresses
 };
 
 #ifdef __CUDACC__
@@ -123,12 +124,12 @@ __global__ void __launch_bounds__(32 * kGradWarps)
     Real* Gam   = Xs + W::kX;
     Real* Sb    = Gam + W::kGam; // kGroup rows of kScal scalars
     constexpr int kScal = W::kScal;
+    double* grad   = v.grad + static_cast<size_t>(blockIdx.x % v.copies) * 3 * v.natom;
     const Real* Dt = static_cast<const Real*>(v.Dt);
     const Real* Da = static_cast<const Real*>(v.Da);
     const Real* Db = static_cast<const Real*>(v.Db);
 
-    unsigned long long m = sp.prims / sp.lanes;
-    m = m < 1 ? 1 : m;
+    const unsigned long long m = split_share(sp.prims, sp.lanes, sp.next != nullptr);
     unsigned long long round = 0, it = 0, end = 0;
     while (take_items(sp, items, (static_cast<unsigned long long>(blockIdx.x) * kGradWarps + wib) * NG + grp,
                       static_cast<unsigned long long>(gridDim.x) * kGradWarps * NG, false, gmask, grp * GS, nullptr, round, it, end))
@@ -142,7 +143,10 @@ __global__ void __launch_bounds__(32 * kGradWarps)
         {
             const int slc = static_cast<int>(it) & (S1 - 1), g = split_lanes(bra.npp * ket.npp, m, S1);
             if (slc >= g)
+            {
+                it |= S1 - 1; // on to the next quartet of the run
                 continue;
+            }
             pr = split_range(bra.npp, ket.npp, slc, g);
         }
         const int a0 = bra.ao1, b0 = bra.ao2, c0 = ket.ao1, d0 = ket.ao2;
@@ -375,10 +379,10 @@ __global__ void __launch_bounds__(32 * kGradWarps)
             const int tc = v.shell_atom[ket.sh1], td = v.shell_atom[ket.sh2];
             for (int x = 0; x < 3; ++x)
             {
-                atomicAdd(v.grad + 3 * ta + x, widen(gA[x]));
-                atomicAdd(v.grad + 3 * tb + x, widen(gB[x]));
-                atomicAdd(v.grad + 3 * tc + x, widen(gC[x]));
-                atomicAdd(v.grad + 3 * td + x, widen(-(gA[x] + gB[x] + gC[x])));
+                atomicAdd(grad + 3 * ta + x, widen(gA[x]));
+                atomicAdd(grad + 3 * tb + x, widen(gB[x]));
+                atomicAdd(grad + 3 * tc + x, widen(gC[x]));
+                atomicAdd(grad + 3 * td + x, widen(-(gA[x] + gB[x] + gC[x])));
             }
         }
         __syncwarp(gmask);
@@ -432,13 +436,13 @@ __global__ void __launch_bounds__(128)
     const unsigned long long items = ((n + 31) >> 5) * static_cast<unsigned long long>(S);
     if (static_cast<unsigned long long>(blockIdx.x) * 4 >= items)
         return;
-    unsigned long long m = sp.prims / sp.lanes;
-    m = m < 1 ? 1 : m;
+    const unsigned long long m = split_share(sp.prims, sp.lanes, sp.next != nullptr);
     stage_boys<Real, boys_slice_size<Real>()>(boys_slice, slice);
     const Real* __restrict__ tbf = static_cast<const Real*>(v.pptab[PCB]);
     const Real* __restrict__ tkf = static_cast<const Real*>(v.pptab[PCK]);
     const Real* __restrict__ tbg = static_cast<const Real*>(v.gtab[PCB]);
     const Real* __restrict__ tkg = static_cast<const Real*>(v.gtab[PCK]);
+    double* grad   = v.grad + static_cast<size_t>(blockIdx.x % v.copies) * 3 * v.natom;
     const Real* Dt = static_cast<const Real*>(v.Dt);
     const Real* Da = static_cast<const Real*>(v.Da);
     const Real* Db = static_cast<const Real*>(v.Db);
@@ -458,7 +462,10 @@ __global__ void __launch_bounds__(128)
             const Quartet w = list[q < n ? q : base];
             g = split_lanes(__reduce_max_sync(0xffffffffu, v.pairs[w.bra].npp * v.pairs[w.ket].npp), m, S);
             if (slc >= g)
+            {
+                it |= S - 1; // on to the next window of the run
                 continue;
+            }
             q = base + (g <= 32 ? slc * (32 / g) + lane / g : slc / (g / 32));
             r = g <= 32 ? lane % g : (slc % (g / 32)) * 32 + lane;
         }
@@ -728,8 +735,8 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
             for (int x = 0; x < 3; ++x)
             {
-                atomicAdd(v.grad + 3 * ta + x, widen(gA[x]));
-                atomicAdd(v.grad + 3 * tb + x, widen(gB[x]));
+                atomicAdd(grad + 3 * ta + x, widen(gA[x]));
+                atomicAdd(grad + 3 * tb + x, widen(gB[x]));
             }
         if (active)
         {
@@ -737,8 +744,8 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
             for (int x = 0; x < 3; ++x)
             {
-                atomicAdd(v.grad + 3 * tc + x, widen(gC[x]));
-                atomicAdd(v.grad + 3 * td + x, widen(gD[x]));
+                atomicAdd(grad + 3 * tc + x, widen(gC[x]));
+                atomicAdd(grad + 3 * td + x, widen(gD[x]));
             }
         }
     }

@@ -640,7 +640,9 @@ __device__ __forceinline__ void stage_boys(const Real* __restrict__ g, Real* s)
 // are summed before one of them digests.  G grows with the window's primitive count P until each lane
 // has at most m = max(1, prims / lanes) primitive quartets, `prims` being the whole list's primitive
 // quartets and `lanes` what fills the GPU: a long list (m above any P) runs one lane per quartet, as
-// before, and pays nothing.
+// before, and pays nothing.  A list of many waves, whose items go to whoever is free (`next`), splits eight
+// times finer, down to four primitive quartets a lane, so that its last items are an eighth of a warp's
+// share and not all of it.
 struct SplitArgs
 {
     int smax = 1;                             // warps per window at most, a power of two; 1: no split
@@ -653,6 +655,15 @@ struct SplitArgs
     unsigned long long prims = 0;             // the list's primitive quartets,
     const unsigned long long* prims_dev = nullptr; // or where they stand (a captured graph's lists)
 };
+
+// Primitive quartets a lane of a split list has at most.
+__host__ __device__ inline unsigned long long split_share(unsigned long long prims, unsigned lanes, bool queued)
+{
+    unsigned long long m = prims / lanes;
+    if (queued && m > 4)
+        m = m / 8 > 4 ? m / 8 : 4;
+    return m > 1 ? m : 1;
+}
 
 // Lanes per quartet for P primitive quartets at m a lane.
 __device__ __forceinline__ int split_lanes(int P, unsigned long long m, int smax)
@@ -795,16 +806,13 @@ __device__ __forceinline__ void class_body(const Quartet* __restrict__ list, uns
     const unsigned long long items = ((n + 31) >> 5) * static_cast<unsigned long long>(S);
     unsigned long long m = 0;
     if (kSplit && S > 1)
-    {
-        m = (sp.prims_dev ? *sp.prims_dev : sp.prims) / sp.lanes;
-        m = m < 1 ? 1 : m;
-    }
+        m = split_share(sp.prims_dev ? *sp.prims_dev : sp.prims, sp.lanes, sp.next != nullptr);
     // Warp-uniform iteration (every lane runs the same trip count, inactive lanes past the end), so that
-    // the digestion may sum the bra block over the warp.  With S >= 4 the four warps of a block are slices of
+    // the digestion may sum the bra block over the warp.  With S >= 64 the four warps of a block take slices of
     // one window, so that they may share a quartet (G = 64, 128): their branches on G are block-uniform.
     // Runs keep the windows of one bra pair together, whose rows of D and records are then found in L1.
     __shared__ unsigned long long box;
-    const bool by_block = S >= 4;
+    const bool by_block = S >= 64; // the four warps of a block share a quartet (G = 64, 128)
     unsigned long long round = 0, at = 0, end = 0;
     while (take_items(sp, by_block ? items / 4 : items, by_block ? blockIdx.x : blockIdx.x * 4ull + wib,
                       by_block ? gridDim.x : gridDim.x * 4ull, by_block, 0xffffffffu, 0, &box, round, at, end))
@@ -823,7 +831,11 @@ __device__ __forceinline__ void class_body(const Quartet* __restrict__ list, uns
             const Quartet w = list[q < n ? q : base];
             g = split_lanes(__reduce_max_sync(0xffffffffu, v.pairs[w.bra].npp * v.pairs[w.ket].npp), m, S);
             if (slc >= g)
+            {
+                if (!by_block)
+                    at |= S - 1; // on to the next window of the run
                 continue;
+            }
             q = base + (g <= 32 ? slc * (32 / g) + lane / g : slc / (g / 32));
             r = g <= 32 ? lane % g : (slc % (g / 32)) * 32 + lane;
         }
