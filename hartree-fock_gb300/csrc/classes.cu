@@ -1,7 +1,8 @@
-// Kernel instantiations and launchers of ONE shell-quartet class.  The build compiles this file three
-// times per class, -DHFG_QCLASS=<0..20> -DHFG_PART=<0..2>: part 0 the FP64 Fock kernels (and the form
-// mask), part 1 the FP32 Fock kernels, part 2 the gradient kernels, so that the 63 units compile in
-// parallel and the largest class does not serialise the build.
+// Kernel instantiations and launchers of ONE shell-quartet class.  The build compiles this file four
+// times per class, -DHFG_QCLASS=<0..20> -DHFG_PART=<0..3>: part 0 the RHF FP64 Fock kernels (with the store and
+// stored-integral kernels and the form mask), part 1 the FP32 Fock kernels, part 2 the gradient kernels, part 3
+// the UHF FP64 Fock kernels, so that the 84 units compile in parallel and the largest class does not
+// serialise the build.
 #include "engine.h"
 #include "eri_grad.cuh"
 #include "eri_group.cuh"
@@ -10,7 +11,7 @@
 #error "compile with -DHFG_QCLASS=<quartet class>"
 #endif
 #ifndef HFG_PART
-#error "compile with -DHFG_PART=<0: FP64 Fock kernels, 1: FP32 Fock kernels, 2: gradient kernels>"
+#error "compile with -DHFG_PART=<0: RHF FP64, 1: FP32, 2: gradient, 3: UHF FP64 kernels>"
 #endif
 
 namespace hfg
@@ -46,13 +47,13 @@ constexpr bool dual_form(bool fp32) { return fp32 && (QC == 11 || QC == 12 || QC
 // Ket-chunked thread form (FP32 d classes): ket components per thread, chosen so that R, G[HAB][CH] and
 // ERI[NAB][CH] stay in registers (HL + (HAB + NAB) * CH floats well below 255); 0 = not compiled.
 //   (dp|pp) (dp|ds): 3   (dp|dp): 2   (dd|ps) (dd|pp) (dd|ds) (dd|dp): 1
-// In FP64 (dp|pp) (dp|ds) (dp|dp): 3   (dd|ps) (dd|pp) (dd|ds): 1; what does not fit the registers spills to
-// L1, whose traffic (two wavefronts per warp and value) hides behind the FP64 pipe (16 SM cycles per warp
-// instruction).
+// In FP64 (dp|pp) (dp|ds) (dp|dp): 3   (dd|ps) (dd|pp) (dd|ds) (dd|dp): 1; what does not fit the registers
+// spills to L1, whose traffic (two wavefronts per warp and value) hides behind the FP64 pipe (16 SM cycles per
+// warp instruction).
 constexpr int chunk_width(bool fp32)
 {
     if (!fp32)
-        return (QC >= 12 && QC <= 14) ? 3 : (QC >= 16 && QC <= 18) ? 1 : 0;
+        return (QC >= 12 && QC <= 14) ? 3 : (QC >= 16 && QC <= 19) ? 1 : 0;
     return (QC == 12 || QC == 13) ? 3 : QC == 14 ? 2 : (QC >= 16 && QC <= 19) ? 1 : 0;
 }
 // The form a launch with form 0 runs (before or without autotuning): the chunked form where the tuner
@@ -284,10 +285,13 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
 #define HFG_CAT2(a, b) a##b
 #define HFG_CAT(a, b) HFG_CAT2(a, b)
 
-#if HFG_PART == 0
+#if HFG_PART == 3
+cudaError_t HFG_CAT(launch_class64u_, HFG_QCLASS)(const ClassLaunch& c) { return launch_t<double, true>(c); }
+#elif HFG_PART == 0
+cudaError_t HFG_CAT(launch_class64u_, HFG_QCLASS)(const ClassLaunch& c);
 cudaError_t HFG_CAT(launch_class64_, HFG_QCLASS)(const ClassLaunch& c)
 {
-    return c.uhf ? launch_t<double, true>(c) : launch_t<double, false>(c);
+    return c.uhf ? HFG_CAT(launch_class64u_, HFG_QCLASS)(c) : launch_t<double, false>(c);
 }
 
 cudaError_t HFG_CAT(launch_stored_, HFG_QCLASS)(const StoredLaunch& c)

@@ -641,8 +641,8 @@ __device__ __forceinline__ void stage_boys(const Real* __restrict__ g, Real* s)
 // has at most m = max(1, prims / lanes) primitive quartets, `prims` being the whole list's primitive
 // quartets and `lanes` what fills the GPU: a long list (m above any P) runs one lane per quartet, as
 // before, and pays nothing.  A list of many waves, whose items go to whoever is free (`next`), splits eight
-// times finer, down to four primitive quartets a lane, so that its last items are an eighth of a warp's
-// share and not all of it.
+// times finer, down to 32 primitive quartets a lane (every lane repeats the transform of its bra primitives and
+// joins the sum over lanes), so that its last items are an eighth of a lane's share and not all of it.
 struct SplitArgs
 {
     int smax = 1;                             // warps per window at most, a power of two; 1: no split
@@ -660,8 +660,8 @@ struct SplitArgs
 __host__ __device__ inline unsigned long long split_share(unsigned long long prims, unsigned lanes, bool queued)
 {
     unsigned long long m = prims / lanes;
-    if (queued && m > 4)
-        m = m / 8 > 4 ? m / 8 : 4;
+    if (queued && m > 32)
+        m = m / 8 > 32 ? m / 8 : 32;
     return m > 1 ? m : 1;
 }
 

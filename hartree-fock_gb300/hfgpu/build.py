@@ -57,7 +57,7 @@ def _units():
     units = []
     for c in range(NUM_CLASSES):
         src = os.path.join(CSRC, "classes.cu")
-        for part in range(3):  # FP64 Fock kernels, FP32 Fock kernels, gradient kernels
+        for part in range(4):  # RHF FP64 Fock kernels, FP32 Fock kernels, gradient kernels, UHF FP64 Fock kernels
             flags = NVCC_FLAGS + [f"-DHFG_QCLASS={c}", f"-DHFG_PART={part}"]
             units.append(("nvcc", src, flags, f"class{c:02d}p{part}", hdrs))
     for name in ("engine.cu", "dispatch.cu", "peak.cu", "boys_check.cu", "scf_device.cu", "onee.cu", "persistent.cu"):
