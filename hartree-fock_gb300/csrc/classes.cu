@@ -120,6 +120,24 @@ inline unsigned long long plan_items(SplitArgs& s, bool split, unsigned long lon
     return need < cap ? need : cap;
 }
 
+// Allows the kernel its shared memory and asks how many of its blocks an SM holds, once per engine (`slot`, zero
+// before): the two calls cost more host time than the launch, 72 times in a build of two waters.
+template <typename Kern> cudaError_t resident_blocks(Kern kern, int threads, size_t smem, int* slot, int& per_sm)
+{
+    if (slot != nullptr && *slot > 0)
+    {
+        per_sm = *slot;
+        return cudaSuccess;
+    }
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+    per_sm = per_sm > 0 ? per_sm : 1;
+    if (slot != nullptr && e == cudaSuccess)
+        *slot = per_sm;
+    return e;
+}
+
 // Resident blocks per SM a grid may take: the occupancy limit times the share, at least one.
 inline unsigned long long resident(int per_sm, float share)
 {
@@ -179,11 +197,8 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
         {
             auto kern         = jk_class_group_kernel<LA, LB, LC, LD, Real, UHF>;
             const size_t smem = slice_bytes;
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-            if (e != cudaSuccess)
-                return e;
-            int per_sm = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
+            int per_sm    = 0;
+            cudaError_t e = resident_blocks(kern, 128, smem, c.occ ? c.occ + kMaxChunks + 2 : nullptr, per_sm);
             if (e != cudaSuccess)
                 return e;
             const unsigned long long need = (c.count_host + 127) / 128; // 4 warps x 32-quartet windows
@@ -211,11 +226,8 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
                     auto kern         = jk_class_chunk_kernel<LA, LB, LC, LD, Real, UHF, k0, k1>;
                     SplitArgs sp = split_args<Real>(c);
                     const size_t smem = kFastBytes + (sizeof(Real) == 8 ? sizeof(Real) * split_scratch<LA, LB, k0, k1>() : 0);
-                    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-                    if (err != cudaSuccess)
-                        return;
                     int per_sm = 0;
-                    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
+                    err = resident_blocks(kern, 128, smem, c.occ ? c.occ + decltype(C)::value : nullptr, per_sm);
                     if (err != cudaSuccess)
                         return;
                     const unsigned long long grid =
@@ -240,11 +252,8 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
             using W             = WarpLayout<LA, LB, LC, LD, Real>;
             const size_t smem   = slice_bytes + sizeof(Real) * W::kPerWarp * kWarpKernelWarps;
             auto kern           = jk_class_warp_kernel<LA, LB, LC, LD, Real, UHF>;
-            cudaError_t e       = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-            if (e != cudaSuccess)
-                return e;
-            int per_sm = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarpKernelWarps, smem);
+            int per_sm    = 0;
+            cudaError_t e = resident_blocks(kern, 32 * kWarpKernelWarps, smem, c.occ ? c.occ + kMaxChunks + 1 : nullptr, per_sm);
             if (e != cudaSuccess)
                 return e;
             const unsigned long long need = (c.count_host + kWarpKernelWarps - 1) / kWarpKernelWarps;
@@ -262,11 +271,8 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
             auto kern           = jk_class_kernel<LA, LB, LC, LD, Real, UHF>;
             SplitArgs sp        = split_args<Real>(c);
             const size_t smem   = kFastBytes + (sizeof(Real) == 8 ? sizeof(Real) * split_scratch<LA, LB, 0, NCD>() : 0);
-            cudaError_t e       = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-            if (e != cudaSuccess)
-                return e;
-            int per_sm = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
+            int per_sm    = 0;
+            cudaError_t e = resident_blocks(kern, 128, smem, c.occ ? c.occ + kMaxChunks : nullptr, per_sm);
             if (e != cudaSuccess)
                 return e;
             const unsigned long long grid =
@@ -327,12 +333,13 @@ cudaError_t HFG_CAT(launch_class32_, HFG_QCLASS)(const ClassLaunch& c)
 #else
 namespace
 {
-// Thread-per-quartet gradient form where the per-thread arrays fit in registers (GradThread::kValues: at
-// most 72 doubles or 160 floats):
-//   FP64: (ss|ss) (ps|ss) (ps|ps) (pp|ss) (ds|ss);  FP32: also (pp|ps) (ds|ps) (dp|ss).
+// Thread-per-quartet gradient form: up to 300 values a thread (GradThread::kValues).  What does not fit the
+// registers spills to L1; the lane-group form keeps half its lanes idle in its dynamic index loops.
+//   FP64: every class up to (pp|ps), (ds|ps), (ds|pp), (ds|ds), (dp|ss), (dp|ps), (dd|ss) but (pp|pp);
+//   FP32: up to 160 values, and to 300 with d shells, which adds (ds|pp) (ds|ds) (dp|ps) (dd|ss).
 template <typename Real> constexpr bool grad_thread_form()
 {
-    return GradThread<LA, LB, LC, LD>::kValues <= (sizeof(Real) == 8 ? 300 : 160);
+    return GradThread<LA, LB, LC, LD>::kValues <= (sizeof(Real) == 8 || LA == 2 ? 300 : 160);
 }
 
 // The split of a gradient launch: `width` lanes work on one slice together.
@@ -351,11 +358,8 @@ template <typename Real> cudaError_t launch_grad_thread(const GradLaunch& c)
 {
     const size_t smem = sizeof(Real) * boys_slice_size<Real>();
     auto kern         = grad_thread_kernel<LA, LB, LC, LD, Real>;
-    cudaError_t e     = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess)
-        return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
+    int per_sm    = 0;
+    cudaError_t e = resident_blocks(kern, 128, smem, c.occ, per_sm);
     if (e != cudaSuccess)
         return e;
     SplitArgs sp                  = grad_split<Real>(c, 1);
@@ -377,11 +381,8 @@ template <typename Real> cudaError_t launch_grad_t(const GradLaunch& c)
     using W           = GradLayout<LA, LB, LC, LD>;
     const size_t smem = sizeof(Real) * (boys_slice_size<Real>() + W::kPerWarp * kGradWarps);
     auto kern         = grad_class_kernel<LA, LB, LC, LD, Real>;
-    cudaError_t e     = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess)
-        return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kGradWarps, smem);
+    int per_sm    = 0;
+    cudaError_t e = resident_blocks(kern, 32 * kGradWarps, smem, c.occ + 1, per_sm);
     if (e != cudaSuccess)
         return e;
     constexpr unsigned per_block = kGradWarps * (32 / W::kGroup); // quartets in flight per block

@@ -217,6 +217,8 @@ struct hfg_engine
     hfg::DevBuf<float4> d_cls_diff[hfg::kNumPairClasses]; // most diffuse primitive pair of each sorted position: P, p
     hfg::DevBuf<unsigned> d_bra_cnt[hfg::kNumQuartetClasses];            // per bra pair: survivors (fp64, fp32)
     hfg::DevBuf<unsigned> d_bra_near[hfg::kNumQuartetClasses];           // per bra pair: near FP64 survivors
+    hfg::DevBuf<unsigned> d_group_off[hfg::kNumQuartetClasses];          // per bra pair: first candidate group
+    hfg::DevBuf<uint4> d_groups[hfg::kNumQuartetClasses];                // survivor bits of 32 candidates each
     hfg::DevBuf<unsigned long long> d_bra_off[hfg::kNumQuartetClasses];  // per bra pair: list offsets
 
     // Quartet lists (capacity for the Schwartz threshold they were sized for).
@@ -224,6 +226,9 @@ struct hfg_engine
     unsigned long long cap[hfg::kNumQuartetClasses] {};
     bool cap_mixed = false;
     hfg::DevBuf<hfg::Quartet> d_list[hfg::kNumQuartetClasses][2];
+    // Resident blocks of the class kernels (ClassLaunch::occ, GradLaunch::occ), asked once.
+    int occ[2][2][hfg::kNumQuartetClasses][hfg::kOccSlots] {};
+    int occ_grad[2][hfg::kNumQuartetClasses][2] {};
     hfg::DevBuf<unsigned long long> d_next;   // item counters [prec][qclass][kMaxChunks] of the class launches
     hfg::DevBuf<unsigned long long> d_counts; // [qclass][prec] quartets, then [qclass][prec] prim quartets, then overflow
     std::vector<unsigned long long> h_counts;
@@ -395,7 +400,9 @@ struct ClassBuild
     const float4* diff2;
     unsigned* bra_cnt;             // [n1][2]
     unsigned* bra_near;            // [n1] FP64 survivors that are not far (below)
-    unsigned long long* bra_off;   // [n1][2] exclusive offsets (pass 1)
+    unsigned long long* bra_off;   // [n1][2] exclusive offsets
+    const unsigned* group_off;     // [n1 + 1] first candidate group of every bra pair
+    uint4* groups;                 // first ket position; near FP64, far FP64 and FP32 survivors of 32 candidates (bits)
     Quartet* out64;
     Quartet* out32;
     unsigned long long cap; // list capacity (the Schwartz-only count): writes beyond it are dropped
@@ -422,23 +429,24 @@ struct BuildArgs
     double sthr, dthr;
     float cutoff;
     int mixed;
-    int pass;                   // 0: count per bra pair, 1: write at the scanned offsets
     unsigned long long* counts; // [2 qc + prec] quartets, then [2 qc + prec] primitive quartets
 };
 
-// Survival list of one quartet class in two deterministic passes, one warp per bra pair.  Ket
-// candidates are visited segment by segment (segments of equal primitive-pair count, Q descending
-// inside each), and inside a segment only the Schwartz prefix Q_i*Q_j >= thr is tested (the product is
-// monotone in Q_j); the density predicate is that of SCF.cpp:610-623.  Pass 0 counts survivors per
-// bra pair and precision, pass 1 writes them at scanned offsets in candidate order, so the list is
-// ordered by bra pair and, inside a bra pair, by ket primitive count: a warp of the class kernels sees
-// quartets of equal primitive counts.  FP32 / FP64 split by the quartet bound Q_i Q_j max|dD|.
+// Survival lists in two deterministic passes, one warp per bra pair.  Ket candidates are visited segment by
+// segment (segments of equal primitive-pair count, Q descending inside each), and inside a segment only the
+// Schwartz prefix Q_i*Q_j >= thr is tested (the product is monotone in Q_j); the density predicate is that of
+// SCF.cpp:610-623.  This pass tests: it leaves one record of survivor bits per group of 32 candidates and
+// the counts per bra pair and precision; write_lists_kernel expands the records at the scanned offsets.
+// (Testing in both passes reads the shell maxima of every candidate twice, eight scattered values each: 34.7 ms
+// of a mixed (H2O)_64 build.)  The list is ordered by bra pair and, inside a bra pair, by ket primitive
+// count: a warp of the class kernels sees quartets of equal primitive counts.  FP32 / FP64 split by the
+// quartet bound Q_i Q_j max|dD|.
 // The FP64 survivors of a bra pair are written in two parts, near and far: far is where the most diffuse
 // primitive quartet (and so, but for the shift between primitive centres, every one) has T > 30, the
 // asymptotic branch of the Boys function.  A warp with both kinds runs both branches, each with part of
 // its lanes: (ps|ss) of (H2O)_16 ran its FP64 instructions with 20.9 of 32 lanes.  FP32 survivors keep one
 // part, whose order their FP32 sums follow.
-__global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __grid_constant__ BuildArgs b)
+__global__ void __launch_bounds__(32 * kBuildWarps) test_lists_kernel(const __grid_constant__ BuildArgs b)
 {
     int ci = 0;
     while (ci + 1 < b.ncls && b.cls[ci + 1].first_block <= static_cast<int>(blockIdx.x)) ++ci;
@@ -464,11 +472,10 @@ __global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __g
     const long long ra = so + (long long)sa * ns, rb2 = so + (long long)sb * ns;
     const float Qfi = a.Qf1[i];
     const float4 di = a.diff1[i];
-    unsigned c64 = 0, c32 = 0, cfar = 0; // c64: near survivors in pass 1
-    const unsigned near64 = b.pass ? a.bra_near[i] : 0u;
+    unsigned c64 = 0, c32 = 0, cfar = 0; // c64: near
+    unsigned group = a.group_off[i];
+    const unsigned last = a.group_off[i + 1]; // the host counted the same groups
     unsigned long long p64 = 0, p32 = 0;
-    const unsigned long long o64 = b.pass ? a.bra_off[2 * i] : 0ull;
-    const unsigned long long o32 = b.pass ? a.bra_off[2 * i + 1] : 0ull;
     for (int sidx = ms.x; sidx < ms.y; ++sidx)
     {
         const int4 seg = a.seg2[sidx];
@@ -476,14 +483,15 @@ __global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __g
         const int je = a.same_class ? min(seg.y, i + 1) : seg.y;
         if (jb >= je)
             continue;
+        // First position of the segment below the threshold, 32 probes at a time.
         int lo = jb, hi = je;
         while (lo < hi)
         {
-            const int mid = (lo + hi) >> 1;
-            if (Qi * a.Q2[mid] < b.sthr)
-                hi = mid;
-            else
-                lo = mid + 1;
+            const int step  = (hi - lo + 31) >> 5, at = lo + lane * step;
+            const unsigned m = __ballot_sync(0xffffffffu, at >= hi || Qi * a.Q2[at] < b.sthr);
+            const int f      = m ? __ffs(static_cast<int>(m)) - 1 : 32; // the first probe below
+            hi = min(hi, lo + f * step);
+            lo = f > 0 ? lo + (f - 1) * step + 1 : lo;
         }
         const int jend = lo;
         for (int base = jb; base < jend; base += 32)
@@ -517,17 +525,9 @@ __global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __g
             const unsigned mfar = __ballot_sync(0xffffffffu, far);
             const unsigned m64  = __ballot_sync(0xffffffffu, s64 && !far);
             const unsigned m32  = __ballot_sync(0xffffffffu, s32);
-            const unsigned lt   = (1u << lane) - 1u;
-            if (b.pass)
-            {
-                const Quartet qv {static_cast<uint32_t>(a.base1 + i), static_cast<uint32_t>(a.base2 + j)};
-                const unsigned long long w64 = o64 + (far ? near64 + cfar + __popc(mfar & lt) : c64 + __popc(m64 & lt)),
-                                         w32 = o32 + c32 + __popc(m32 & lt);
-                if (s64 && w64 < a.cap)
-                    a.out64[w64] = qv;
-                if (s32 && w32 < a.cap)
-                    a.out32[w32] = qv;
-            }
+            if (lane == 0 && group < last)
+                a.groups[group] = make_uint4(static_cast<unsigned>(base), m64, mfar, m32);
+            ++group;
             c64 += __popc(m64);
             cfar += __popc(mfar);
             c32 += __popc(m32);
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __g
             p32 += pp * __popc(m32);
         }
     }
-    if (b.pass == 0 && lane == 0)
+    if (lane == 0)
     {
         a.bra_near[i]        = c64;
         a.bra_cnt[2 * i]     = c64 + cfar;
@@ -546,6 +546,42 @@ __global__ void __launch_bounds__(32 * kBuildWarps) build_lists_kernel(const __g
             atomicAdd(prims, p64);
         if (p32)
             atomicAdd(prims + 1, p32);
+    }
+}
+
+// Writes the lists from the records of test_lists_kernel, one warp per bra pair.
+__global__ void __launch_bounds__(32 * kBuildWarps) write_lists_kernel(const __grid_constant__ BuildArgs b)
+{
+    int ci = 0;
+    while (ci + 1 < b.ncls && b.cls[ci + 1].first_block <= static_cast<int>(blockIdx.x)) ++ci;
+    const ClassBuild& a = b.cls[ci];
+    const int lane = threadIdx.x & 31;
+    const int i    = (static_cast<int>(blockIdx.x) - a.first_block) * kBuildWarps + (threadIdx.x >> 5);
+    if (i >= a.n1)
+        return;
+    unsigned long long w64 = a.bra_off[2 * i], w32 = a.bra_off[2 * i + 1], wfar = w64 + a.bra_near[i];
+    const unsigned last = a.group_off[i + 1], lt = (1u << lane) - 1u;
+    for (unsigned g0 = a.group_off[i]; g0 < last; g0 += 32)
+    {
+        const uint4 own = g0 + lane < last ? a.groups[g0 + lane] : make_uint4(0u, 0u, 0u, 0u);
+        unsigned some   = __ballot_sync(0xffffffffu, (own.y | own.z | own.w) != 0u);
+        for (; some; some &= some - 1)
+        {
+            const int k          = __ffs(static_cast<int>(some)) - 1;
+            const unsigned j     = __shfl_sync(0xffffffffu, own.x, k) + lane;
+            const unsigned mnear = __shfl_sync(0xffffffffu, own.y, k), mfar = __shfl_sync(0xffffffffu, own.z, k),
+                           m32   = __shfl_sync(0xffffffffu, own.w, k);
+            const Quartet qv {static_cast<uint32_t>(a.base1 + i), static_cast<uint32_t>(a.base2) + j};
+            auto put = [&](Quartet* out, unsigned long long& w, unsigned m) {
+                const unsigned long long at = w + __popc(m & lt);
+                if (((m >> lane) & 1u) && at < a.cap)
+                    out[at] = qv;
+                w += __popc(m);
+            };
+            put(a.out64, w64, mnear);
+            put(a.out64, wfar, mfar);
+            put(a.out32, w32, m32);
+        }
     }
 }
 
@@ -1272,7 +1308,9 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
         for (int P2 = 0; P2 <= P1; ++P2)
         {
             const int qc = quartet_class(P1, P2);
-            unsigned long long c = 0;
+            unsigned long long c = 0, groups = 0;
+            std::vector<unsigned> group_off(1, 0u);
+            group_off.reserve(e->cls_ids[P1].size() + 1);
             for (size_t i = 0; i < e->cls_ids[P1].size(); ++i)
             {
                 const int mol = e->pairs[e->cls_ids[P1][i]].mol;
@@ -1280,9 +1318,17 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
                 for (int sg = ms.x; sg < ms.y; ++sg)
                 {
                     const int4& seg = e->cls_seg[P2][sg];
-                    c += static_cast<unsigned long long>(std::max(0, prefix_end(e, P1, P2, i, seg, sthr) - seg.x));
+                    const int len   = std::max(0, prefix_end(e, P1, P2, i, seg, sthr) - seg.x);
+                    c += static_cast<unsigned long long>(len);
+                    groups += static_cast<unsigned long long>((len + 31) / 32);
                 }
+                if (groups > 0xffffffe0ull)
+                    throw HfgError(HFG_ERR_OVERFLOW, "fock: too many candidates in one quartet class");
+                group_off.push_back(static_cast<unsigned>(groups));
             }
+            e->d_group_off[qc].upload(group_off, e->stream);
+            HFG_CUDA(cudaStreamSynchronize(e->stream)); // group_off dies here
+            e->d_groups[qc].alloc(std::max<unsigned long long>(groups, 1));
             e->cap[qc] = c;
             e->d_list[qc][0].alloc(std::max<unsigned long long>(c, 1));
             if (mixed)
@@ -1342,6 +1388,8 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
         c.Qf2         = e->d_cls_Qf[P2].p;
         c.bra_cnt     = e->d_bra_cnt[qc].p;
         c.bra_near    = e->d_bra_near[qc].p;
+        c.group_off   = e->d_group_off[qc].p;
+        c.groups      = e->d_groups[qc].p;
         c.diff1       = e->d_cls_diff[P1].p;
         c.diff2       = e->d_cls_diff[P2].p;
         c.bra_off     = e->d_bra_off[qc].p;
@@ -1365,10 +1413,9 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
     int launches = 0;
     if (a.ncls > 0)
     {
-        build_lists_kernel<<<static_cast<unsigned>(blocks), 32 * kBuildWarps, 0, s>>>(a);
+        test_lists_kernel<<<static_cast<unsigned>(blocks), 32 * kBuildWarps, 0, s>>>(a);
         scan_lists_kernel<<<static_cast<unsigned>(a.ncls), kScanBlock, 0, s>>>(a);
-        a.pass = 1;
-        build_lists_kernel<<<static_cast<unsigned>(blocks), 32 * kBuildWarps, 0, s>>>(a);
+        write_lists_kernel<<<static_cast<unsigned>(blocks), 32 * kBuildWarps, 0, s>>>(a);
         HFG_CUDA(cudaGetLastError());
         launches = 3;
     }
@@ -1641,6 +1688,7 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             c.prims_dev  = e->d_counts.p + 2 * kNumQuartetClasses + 2 * qc + prec;
             c.prims      = prims;
             c.next       = e->d_next.p + (prec * kNumQuartetClasses + qc) * kMaxChunks;
+            c.occ        = e->occ[prec][uhf ? 1 : 0][qc];
             if (graph)
             {
                 const int set  = e->form_set[qc][prec];
@@ -2262,7 +2310,7 @@ static double gradient_two_electron(hfg_engine* e, const std::vector<int>& shell
             const void* slice = prec ? static_cast<const void*>(e->d_boys32[L + 1].p) : e->d_boysf[L + 1].p;
             GradLaunch g {e->d_list[qc][prec].p, n, v[prec], slice, e->d_tables.p, pass == 1 ? side.next() : side.own,
                           e->num_sms, prec == 1, e->grad_group_only, prims, max_prims(e, P1, P2, true),
-                          e->d_next.p + (prec * kNumQuartetClasses + qc) * kMaxChunks};
+                          e->d_next.p + (prec * kNumQuartetClasses + qc) * kMaxChunks, e->occ_grad[prec][qc]};
             HFG_CUDA(launch_grad(qc, g));
         }
         side.join();

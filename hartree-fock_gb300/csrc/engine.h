@@ -12,6 +12,7 @@
 namespace hfg
 {
 constexpr int kMaxChunks = 18; // launches of one class in the chunk form at most
+constexpr int kOccSlots  = kMaxChunks + 3; // one per chunk, then the thread, warp and group forms
 
 // Launches the class kernel of one quartet class for one list.
 struct ClassLaunch
@@ -35,6 +36,7 @@ struct ClassLaunch
     const unsigned long long* prims_dev = nullptr;
     int pmax = 1;
     unsigned long long* next = nullptr; // kMaxChunks item counters (SplitArgs::next), or null: static order
+    int* occ = nullptr; // kOccSlots resident-block counts of the class's kernels, 0: not asked yet (or null)
     float share = 1.f; // fraction of the resident blocks per SM the grid may take (concurrent precisions)
 };
 // Kernel forms of a class kernel (eri_jk.cuh, eri_warp.cuh, eri_group.cuh).
@@ -78,6 +80,7 @@ struct GradLaunch
     unsigned long long prims; // as in ClassLaunch, for the split of short lists
     int pmax;
     unsigned long long* next; // one item counter, as in ClassLaunch
+    int* occ;                 // resident-block counts of the thread and the lane-group kernel
 };
 cudaError_t launch_grad(int qclass, const GradLaunch& L);
 
