@@ -159,38 +159,42 @@ constexpr double exp_coefficient(int k)
 }
 template <int K> constexpr double kExpCoefficient = exp_coefficient(K);
 
-// Host: the BoysFast slice of total angular momentum L, row-major [point][kRow].
-inline std::vector<double> boys_fast_slice_host(int L)
+// Host: the BoysFast slices of total angular momentum 0 .. l_max, each row-major [point][kRow].
+inline std::vector<std::vector<double>> boys_fast_slices_host(int l_max)
 {
     using G               = BoysFast;
     constexpr int kTaylor = 14;
-    std::vector<double> out(static_cast<size_t>(G::kPoints) * G::kRow);
+    std::vector<std::vector<double>> out(l_max + 1, std::vector<double>(static_cast<size_t>(G::kPoints) * G::kRow));
     double eco[kTaylor][kTaylor] {}; // what economising moves from coefficient k to the lower ones
     for (int k = G::kTerms; k < kTaylor; ++k)
     {
         eco[k][k] = 1.0;
         economise(eco[k], kTaylor, G::kTerms, G::kStep / 2);
     }
+    std::vector<long double> F(l_max + kTaylor);
     for (int i = 0; i < G::kPoints; ++i)
     {
-        // The orders from the highest by the downward recursion, then the Taylor coefficients F_{L+k} / k!.
+        // All orders from the highest by the downward recursion (one series per point: long double is slow software
+        // on some hosts), then per slice the Taylor coefficients F_{L+k} / k!.
         const long double Ti = i * static_cast<long double>(G::kStep), e = std::exp(-Ti);
-        long double c[kTaylor], kfact = 1.0L;
-        c[kTaylor - 1] = boys_series_host(L + kTaylor - 1, Ti);
-        for (int k = kTaylor - 1; k > 0; --k) c[k - 1] = (2 * Ti * c[k] + e) / (2 * (L + k) - 1);
-        for (int k = 2; k < kTaylor; ++k)
+        const int top = l_max + kTaylor - 1;
+        F[top]        = boys_series_host(top, Ti);
+        for (int m = top; m > 0; --m) F[m - 1] = (2 * Ti * F[m] + e) / (2 * m - 1);
+        for (int L = 0; L <= l_max; ++L)
         {
-            kfact *= k;
-            c[k] /= kfact;
+            double* row = &out[L][static_cast<size_t>(i) * G::kRow];
+            double moved[G::kTerms] {};
+            for (int k = kTaylor - 1; k >= G::kTerms; --k)
+                for (int j = 0; j < G::kTerms; ++j) moved[j] += static_cast<double>(F[L + k]) * inv_fact(k) * eco[k][j];
+            long double kfact = 1.0L;
+            for (int j = 0; j < G::kTerms; ++j)
+            {
+                if (j > 1)
+                    kfact *= j;
+                row[j] = static_cast<double>(F[L + j] / kfact + moved[j]);
+            }
+            row[G::kTerms] = static_cast<double>(e);
         }
-        double* row = &out[static_cast<size_t>(i) * G::kRow];
-        for (int j = 0; j < G::kTerms; ++j)
-        {
-            double moved = 0.0;
-            for (int k = kTaylor - 1; k >= G::kTerms; --k) moved += static_cast<double>(c[k]) * eco[k][j];
-            row[j] = static_cast<double>(c[j] + moved);
-        }
-        row[G::kTerms] = static_cast<double>(e);
     }
     return out;
 }

@@ -93,6 +93,8 @@ template <typename T> struct DevBuf
     }
 };
 
+constexpr int kSideStreams = 8; // per precision
+
 struct MolInfo
 {
     int nshells, nao;
@@ -124,11 +126,11 @@ struct hfg_engine
     // ev2: fork, join, FP32 start, FP32 end.
     cudaStream_t stream2 = nullptr;
     cudaEvent_t ev2[4] {};
-    // Short lists (a class kernel that cannot fill the GPU by itself) run side by side on side[precision][0..3],
+    // Short lists (a class kernel that cannot fill the GPU by itself) run side by side on side[precision][0..7],
     // forked from and joined to the precision's own stream: a small molecule has up to 21 of them per
     // precision, each as long as its longest quartet.
-    cudaStream_t side[2][4] {};
-    cudaEvent_t ev_side[2][5] {}; // fork, then the end of each side stream
+    cudaStream_t side[2][hfg::kSideStreams] {};
+    cudaEvent_t ev_side[2][hfg::kSideStreams + 1] {}; // fork, then the end of each side stream
     bool overlap = true;
     float overlap_share = 1.0f;   // FP64 class kernels' grids
     float overlap_share32 = 1.0f; // FP32 class kernels' grids
@@ -205,7 +207,8 @@ struct hfg_engine
     bool have_Q = false;
     std::vector<int> cls_ids[hfg::kNumPairClasses];
     std::vector<double> cls_Q[hfg::kNumPairClasses];
-    // Segments of equal primitive-pair count: x = begin, y = end (positions in the class list), z = npp.
+    // Segments of equal primitive-pair count: x = begin, y = end (positions in the class list), z = npp, w = bucket
+    // of z among the class's counts.
     std::vector<int4> cls_seg[hfg::kNumPairClasses];
     std::vector<int2> cls_molseg[hfg::kNumPairClasses]; // per molecule: [first, end) segment
     hfg::DevBuf<int> d_cls_ids[hfg::kNumPairClasses];
@@ -215,11 +218,11 @@ struct hfg_engine
     hfg::DevBuf<int2> d_cls_sh[hfg::kNumPairClasses]; // (sh1, sh2) of each sorted position
     hfg::DevBuf<int2> d_cls_molseg[hfg::kNumPairClasses];
     hfg::DevBuf<float4> d_cls_diff[hfg::kNumPairClasses]; // most diffuse primitive pair of each sorted position: P, p
-    hfg::DevBuf<unsigned> d_bra_cnt[hfg::kNumQuartetClasses];            // per bra pair: survivors (fp64, fp32)
-    hfg::DevBuf<unsigned> d_bra_near[hfg::kNumQuartetClasses];           // per bra pair: near FP64 survivors
+    hfg::DevBuf<unsigned> d_bra_cnt[hfg::kNumQuartetClasses];            // per sequence and bra pair: survivors
+    hfg::DevBuf<unsigned long long> d_seq_tot;                           // per class and sequence: length
     hfg::DevBuf<unsigned> d_group_off[hfg::kNumQuartetClasses];          // per bra pair: first candidate group
     hfg::DevBuf<uint4> d_groups[hfg::kNumQuartetClasses];                // survivor bits of 32 candidates each
-    hfg::DevBuf<unsigned long long> d_bra_off[hfg::kNumQuartetClasses];  // per bra pair: list offsets
+    hfg::DevBuf<unsigned long long> d_bra_off[hfg::kNumQuartetClasses];  // per sequence and bra pair: offsets
 
     // Quartet lists (capacity for the Schwartz threshold they were sized for).
     double cap_thr = -1.0;
@@ -398,11 +401,13 @@ struct ClassBuild
     const int2* molseg2; // per molecule: ket segment range
     const float4* diff1; // per position: centre and exponent p of the pair's most diffuse primitive pair
     const float4* diff2;
-    unsigned* bra_cnt;             // [n1][2]
-    unsigned* bra_near;            // [n1] FP64 survivors that are not far (below)
-    unsigned long long* bra_off;   // [n1][2] exclusive offsets
+    // Sequences of the class: the FP64 keys (ket bucket, near or far) in list order, then the FP32 list.
+    unsigned* bra_cnt;             // [kListSeqs][n1] survivors per bra pair
+    unsigned long long* bra_off;   // [kListSeqs][n1] exclusive offsets inside the sequence
+    unsigned long long* seq_tot;   // [kListSeqs] lengths
     const unsigned* group_off;     // [n1 + 1] first candidate group of every bra pair
-    uint4* groups;                 // first ket position; near FP64, far FP64 and FP32 survivors of 32 candidates (bits)
+    uint4* groups;                 // first ket position | ket bucket << 28; near FP64, far FP64 and FP32 survivors of
+                                   // 32 candidates (bits)
     Quartet* out64;
     Quartet* out32;
     unsigned long long cap; // list capacity (the Schwartz-only count): writes beyond it are dropped
@@ -413,6 +418,7 @@ struct ClassBuild
     int same_class;
 };
 constexpr int kBuildWarps = 4;
+constexpr int kListBuckets = 8, kListKeys = 2 * kListBuckets, kListSeqs = kListKeys + 1;
 
 // All classes of a build, worked through by one launch per pass: 21 launches a pass, each with its own ramp
 // and tail, took 0.12 of the 0.2 ms that the lists of one water cost.
@@ -429,6 +435,7 @@ struct BuildArgs
     double sthr, dthr;
     float cutoff;
     int mixed;
+    int keyed; // order the FP64 lists by key (else by bra pair alone)
     unsigned long long* counts; // [2 qc + prec] quartets, then [2 qc + prec] primitive quartets
 };
 
@@ -438,14 +445,17 @@ struct BuildArgs
 // SCF.cpp:610-623.  This pass tests: it leaves one record of survivor bits per group of 32 candidates and
 // the counts per bra pair and precision; write_lists_kernel expands the records at the scanned offsets.
 // (Testing in both passes reads the shell maxima of every candidate twice, eight scattered values each: 34.7 ms
-// of a mixed (H2O)_64 build.)  The list is ordered by bra pair and, inside a bra pair, by ket primitive
-// count: a warp of the class kernels sees quartets of equal primitive counts.  FP32 / FP64 split by the
-// quartet bound Q_i Q_j max|dD|.
-// The FP64 survivors of a bra pair are written in two parts, near and far: far is where the most diffuse
-// primitive quartet (and so, but for the shift between primitive centres, every one) has T > 30, the
-// asymptotic branch of the Boys function.  A warp with both kinds runs both branches, each with part of
-// its lanes: (ps|ss) of (H2O)_16 ran its FP64 instructions with 20.9 of 32 lanes.  FP32 survivors keep one
-// part, whose order their FP32 sums follow.
+// of a mixed (H2O)_64 build.)  FP32 / FP64 split by the quartet bound Q_i Q_j max|dD|.
+//
+// An FP32 list is ordered by bra pair and, inside a bra pair, by ket primitive count; its order decides how FP32
+// sums round and stays.  An FP64 list is ordered by key first, then by bra pair, so that the 32 quartets of a
+// warp do the same work even where a bra pair has few kets:
+//   * the bucket of the ket's primitive count (the counts of the class, dealt to eight buckets, largest first);
+//   * near or far: far is where the most diffuse primitive quartet (and so, but for the shift between primitive
+//     centres, every one) has T > 30, the asymptotic branch of the Boys function; a warp with both kinds
+//     runs both branches, each with part of its lanes.
+// Ordered by bra pair alone, (ps|ss) of (H2O)_16 ran its FP64 instructions with 20.7 of 32 lanes, and with the
+// near and far parts of each bra pair apart with 24.6.
 __global__ void __launch_bounds__(32 * kBuildWarps) test_lists_kernel(const __grid_constant__ BuildArgs b)
 {
     int ci = 0;
@@ -472,7 +482,12 @@ __global__ void __launch_bounds__(32 * kBuildWarps) test_lists_kernel(const __gr
     const long long ra = so + (long long)sa * ns, rb2 = so + (long long)sb * ns;
     const float Qfi = a.Qf1[i];
     const float4 di = a.diff1[i];
-    unsigned c64 = 0, c32 = 0, cfar = 0; // c64: near
+    __shared__ unsigned counts_s[kBuildWarps][kListKeys];
+    unsigned* keys = counts_s[threadIdx.x >> 5];
+    if (lane < kListKeys)
+        keys[lane] = 0u;
+    __syncwarp();
+    unsigned c32 = 0;
     unsigned group = a.group_off[i];
     const unsigned last = a.group_off[i + 1]; // the host counted the same groups
     unsigned long long p64 = 0, p32 = 0;
@@ -516,7 +531,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) test_lists_kernel(const __gr
                 }
             }
             bool far = false;
-            if (s64)
+            if (s64 && b.keyed)
             {
                 const float4 dj = a.diff2[j];
                 const float x = di.x - dj.x, y = di.y - dj.y, z = di.z - dj.z;
@@ -525,22 +540,26 @@ __global__ void __launch_bounds__(32 * kBuildWarps) test_lists_kernel(const __gr
             const unsigned mfar = __ballot_sync(0xffffffffu, far);
             const unsigned m64  = __ballot_sync(0xffffffffu, s64 && !far);
             const unsigned m32  = __ballot_sync(0xffffffffu, s32);
-            if (lane == 0 && group < last)
-                a.groups[group] = make_uint4(static_cast<unsigned>(base), m64, mfar, m32);
+            const unsigned bucket = b.keyed ? static_cast<unsigned>(seg.w) : 0u;
+            if (lane == 0)
+            {
+                if (group < last)
+                    a.groups[group] = make_uint4(static_cast<unsigned>(base) | bucket << 28, m64, mfar, m32);
+                keys[2 * bucket] += __popc(m64);
+                keys[2 * bucket + 1] += __popc(mfar);
+            }
             ++group;
-            c64 += __popc(m64);
-            cfar += __popc(mfar);
             c32 += __popc(m32);
             const unsigned long long pp = (unsigned long long)pi.npp * seg.z;
             p64 += pp * (__popc(m64) + __popc(mfar));
             p32 += pp * __popc(m32);
         }
     }
+    __syncwarp();
+    if (lane < kListSeqs)
+        a.bra_cnt[static_cast<size_t>(lane) * a.n1 + i] = lane < kListKeys ? keys[lane] : c32;
     if (lane == 0)
     {
-        a.bra_near[i]        = c64;
-        a.bra_cnt[2 * i]     = c64 + cfar;
-        a.bra_cnt[2 * i + 1] = c32;
         unsigned long long* prims = b.counts + 2 * kNumQuartetClasses + 2 * a.qc;
         if (p64)
             atomicAdd(prims, p64);
@@ -559,7 +578,17 @@ __global__ void __launch_bounds__(32 * kBuildWarps) write_lists_kernel(const __g
     const int i    = (static_cast<int>(blockIdx.x) - a.first_block) * kBuildWarps + (threadIdx.x >> 5);
     if (i >= a.n1)
         return;
-    unsigned long long w64 = a.bra_off[2 * i], w32 = a.bra_off[2 * i + 1], wfar = w64 + a.bra_near[i];
+    // Lane k < kListKeys keeps the place of key k, lane kListKeys that of the FP32 list.
+    unsigned long long place = 0, before = lane < kListKeys ? a.seq_tot[lane] : 0ull;
+    const unsigned long long own_tot = before;
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o)
+            before += y;
+    }
+    if (lane < kListSeqs)
+        place = a.bra_off[static_cast<size_t>(lane) * a.n1 + i] + (lane < kListKeys ? before - own_tot : 0ull);
     const unsigned last = a.group_off[i + 1], lt = (1u << lane) - 1u;
     for (unsigned g0 = a.group_off[i]; g0 < last; g0 += 32)
     {
@@ -568,91 +597,90 @@ __global__ void __launch_bounds__(32 * kBuildWarps) write_lists_kernel(const __g
         for (; some; some &= some - 1)
         {
             const int k          = __ffs(static_cast<int>(some)) - 1;
-            const unsigned j     = __shfl_sync(0xffffffffu, own.x, k) + lane;
+            const unsigned x     = __shfl_sync(0xffffffffu, own.x, k), j = (x & 0x0fffffffu) + lane;
+            const int key        = 2 * static_cast<int>(x >> 28);
             const unsigned mnear = __shfl_sync(0xffffffffu, own.y, k), mfar = __shfl_sync(0xffffffffu, own.z, k),
                            m32   = __shfl_sync(0xffffffffu, own.w, k);
             const Quartet qv {static_cast<uint32_t>(a.base1 + i), static_cast<uint32_t>(a.base2) + j};
-            auto put = [&](Quartet* out, unsigned long long& w, unsigned m) {
-                const unsigned long long at = w + __popc(m & lt);
+            auto put = [&](Quartet* out, int seq, unsigned m) {
+                const unsigned long long at = __shfl_sync(0xffffffffu, place, seq) + __popc(m & lt);
                 if (((m >> lane) & 1u) && at < a.cap)
                     out[at] = qv;
-                w += __popc(m);
+                if (lane == seq)
+                    place += __popc(m);
             };
-            put(a.out64, w64, mnear);
-            put(a.out64, wfar, mfar);
-            put(a.out32, w32, m32);
+            if (mnear)
+                put(a.out64, key, mnear);
+            if (mfar)
+                put(a.out64, key + 1, mfar);
+            if (m32)
+                put(a.out32, kListKeys, m32);
         }
     }
 }
 
-// Exclusive scan of the per-bra counts (two interleaved sequences, fp64 and fp32), one block per class: the
-// block walks the class's bra pairs kScanBlock * kScanItems at a time with a running total, and leaves
-// the grand totals in counts[2 qc], counts[2 qc + 1] (the class kernels' list lengths).  One block is enough:
-// the longest class of (H2O)_64 (115k bra pairs) is 29 rounds.
+// Exclusive scan of the per-bra counts, one block per class and sequence: the block walks the class's bra pairs
+// kScanBlock * kScanItems at a time with a running total, and adds the total to counts[2 qc] (FP64) or
+// counts[2 qc + 1] (the class kernels' list lengths).  The longest class of (H2O)_64 (115k bra pairs) is 29 rounds.
 constexpr int kScanBlock = 1024, kScanItems = 4;
 __global__ void __launch_bounds__(kScanBlock) scan_lists_kernel(const __grid_constant__ BuildArgs b)
 {
-    const ClassBuild& a = b.cls[blockIdx.x];
-    __shared__ unsigned long long warp_tot[2][32];
+    const ClassBuild& a                     = b.cls[blockIdx.x / kListSeqs];
+    const int seq                           = blockIdx.x % kListSeqs;
+    const unsigned* __restrict__ cnt        = a.bra_cnt + static_cast<size_t>(seq) * a.n1;
+    unsigned long long* __restrict__ out    = a.bra_off + static_cast<size_t>(seq) * a.n1;
+    __shared__ unsigned long long warp_tot[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    unsigned long long run[2] = {0ull, 0ull};
+    unsigned long long run = 0;
     for (int base = 0; base < a.n1; base += kScanBlock * kScanItems)
     {
         const int i0 = base + static_cast<int>(threadIdx.x) * kScanItems;
-        uint2 c[kScanItems];
-        unsigned long long own[2] = {0ull, 0ull}, x[2];
+        unsigned c[kScanItems];
+        unsigned long long own = 0;
 #pragma unroll
         for (int k = 0; k < kScanItems; ++k)
         {
-            c[k] = i0 + k < a.n1 ? reinterpret_cast<const uint2*>(a.bra_cnt)[i0 + k] : make_uint2(0u, 0u);
-            own[0] += c[k].x;
-            own[1] += c[k].y;
+            c[k] = i0 + k < a.n1 ? cnt[i0 + k] : 0u;
+            own += c[k];
         }
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
+        unsigned long long x = own;
+        for (int o = 1; o < 32; o <<= 1)
         {
-            x[q] = own[q];
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const unsigned long long y = __shfl_up_sync(0xffffffffu, x[q], o);
-                if (lane >= o)
-                    x[q] += y;
-            }
-            if (lane == 31)
-                warp_tot[q][w] = x[q];
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o)
+                x += y;
         }
+        if (lane == 31)
+            warp_tot[w] = x;
         __syncthreads();
-        if (w < 2) // warp w turns sequence w's warp totals into inclusive sums
+        if (w == 0)
         {
-            unsigned long long t = warp_tot[w][lane];
+            unsigned long long t = warp_tot[lane];
             for (int o = 1; o < 32; o <<= 1)
             {
                 const unsigned long long y = __shfl_up_sync(0xffffffffu, t, o);
                 if (lane >= o)
                     t += y;
             }
-            warp_tot[w][lane] = t;
+            warp_tot[lane] = t; // inclusive
         }
         __syncthreads();
-        unsigned long long off[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) off[q] = run[q] + (w > 0 ? warp_tot[q][w - 1] : 0ull) + x[q] - own[q];
+        unsigned long long off = run + (w > 0 ? warp_tot[w - 1] : 0ull) + x - own;
 #pragma unroll
         for (int k = 0; k < kScanItems; ++k)
         {
             if (i0 + k < a.n1)
-                reinterpret_cast<ulonglong2*>(a.bra_off)[i0 + k] = make_ulonglong2(off[0], off[1]);
-            off[0] += c[k].x;
-            off[1] += c[k].y;
+                out[i0 + k] = off;
+            off += c[k];
         }
-        run[0] += warp_tot[0][31];
-        run[1] += warp_tot[1][31];
+        run += warp_tot[31];
         __syncthreads(); // the next round overwrites warp_tot
     }
     if (threadIdx.x == 0)
     {
-        b.counts[2 * a.qc]     = run[0];
-        b.counts[2 * a.qc + 1] = run[1];
+        a.seq_tot[seq] = run;
+        if (run)
+            atomicAdd(b.counts + 2 * a.qc + (seq == kListKeys ? 1 : 0), run);
     }
 }
 
@@ -1094,10 +1122,11 @@ static void pack_molecules(hfg_engine* e)
     e->d_tables.alloc(1);
     e->d_next.alloc(2 * kNumQuartetClasses * kMaxChunks);
     HFG_CUDA(cudaMemcpyAsync(e->d_tables.p, tables.get(), sizeof(WarpTables), cudaMemcpyHostToDevice, e->stream));
+    const std::vector<std::vector<double>> fast = boys_fast_slices_host(kMaxLt + 1);
     for (int L = 0; L <= kMaxLt + 1; ++L)
     {
         e->d_boys64[L].upload(boys_slice_host<double>(L), e->stream);
-        e->d_boysf[L].upload(boys_fast_slice_host(L), e->stream);
+        e->d_boysf[L].upload(fast[L], e->stream);
         e->d_boys32[L].upload(boys_slice_host<float>(L), e->stream);
     }
     HFG_CUDA(cudaStreamSynchronize(e->stream));
@@ -1224,6 +1253,17 @@ static void sort_classes(hfg_engine* e)
             }
             e->cls_molseg[pc][m] = make_int2(first, static_cast<int>(e->cls_seg[pc].size()));
         }
+        // Buckets of the primitive counts, largest first (the FP64 lists' keys), in the segments' fourth field.
+        std::vector<int> counts;
+        for (const int4& seg : e->cls_seg[pc]) counts.push_back(-seg.z);
+        std::sort(counts.begin(), counts.end());
+        counts.erase(std::unique(counts.begin(), counts.end()), counts.end());
+        const int kinds = static_cast<int>(counts.size());
+        for (int4& seg : e->cls_seg[pc])
+        {
+            const int at = static_cast<int>(std::lower_bound(counts.begin(), counts.end(), -seg.z) - counts.begin());
+            seg.w        = kinds <= kListBuckets ? at : at * kListBuckets / kinds;
+        }
         std::vector<int2> sh(ids.size());
         for (size_t k2 = 0; k2 < ids.size(); ++k2) sh[k2] = make_int2(e->pairs[ids[k2]].sh1, e->pairs[ids[k2]].sh2);
         e->d_cls_sh[pc].upload(sh, e->stream);
@@ -1333,9 +1373,8 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
             e->d_list[qc][0].alloc(std::max<unsigned long long>(c, 1));
             if (mixed)
                 e->d_list[qc][1].alloc(std::max<unsigned long long>(c, 1));
-            e->d_bra_cnt[qc].alloc(2 * std::max<size_t>(e->cls_ids[P1].size(), 1));
-            e->d_bra_near[qc].alloc(std::max<size_t>(e->cls_ids[P1].size(), 1));
-            e->d_bra_off[qc].alloc(2 * std::max<size_t>(e->cls_ids[P1].size(), 1));
+            e->d_bra_cnt[qc].alloc(kListSeqs * std::max<size_t>(e->cls_ids[P1].size(), 1));
+            e->d_bra_off[qc].alloc(kListSeqs * std::max<size_t>(e->cls_ids[P1].size(), 1));
         }
     e->cap_thr   = sthr;
     e->cap_mixed = mixed;
@@ -1344,7 +1383,8 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
 // Screening and the survival lists of every quartet class from the densities already in d_dD[0..2]
 // (the shell-pair maxima, then count pass, scan and write pass per class).  Returns the launches.
 // graph: enqueue only (no host synchronisation); the counts go to the pinned buffer, checked after replay.
-static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double dthr, double cutoff, bool graph = false)
+static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double dthr, double cutoff, bool graph = false,
+                       bool keyed = true)
 {
     cudaStream_t s  = e->stream;
     const int nspin = uhf ? 3 : 2;
@@ -1362,6 +1402,7 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
     // Lists: count pass, scan, write pass, per quartet class.
     const int ncnt = kNumQuartetClasses * 2;
     e->d_counts.alloc(2 * ncnt + 1);
+    e->d_seq_tot.alloc(kNumQuartetClasses * kListSeqs);
     HFG_CUDA(cudaMemsetAsync(e->d_counts.p, 0, sizeof(unsigned long long) * (2 * ncnt + 1), s));
     BuildArgs a {};
     int blocks = 0;
@@ -1387,12 +1428,12 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
         c.Qf1         = e->d_cls_Qf[P1].p;
         c.Qf2         = e->d_cls_Qf[P2].p;
         c.bra_cnt     = e->d_bra_cnt[qc].p;
-        c.bra_near    = e->d_bra_near[qc].p;
         c.group_off   = e->d_group_off[qc].p;
         c.groups      = e->d_groups[qc].p;
         c.diff1       = e->d_cls_diff[P1].p;
         c.diff2       = e->d_cls_diff[P2].p;
         c.bra_off     = e->d_bra_off[qc].p;
+        c.seq_tot     = e->d_seq_tot.p + qc * kListSeqs;
         c.out64       = e->d_list[qc][0].p;
         c.out32       = mixed ? e->d_list[qc][1].p : nullptr;
         c.cap         = e->cap[qc];
@@ -1409,12 +1450,13 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
     a.dthr     = dthr;
     a.cutoff   = static_cast<float>(cutoff);
     a.mixed    = mixed ? 1 : 0;
+    a.keyed    = keyed ? 1 : 0;
     a.counts   = e->d_counts.p;
     int launches = 0;
     if (a.ncls > 0)
     {
         test_lists_kernel<<<static_cast<unsigned>(blocks), 32 * kBuildWarps, 0, s>>>(a);
-        scan_lists_kernel<<<static_cast<unsigned>(a.ncls), kScanBlock, 0, s>>>(a);
+        scan_lists_kernel<<<static_cast<unsigned>(a.ncls * kListSeqs), kScanBlock, 0, s>>>(a);
         write_lists_kernel<<<static_cast<unsigned>(blocks), 32 * kBuildWarps, 0, s>>>(a);
         HFG_CUDA(cudaGetLastError());
         launches = 3;
@@ -1467,8 +1509,10 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
     if (n < kTuneMin || !e->autotune || (tried & (tried - 1)) == 0)
         return 0; // too small to time, or tuning off: the default form runs and the class stays untuned
     const auto t0 = std::chrono::steady_clock::now();
-    const unsigned long long nch   = n <= kTuneSample ? 1 : kTuneChunks;
-    const unsigned long long chunk = n <= kTuneSample ? n : kTuneSample / kTuneChunks;
+    // FP64 quartets take some ten times as long: an eighth of the sample.
+    const unsigned long long most  = prec == 0 ? kTuneSample / 8 : kTuneSample;
+    const unsigned long long nch   = n <= most ? 1 : kTuneChunks;
+    const unsigned long long chunk = n <= most ? n : most / kTuneChunks;
     const unsigned long long m     = nch * chunk;
     cudaStream_t s = base.stream;
     e->d_tune_list.alloc(m);
@@ -1530,14 +1574,14 @@ struct SideStreams
     bool is_short(unsigned long long prims) const { return prims < static_cast<unsigned long long>(e->num_sms) * 256 * 64; }
     cudaStream_t next()
     {
-        const int k = used++ % 4;
-        if (used <= 4)
+        const int k = used++ % kSideStreams;
+        if (used <= kSideStreams)
             HFG_CUDA(cudaStreamWaitEvent(e->side[prec][k], e->ev_side[prec][0], 0));
         return e->side[prec][k];
     }
     void join()
     {
-        for (int k = 0; k < std::min(used, 4); ++k)
+        for (int k = 0; k < std::min(used, kSideStreams); ++k)
         {
             HFG_CUDA(cudaEventRecord(e->ev_side[prec][1 + k], e->side[prec][k]));
             HFG_CUDA(cudaStreamWaitEvent(own, e->ev_side[prec][1 + k], 0));
@@ -1909,7 +1953,8 @@ static void store_integrals(hfg_engine* e, double sthr, size_t* bytes_out)
         HFG_CUDA(cudaMemsetAsync(e->d_dD[k].p, 0, sizeof(double) * N2, e->stream));
     }
     e->d_smax2.alloc(e->smax_total);
-    build_lists(e, false, false, sthr, 0.0, 0.0); // density threshold 0: Schwartz survivors only
+    // Density threshold 0: Schwartz survivors only.  By bra pair: the stored build does no primitive work.
+    build_lists(e, false, false, sthr, 0.0, 0.0, false, false);
     size_t bytes = 0;
     for (int qc = 0; qc < kNumQuartetClasses; ++qc)
     {
