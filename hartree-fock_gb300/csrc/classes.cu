@@ -333,13 +333,20 @@ cudaError_t HFG_CAT(launch_class32_, HFG_QCLASS)(const ClassLaunch& c)
 #else
 namespace
 {
-// Thread-per-quartet gradient form: up to 300 values a thread (GradThread::kValues).  What does not fit the
+// Thread-per-quartet gradient form, by the values a thread holds at its peak (GradThread).  What does not fit the
 // registers spills to L1; the lane-group form keeps half its lanes idle in its dynamic index loops.
-//   FP64: every class up to (pp|ps), (ds|ps), (ds|pp), (ds|ds), (dp|ss), (dp|ps), (dd|ss) but (pp|pp);
-//   FP32: up to 160 values, and to 300 with d shells, which adds (ds|pp) (ds|ds) (dp|ps) (dd|ss).
+//   FP64, ss or ps ket (single-pass form): every class ((dd|ps), 465 values, is kept in local memory by ptxas and
+//     still takes 5.5 ms of a (H2O)_16 6-31G** gradient against 13.6 in the lane-group form);
+//   FP64, other kets: (ds|pp), (ds|ds) and (pp|pp) ((H2O)_8 cc-pVDZ 18.5 -> 15.5 ms, (H2O)_16 9.0 -> 9.8);
+//   FP32: up to 160 values ((pp|ps) (ds|ps) (dp|ss) and smaller), and to 300 with d shells: (ds|pp) (ds|ds) (dp|ps)
+//     (dd|ss), 38 -> 7 ms of a (H2O)_16 gradient.  (pp|pp) stays as it is: sums of FP32 terms in another order
+//     are 1e-9 of a 6-31G gradient away.
 template <typename Real> constexpr bool grad_thread_form()
 {
-    return GradThread<LA, LB, LC, LD>::kValues <= (sizeof(Real) == 8 || LA == 2 ? 300 : 160);
+    using W = GradThread<LA, LB, LC, LD>;
+    if (sizeof(Real) == 8 && grad_single_pass(LC, LD))
+        return W::kValuesSingle <= 480;
+    return W::kValues <= (sizeof(Real) == 8 ? 410 : LA == 2 ? 300 : 160);
 }
 
 // The split of a gradient launch: `width` lanes work on one slice together.

@@ -183,6 +183,7 @@ struct hfg_engine
     hfg::DevBuf<double> d_boysf[hfg::kMaxLt + 2]; // BoysFast slices
     hfg::DevBuf<float> d_boys32[hfg::kMaxLt + 2];
     hfg::DevBuf<double> d_gtab[hfg::kNumPairClasses]; // gradient records (built on first use)
+    hfg::DevBuf<double> d_gder[hfg::kNumPairClasses]; // derivative coefficients of the ss and ps classes, same order
     hfg::DevBuf<float> d_gtab32[hfg::kNumPairClasses]; // their FP32 copies (mixed-precision gradient)
     bool have_gtab = false;
     hfg::DevBuf<int> d_shell_atom;
@@ -1586,7 +1587,17 @@ struct SideStreams
             HFG_CUDA(cudaEventRecord(e->ev_side[prec][1 + k], e->side[prec][k]));
             HFG_CUDA(cudaStreamWaitEvent(own, e->ev_side[prec][1 + k], 0));
         }
+        used = 0;
     }
+    // Left by an exception: what was launched still ends before later work on the own stream.
+    ~SideStreams()
+    {
+        for (int k = 0; k < std::min(used, kSideStreams); ++k)
+            if (cudaEventRecord(e->ev_side[prec][1 + k], e->side[prec][k]) == cudaSuccess)
+                cudaStreamWaitEvent(own, e->ev_side[prec][1 + k], 0);
+    }
+    SideStreams(const SideStreams&) = delete;
+    SideStreams& operator=(const SideStreams&) = delete;
 };
 
 // Enqueues one build on the engine stream.  Eager (graph == false): timing events, list lengths read
@@ -2050,7 +2061,7 @@ static void fock_conventional(hfg_engine* e, const hfg_fock_request& r, hfg_fock
         L.view.X      = e->d_acc[0].p;
         L.view.Ya     = e->d_acc[1].p;
         L.view.Yb     = e->d_acc[2].p;
-        L.view.ao_thr = r.schwartz_threshold;
+        L.view.ao_thr = r.schwartz_threshold >= 0.0 ? r.schwartz_threshold : 0.0; // (a NaN skips nothing)
         L.uhf         = uhf;
         L.stream      = side.next();
         L.num_sms     = e->num_sms;
@@ -2222,7 +2233,7 @@ static void build_grad_tables(hfg_engine* e)
 {
     if (e->have_gtab)
         return;
-    std::vector<std::vector<double>> tab(kNumPairClasses);
+    std::vector<std::vector<double>> tab(kNumPairClasses), der(kNumPairClasses);
     for (size_t k = 0; k < e->pairs.size(); ++k)
     {
         const PairRec& pr = e->pairs[k];
@@ -2271,11 +2282,33 @@ static void build_grad_tables(hfg_engine* e)
                             }
                         }
                 }
+                if (!grad_single_pass(l1, l2))
+                    continue;
+                // The first centre's derivatives, d/dA_x = 2a E^{i+1,j} - i E^{i-1,j} on axis x (d3_offset's order).
+                for (int kl = 0; kl < ncart(l1) * ncart(l2); ++kl)
+                    for (int dir = 0; dir < 3; ++dir)
+                        for (int v = 0; v < d3_len(l1, l2, kl, dir, 2); ++v)
+                            for (int u = 0; u < d3_len(l1, l2, kl, dir, 1); ++u)
+                                for (int t = 0; t < d3_len(l1, l2, kl, dir, 0); ++t)
+                                {
+                                    const int tuv[3] = {t, u, v};
+                                    double x = ((t + u + v) & 1) ? -1.0 : 1.0;
+                                    for (int ax = 0; ax < 3; ++ax)
+                                    {
+                                        const double* E = rec + 2 + ax * n1;
+                                        const int i = cart_exp(l1, kl / ncart(l2), ax), j = cart_exp(l2, kl % ncart(l2), ax);
+                                        auto at = [&](int ii, int tt) { return E[(ii * (l2 + 2) + j) * (l1 + l2 + 3) + tt]; };
+                                        x *= ax == dir ? 2.0 * aa * at(i + 1, tuv[ax]) - (i > 0 ? i * at(i - 1, tuv[ax]) : 0.0)
+                                                       : at(i, tuv[ax]);
+                                    }
+                                    der[pc].push_back(x);
+                                }
             }
     }
     for (int pc = 0; pc < kNumPairClasses; ++pc)
     {
         e->d_gtab[pc].upload(tab[pc], e->stream);
+        e->d_gder[pc].upload(der[pc], e->stream);
         e->d_gtab32[pc].upload(std::vector<float>(tab[pc].begin(), tab[pc].end()), e->stream);
     }
     HFG_CUDA(cudaStreamSynchronize(e->stream));
@@ -2319,6 +2352,7 @@ static double gradient_two_electron(hfg_engine* e, const std::vector<int>& shell
         for (int pc = 0; pc < kNumPairClasses; ++pc)
         {
             g.pptab[pc] = prec ? static_cast<const void*>(e->d_pptab32_full[pc].p) : e->d_pptab64_full[pc].p;
+            g.gder[pc]  = e->d_gder[pc].p;
             g.gtab[pc]  = prec ? static_cast<const void*>(e->d_gtab32[pc].p) : e->d_gtab[pc].p;
         }
         g.Dt = prec ? static_cast<const void*>(e->d_dDf[0].p) : e->d_dD[0].p;

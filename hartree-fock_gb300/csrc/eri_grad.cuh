@@ -37,11 +37,30 @@ __host__ __device__ constexpr int g_stride(int l1, int l2)
     return s + (s & 1);
 }
 
+// 3-D Hermite coefficients of the first centre's derivatives of a primitive pair (l1, l2), for the single-pass
+// form: per Cartesian pair kl and direction x, the product of the derivative coefficient of axis x (one order
+// more) with the plain coefficients of the other two, t fastest, with the sign (-1)^{t+u+v} of a ket.
+__host__ __device__ constexpr int d3_len(int l1, int l2, int kl, int dir, int ax)
+{
+    return cart_exp(l1, kl / ncart(l2), ax) + cart_exp(l2, kl % ncart(l2), ax) + 1 + (ax == dir ? 1 : 0);
+}
+__host__ __device__ constexpr int d3_offset(int l1, int l2, int kl, int dir)
+{
+    int off = 0;
+    for (int k = 0; k < kl * 3 + dir; ++k)
+        off += d3_len(l1, l2, k / 3, k % 3, 0) * d3_len(l1, l2, k / 3, k % 3, 1) * d3_len(l1, l2, k / 3, k % 3, 2);
+    return off;
+}
+__host__ __device__ constexpr int d3_total(int l1, int l2) { return d3_offset(l1, l2, ncart(l1) * ncart(l2), 0); }
+// Kets of the single-pass form: ss and ps.
+__host__ __device__ constexpr bool grad_single_pass(int l1, int l2) { return l1 + l2 <= 1; }
+
 struct GradView
 {
     const PairRec* pairs;
     const void* pptab[kNumPairClasses]; // forward records (p, P, W, ...), Real of the kernel
     const void* gtab[kNumPairClasses];  // gradient records, Real of the kernel
+    const double* gder[kNumPairClasses]; // d3 coefficients of the ss and ps classes (FP64 kernels)
     const void* Dt;                     // densities, Real of the kernel
     const void* Da;
     const void* Db;
@@ -398,6 +417,10 @@ __global__ void __launch_bounds__(32 * kGradWarps)
 //               g_A += DA . y,  g_P += E . y(t+1)  (d/dA + d/dB = d/dP: the R index shifted by one);
 //   ket-outer:  Hs[tuv'][ij] = sum_{bra prims} sum_tuv E^{ij}_{tuv} R_{t+tau,..} (tau+nu+phi <= l_cd + 1),
 //               h = sum_ij Gamma_ijkl Hs once per ket primitive pair, g_C += (-1)^{..} DC . h;
+// In FP64 with an ss or ps ket one pass does both: per bra primitive pair yb[tuv][kl] = sum_ij Gamma_ijkl
+// E^{ij}_{tuv}, and per primitive quartet g_C += sum_{kl, tuv'} DC^{kl}_{tuv'} sum_tuv yb[tuv][kl] R_{t+tau,..}.  For
+// these kets that costs less than evaluating R a second time and summing Hs (an s ket: 4 sums over the bra's
+// tuv and 6 products): FP64 instructions per primitive quartet 90 -> 50 for (ss|ss), 133 -> 82 for (ps|ss).
 // g_B = g_P - g_A and g_D = -(g_P + g_C).  The Gamma contraction runs once per primitive pair instead of
 // once per primitive quartet; every term whose Hermite index lies outside the non-zero range of its
 // coefficients is dropped at compile time.  Warp-uniform iteration: when the 32 quartets of a warp share
@@ -411,6 +434,7 @@ template <int LA, int LB, int LC, int LD> struct GradThread
     static constexpr int kPass1 = NAB * NCD + nherm(L) + HAB1 * NCD;
     static constexpr int kPass2 = NAB * NCD + nherm(L) + HCD1 * NAB;
     static constexpr int kValues = kPass1 > kPass2 ? kPass1 : kPass2;
+    static constexpr int kValuesSingle = kPass1 + nherm(LAB) * NCD; // the single-pass form
 };
 
 template <int LA, int LB, int LC, int LD, typename Real>
@@ -505,18 +529,77 @@ __global__ void __launch_bounds__(128)
                 hermite_R<L, Real>(Fs, X, Y, Z, R);
             };
 
-            // Bra-outer pass: centres A and P.
+            constexpr bool kSingle = sizeof(Real) == 8 && grad_single_pass(LC, LD);
+            constexpr int HAB      = nherm(LAB);
+            // Bra-outer pass: centres A and P (and C in the single-pass form).
             for (int ib = pr.ib0; ib < bra.npp; ib += pr.ibs)
             {
                 const Real* __restrict__ rb = tbf + static_cast<size_t>(bra.pp_off + ib) * SB;
                 Real Gs[HAB1 * NCD];
 #pragma unroll
                 for (int x = 0; x < HAB1 * NCD; ++x) Gs[x] = Real(0);
+                Real yb[kSingle ? HAB * NCD : 1];
+                if constexpr (kSingle)
+                {
+#pragma unroll
+                    for (int x = 0; x < HAB * NCD; ++x) yb[x] = Real(0);
+                    static_for<0, NAB>(
+                        [&](auto IJ)
+                        {
+                            constexpr int ij = decltype(IJ)::value;
+                            constexpr int lx = e3_len(LA, LB, ij, 0), ly = e3_len(LA, LB, ij, 1), lz = e3_len(LA, LB, ij, 2);
+                            constexpr int eoff = kPairHeader + e3_offset(LA, LB, ij);
+                            static_for<0, lx * ly * lz>(
+                                [&](auto EE)
+                                {
+                                    constexpr int e = decltype(EE)::value;
+                                    constexpr int h = hidx(e % lx, (e / lx) % ly, e / (lx * ly), LAB);
+#pragma unroll
+                                    for (int kl = 0; kl < NCD; ++kl)
+                                        yb[h * NCD + kl] += LAB == 0 ? Gam[kl] : rb[eoff + e] * Gam[ij * NCD + kl];
+                                });
+                        });
+                }
                 for (int ik = pr.ik0; ik < ket.npp; ik += pr.iks)
                 {
                     const Real* __restrict__ rk = tkf + static_cast<size_t>(ket.pp_off + ik) * SK;
                     Real R[nherm(L)];
                     prim_R(rb, rk, R);
+                    if constexpr (kSingle)
+                    {
+                        const double* __restrict__ dc = v.gder[PCK] + static_cast<size_t>(ket.pp_off + ik) * d3_total(LC, LD);
+                        static_for<0, NCD * HCD1>(
+                            [&](auto KH)
+                            {
+                                constexpr int kl = decltype(KH)::value / HCD1, h = decltype(KH)::value % HCD1;
+                                constexpr int tau = htuv(h, LCD + 1, 0), nu = htuv(h, LCD + 1, 1), phi = htuv(h, LCD + 1, 2);
+                                constexpr auto in = [](int dir)
+                                {
+                                    return tau < d3_len(LC, LD, kl, dir, 0) && nu < d3_len(LC, LD, kl, dir, 1) &&
+                                           phi < d3_len(LC, LD, kl, dir, 2);
+                                };
+                                if constexpr (in(0) || in(1) || in(2))
+                                {
+                                    Real z = Real(0);
+                                    static_for<0, HAB>(
+                                        [&](auto B)
+                                        {
+                                            constexpr int hb = decltype(B)::value;
+                                            z += yb[hb * NCD + kl] * R[hidx(htuv(hb, LAB, 0) + tau, htuv(hb, LAB, 1) + nu,
+                                                                            htuv(hb, LAB, 2) + phi, L)];
+                                        });
+                                    static_for<0, 3>(
+                                        [&](auto D)
+                                        {
+                                            constexpr int dir = decltype(D)::value;
+                                            if constexpr (in(dir))
+                                                gC[dir] += z * dc[d3_offset(LC, LD, kl, dir) +
+                                                                  (phi * d3_len(LC, LD, kl, dir, 1) + nu) * d3_len(LC, LD, kl, dir, 0) +
+                                                                  tau];
+                                        });
+                                }
+                            });
+                    }
                     static_for<0, NCD>(
                         [&](auto KL)
                         {
@@ -609,6 +692,7 @@ __global__ void __launch_bounds__(128)
             }
 
             // Ket-outer pass: centre C.
+            if constexpr (!kSingle)
             for (int ik = pr.ik0; ik < ket.npp; ik += pr.iks)
             {
                 const Real* __restrict__ rk = tkf + static_cast<size_t>(ket.pp_off + ik) * SK;

@@ -144,7 +144,7 @@ int hfg_store_integrals(hfg_engine* engine, double schwartz_threshold, size_t* b
 int hfg_fock_conventional(hfg_engine* engine, const hfg_fock_request* req, hfg_fock_stats* stats);
 
 /* Kernel forms of a class kernel.  THREAD: one thread per shell quartet.  WARP: one warp per quartet
- * (the large d classes).  GROUP: a power-of-two group of lanes per quartet, splitting its primitive
+ * (the largest d classes).  GROUP: a power-of-two group of lanes per quartet, splitting its primitive
  * quartets (the small contracted classes, L <= 3).  AUTO: on the first build that runs the class with
  * enough quartets, every compiled form runs on an evenly spaced sample of the real list and the fastest
  * is kept for the life of the engine (per class, precision and RHF/UHF).
@@ -153,7 +153,7 @@ int hfg_fock_conventional(hfg_engine* engine, const hfg_fock_request* req, hfg_f
 #define HFG_FORM_THREAD 1
 #define HFG_FORM_WARP 2
 #define HFG_FORM_GROUP 3
-#define HFG_FORM_CHUNK 4 /* one thread per (quartet, chunk of ket Cartesian components): the FP32 d classes */
+#define HFG_FORM_CHUNK 4 /* one thread per (quartet, chunk of ket Cartesian components): the dp and dd classes */
 #define HFG_FORM_PERSISTENT 5 /* in hfg_fock_stats only: the class ran in the persistent work queue */
 /* Set the form of class `qclass` (-1: every class) at precision `fp32` (0: FP64 kernels, 1: FP32
  * kernels).  HFG_FORM_AUTO forgets earlier timings; a form the class was not compiled in returns
@@ -192,9 +192,9 @@ int hfg_set_persistent(hfg_engine* engine, int on);
 int hfg_set_autotune(hfg_engine* engine, int on);
 
 /* Gradient kernel form (no reference counterpart): 0 (default) runs the thread-per-quartet gradient kernel
- * for the classes whose per-quartet arrays fit in registers ((ss|ss) (ps|ss) (ps|ps) (pp|ss) (ds|ss) in
- * FP64, and (pp|ps) (ds|ps) (dp|ss) as well in FP32) and the lane-group kernel for the others; 1 runs the
- * lane-group kernel for every class.  Both give the same gradient to rounding. */
+ * for the classes it is compiled for (up to (pp|ps), (ds|ds), (dp|ps) and (dd|ss), in FP64 also (pp|pp) and
+ * (dd|ps)) and the lane-group kernel for the others; 1 runs the lane-group kernel for every class.  Both
+ * give the same gradient to rounding. */
 int hfg_set_gradient_form(hfg_engine* engine, int group_only);
 
 /* Forms in use: forms[qc] for the given precision and spin case, 0 where AUTO has not decided yet.

@@ -93,3 +93,48 @@ def test_gpu_split_gradient_forms_agree(port, basis_name, system, uhf):
     assert np.max(np.abs(g[False] - g[True])) <= 1e-10 * max(1.0, np.max(np.abs(g[True])))
     # Translational invariance of the whole gradient.
     assert np.max(np.abs(g[False].sum(axis=0))) <= 1e-9 * max(1.0, np.max(np.abs(g[False])))
+
+
+@pytest.mark.parametrize("count,kmax", [(3, 2), (24, 5)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_gpu_batch_lists_match_single_engines(count, kmax, precision):
+    """Lists whose keys mix the bra pairs of many molecules, against one engine per molecule (mixed: the same
+    FP32 quartets, summed in lists of another alignment: 1e-7)."""
+    from hfgpu import basis, workloads
+    from hfgpu.engine import Engine
+
+    mols = workloads.uneven_batch(count, kmax, seed=5)
+    soas = [basis.pack("6-31G", Z, xyz) for Z, xyz in mols]
+    singles = [Engine(s) for s in soas]
+    D = [_sym(e.nao, k, 0.05) for k, e in enumerate(singles)]
+    flat = np.concatenate([d.ravel() for d in D])
+    J, K, _, _ = Engine(soas).fock(2 * flat, flat, precision=precision)
+    at = 0
+    for e, d in zip(singles, D):
+        j, k, _, _ = e.fock(2 * d, d, precision=precision)
+        n2 = e.nao ** 2
+        tol = 1e-10 if precision == 0 else 1e-7
+        assert np.max(np.abs(J[at:at + n2] - j.ravel(order="F"))) <= tol
+        assert np.max(np.abs(K[at:at + n2] - k.ravel(order="F"))) <= tol
+        at += n2
+
+
+@pytest.mark.parametrize("basis_name,system", [("cc-pVDZ", "2"), ("6-31G", "5")])
+def test_gpu_split_graph_replay_with_another_density(port, basis_name, system):
+    """A captured build sizes its grids by the eager one and reads the replay's lists on the device."""
+    torch = pytest.importorskip("torch")
+    e, B, Q, _, _ = _setup(port, basis_name, system)
+    n = B.nao
+    ins = [torch.zeros(n * n, dtype=torch.float64, device="cuda") for _ in range(2)]
+    outs = [torch.zeros(n * n, dtype=torch.float64, device="cuda") for _ in range(2)]
+    ptrs = dict(dD_tot=ins[0].data_ptr(), dD_alpha=ins[1].data_ptr(), J=outs[0].data_ptr(), K_alpha=outs[1].data_ptr())
+    e.set_graph_mode(True)
+    for seed, scale in ((1, 1e-9), (2, 0.1), (3, 1e-6)):  # few survivors when captured, many in the replay
+        D = _sym(n, seed, scale)
+        ins[0].copy_(torch.from_numpy(2 * D.ravel()))
+        ins[1].copy_(torch.from_numpy(D.ravel().copy()))
+        torch.cuda.synchronize()
+        e.fock_device(ptrs)
+        Jr, Kr, _, _ = B.fock_direct(Q, 2 * D, D)
+        J, K = (o.cpu().numpy().reshape(n, n, order="F") for o in outs)
+        assert np.max(np.abs(J - Jr)) <= 1e-10 and np.max(np.abs(K - Kr)) <= 1e-10
