@@ -307,28 +307,59 @@ __global__ void to_float_kernel(const double* __restrict__ a, float* __restrict_
         b[i] = static_cast<float>(a[i]);
 }
 
-// The transposed copies of the molecule blocks of a: t64, t32 (either may be null).
-__global__ void transpose_kernel(const double* __restrict__ a, double* __restrict__ t64, float* __restrict__ t32,
-                                 const long long* __restrict__ mat_off, const int* __restrict__ mat_ld, int nmol, long long total)
+// The matrices of a build, total / alpha / beta: one launch serves them all (blockIdx.y), since for a small
+// molecule each launch costs as much as its work.
+struct SpinSet
 {
+    const double* dD[3];
+    double* acc[3];   // X, Y accumulators
+    double* dT[3];    // transposed copies (alpha, beta)
+    float* f32[3];    // FP32 copies, alpha and beta transposed (null: FP64 build)
+    double* out[3];   // J, K
+    double* smax[3];  // shell-pair maxima
+    double* smax2;    // 2 * smax[0]
+};
+
+// The molecule block of element e of the packed matrices: its offset and n, and the element's row and column.
+__device__ __forceinline__ long long block_of(long long e, const long long* __restrict__ mat_off, const int* __restrict__ mat_ld,
+                                              int nmol, int& n, int& r, int& c)
+{
+    int lo = 0, hi = nmol - 1;
+    while (lo < hi)
+    {
+        const int mid = (lo + hi + 1) >> 1;
+        if (mat_off[mid] <= e)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const long long off = mat_off[lo];
+    n = mat_ld[lo];
+    r = static_cast<int>((e - off) % n);
+    c = static_cast<int>((e - off) / n);
+    return off;
+}
+
+// Zeroes the accumulators and makes the copies the class kernels read.
+__global__ void prepare_kernel(SpinSet m, const long long* __restrict__ mat_off, const int* __restrict__ mat_ld, int nmol,
+                               long long total)
+{
+    const int k = blockIdx.y;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x)
     {
-        int lo = 0, hi = nmol - 1;
-        while (lo < hi)
+        m.acc[k][e] = 0.0;
+        if (k == 0)
         {
-            const int mid = (lo + hi + 1) >> 1;
-            if (mat_off[mid] <= e)
-                lo = mid;
-            else
-                hi = mid - 1;
+            if (m.f32[0])
+                m.f32[0][e] = static_cast<float>(m.dD[0][e]);
+            continue;
         }
-        const long long off = mat_off[lo], loc = e - off;
-        const int n = mat_ld[lo], r = static_cast<int>(loc % n), c = static_cast<int>(loc / n);
-        const double x = a[off + c + (long long)r * n];
-        if (t64)
-            t64[e] = x;
-        if (t32)
-            t32[e] = static_cast<float>(x);
+        int n, r, c;
+        const long long off = block_of(e, mat_off, mat_ld, nmol, n, r, c);
+        const double x      = m.dD[k][off + c + (long long)r * n];
+        m.dT[k][e]          = x;
+        if (m.f32[k])
+            m.f32[k][e] = static_cast<float>(x);
     }
 }
 
@@ -348,11 +379,14 @@ __global__ void sample_list_kernel(const Quartet* __restrict__ list, unsigned lo
 // Shell-pair maxima of |dD| (SCF.cpp:544-575) for every molecule block, with exact integer operations
 // on the bit patterns (|x| clears the sign bit; non-negative doubles order like their bits).  M2, when
 // given, receives 2*M (exact).
-__global__ void shell_max_kernel(const double* __restrict__ dD, const PairRec* __restrict__ pairs, int npairs,
+__global__ void shell_max_kernel(SpinSet m, const PairRec* __restrict__ pairs, int npairs,
                                  const long long* __restrict__ mat_off, const int* __restrict__ mat_ld,
                                  const long long* __restrict__ smax_off, const int* __restrict__ nsh,
-                                 const int* __restrict__ sh_nao, double* __restrict__ M, double* __restrict__ M2)
+                                 const int* __restrict__ sh_nao)
 {
+    const double* __restrict__ dD = m.dD[blockIdx.y];
+    double* __restrict__ M        = m.smax[blockIdx.y];
+    double* __restrict__ M2       = blockIdx.y == 0 ? m.smax2 : nullptr;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < npairs; k += gridDim.x * blockDim.x)
     {
         const PairRec pr = pairs[k];
@@ -686,25 +720,16 @@ __global__ void __launch_bounds__(kScanBlock) scan_lists_kernel(const __grid_con
 }
 
 // J = X + X^T, K = Y + Y^T over the concatenated molecule blocks.
-__global__ void symmetrize_kernel(const double* __restrict__ X, double* __restrict__ J, const long long* __restrict__ mat_off,
-                                  const int* __restrict__ mat_ld, int nmol, long long total)
+__global__ void symmetrize_kernel(SpinSet m, const long long* __restrict__ mat_off, const int* __restrict__ mat_ld, int nmol,
+                                  long long total)
 {
+    const double* __restrict__ X = m.acc[blockIdx.y];
+    double* __restrict__ J       = m.out[blockIdx.y];
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x)
     {
-        int lo = 0, hi = nmol - 1;
-        while (lo < hi)
-        {
-            const int mid = (lo + hi + 1) >> 1;
-            if (mat_off[mid] <= e)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        const long long off = mat_off[lo];
-        const int n = mat_ld[lo];
-        const long long loc = e - off;
-        const int r = static_cast<int>(loc % n), c = static_cast<int>(loc / n);
-        J[e] = X[e] + X[off + c + (long long)r * n];
+        int n, r, c;
+        const long long off = block_of(e, mat_off, mat_ld, nmol, n, r, c);
+        J[e]                = X[e] + X[off + c + (long long)r * n];
     }
 }
 
@@ -1381,6 +1406,22 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
     e->cap_mixed = mixed;
 }
 
+static SpinSet spin_set(hfg_engine* e, bool mixed)
+{
+    SpinSet m {};
+    for (int k = 0; k < 3; ++k)
+    {
+        m.dD[k]   = e->d_dD[k].p;
+        m.acc[k]  = e->d_acc[k].p;
+        m.dT[k]   = e->d_dDT[k].p;
+        m.f32[k]  = mixed ? e->d_dDf[k].p : nullptr;
+        m.out[k]  = e->d_out[k].p;
+        m.smax[k] = e->d_smax[k].p;
+    }
+    m.smax2 = e->d_smax2.p;
+    return m;
+}
+
 // Screening and the survival lists of every quartet class from the densities already in d_dD[0..2]
 // (the shell-pair maxima, then count pass, scan and write pass per class).  Returns the launches.
 // graph: enqueue only (no host synchronisation); the counts go to the pinned buffer, checked after replay.
@@ -1390,15 +1431,11 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
     cudaStream_t s  = e->stream;
     const int nspin = uhf ? 3 : 2;
     // Shell-pair maxima.
-    for (int k = 0; k < nspin; ++k)
-    {
-        if (k == 0)
-            e->d_smax2.alloc(e->smax_total);
-        shell_max_kernel<<<grid_for(e->pairs.size(), 128, e->num_sms), 128, 0, s>>>(
-            e->d_dD[k].p, e->d_pairs.p, static_cast<int>(e->pairs.size()), e->d_mat_off.p, e->d_mat_ld.p, e->d_smax_off.p,
-            e->d_nsh.p, e->d_shnao.p, e->d_smax[k].p, k == 0 ? e->d_smax2.p : nullptr);
-        HFG_CUDA(cudaGetLastError());
-    }
+    e->d_smax2.alloc(e->smax_total);
+    shell_max_kernel<<<dim3(grid_for(e->pairs.size(), 128, e->num_sms), nspin), 128, 0, s>>>(
+        spin_set(e, mixed), e->d_pairs.p, static_cast<int>(e->pairs.size()), e->d_mat_off.p, e->d_mat_ld.p, e->d_smax_off.p,
+        e->d_nsh.p, e->d_shnao.p);
+    HFG_CUDA(cudaGetLastError());
 
     // Lists: count pass, scan, write pass, per quartet class.
     const int ncnt = kNumQuartetClasses * 2;
@@ -1463,7 +1500,7 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
         launches = 3;
     }
     if (graph)
-        return launches + nspin;
+        return launches + 1;
     e->h_counts.assign(2 * ncnt + 1, 0);
     HFG_CUDA(cudaMemcpyAsync(e->h_counts.data(), e->d_counts.p, sizeof(unsigned long long) * (2 * ncnt + 1),
                              cudaMemcpyDeviceToHost, s));
@@ -1473,7 +1510,7 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
         if (e->h_counts[2 * qc] > e->cap[qc] || e->h_counts[2 * qc + 1] > e->cap[qc])
             throw HfgError(HFG_ERR_OVERFLOW, "fock: quartet list overflow");
 
-    return launches + nspin;
+    return launches + 1;
 }
 
 // Kernel form autotuner.  A class whose list has at least kTuneMin quartets and more than one compiled
@@ -1619,20 +1656,14 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
     {
         HFG_CUDA(cudaMemcpyAsync(e->d_dD[k].p, src[k], sizeof(double) * N2,
                                  r.device_pointers ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
-        HFG_CUDA(cudaMemsetAsync(e->d_acc[k].p, 0, sizeof(double) * N2, s));
-        if (k > 0)
-            transpose_kernel<<<grid_for(N2, 256, e->num_sms), 256, 0, s>>>(e->d_dD[k].p, e->d_dDT[k].p,
-                                                                          mixed ? e->d_dDf[k].p : nullptr, e->d_mat_off.p,
-                                                                          e->d_mat_ld.p, e->nmol, N2);
-        else if (mixed)
-            to_float_kernel<<<grid_for(N2, 256, e->num_sms), 256, 0, s>>>(e->d_dD[k].p, e->d_dDf[k].p, N2);
-        HFG_CUDA(cudaGetLastError());
     }
+    prepare_kernel<<<dim3(grid_for(N2, 256, e->num_sms), nspin), 256, 0, s>>>(spin_set(e, mixed), e->d_mat_off.p, e->d_mat_ld.p,
+                                                                            e->nmol, N2);
+    HFG_CUDA(cudaGetLastError());
     if (!graph)
         HFG_CUDA(cudaEventRecord(e->ev[1], s));
 
-    int launches = nspin - 1 + (mixed ? 1 : 0) +
-                   build_lists(e, uhf, mixed, r.schwartz_threshold, r.density_threshold, r.fp32_cutoff, graph);
+    int launches = 1 + build_lists(e, uhf, mixed, r.schwartz_threshold, r.density_threshold, r.fp32_cutoff, graph);
 
     // Class kernels: FP64 lists on `s`; FP32 lists on stream2 concurrently when overlapping, else after.
     const bool overlap = mixed && e->overlap;
@@ -1770,13 +1801,10 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
     if (!graph)
         HFG_CUDA(cudaEventRecord(e->ev[5], s));
     double* outs[3] = {r.J, r.K_alpha, r.K_beta};
-    for (int k = 0; k < nspin; ++k)
-    {
-        symmetrize_kernel<<<grid_for(N2, 256, e->num_sms), 256, 0, s>>>(e->d_acc[k].p, e->d_out[k].p, e->d_mat_off.p,
-                                                                          e->d_mat_ld.p, e->nmol, N2);
-        HFG_CUDA(cudaGetLastError());
-        ++launches;
-    }
+    symmetrize_kernel<<<dim3(grid_for(N2, 256, e->num_sms), nspin), 256, 0, s>>>(spin_set(e, mixed), e->d_mat_off.p,
+                                                                               e->d_mat_ld.p, e->nmol, N2);
+    HFG_CUDA(cudaGetLastError());
+    ++launches;
     if (!graph)
         HFG_CUDA(cudaEventRecord(e->ev[6], s));
     for (int k = 0; k < nspin; ++k)
@@ -2034,15 +2062,11 @@ static void fock_conventional(hfg_engine* e, const hfg_fock_request& r, hfg_fock
     {
         HFG_CUDA(cudaMemcpyAsync(e->d_dD[k].p, src[k], sizeof(double) * N2,
                                  r.device_pointers ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
-        HFG_CUDA(cudaMemsetAsync(e->d_acc[k].p, 0, sizeof(double) * N2, s));
-        if (k > 0)
-        {
-            transpose_kernel<<<grid_for(N2, 256, e->num_sms), 256, 0, s>>>(e->d_dD[k].p, e->d_dDT[k].p, nullptr, e->d_mat_off.p,
-                                                                          e->d_mat_ld.p, e->nmol, N2);
-            HFG_CUDA(cudaGetLastError());
-        }
     }
-    int launches = nspin - 1;
+    prepare_kernel<<<dim3(grid_for(N2, 256, e->num_sms), nspin), 256, 0, s>>>(spin_set(e, false), e->d_mat_off.p, e->d_mat_ld.p,
+                                                                            e->nmol, N2);
+    HFG_CUDA(cudaGetLastError());
+    int launches = 1;
     // The classes side by side: each streams its own blocks, and the small ones fill the tails of the large.
     SideStreams side(e, 0, s);
     for (int qc = kNumQuartetClasses - 1; qc >= 0; --qc)
@@ -2070,13 +2094,10 @@ static void fock_conventional(hfg_engine* e, const hfg_fock_request& r, hfg_fock
     }
     side.join();
     double* outs[3] = {r.J, r.K_alpha, r.K_beta};
-    for (int k = 0; k < nspin; ++k)
-    {
-        symmetrize_kernel<<<grid_for(N2, 256, e->num_sms), 256, 0, s>>>(e->d_acc[k].p, e->d_out[k].p, e->d_mat_off.p,
-                                                                          e->d_mat_ld.p, e->nmol, N2);
-        HFG_CUDA(cudaGetLastError());
-        ++launches;
-    }
+    symmetrize_kernel<<<dim3(grid_for(N2, 256, e->num_sms), nspin), 256, 0, s>>>(spin_set(e, false), e->d_mat_off.p,
+                                                                               e->d_mat_ld.p, e->nmol, N2);
+    HFG_CUDA(cudaGetLastError());
+    ++launches;
     HFG_CUDA(cudaEventRecord(e->ev[6], s));
     for (int k = 0; k < nspin; ++k)
         HFG_CUDA(cudaMemcpyAsync(outs[k], e->d_out[k].p, sizeof(double) * N2,
