@@ -30,11 +30,11 @@ constexpr int P2 = QC - P1 * (P1 + 1) / 2;
 constexpr int LA = pair_class_l1(P1), LB = pair_class_l2(P1), LC = pair_class_l1(P2), LD = pair_class_l2(P2);
 constexpr int NAB = ncart(LA) * ncart(LB), NCD = ncart(LC) * ncart(LD);
 constexpr int L   = LA + LB + LC + LD;
-// Kernel form per class and precision, from the ptxas footprint of the thread-per-quartet form
-// (sm_103a, -O3): thread-per-quartet where its stack frame stays at or below ~1.2 KB, the
-// warp-cooperative form for the larger d classes.
-//   FP64 warp: (dp|pp) (dp|ds) (dp|dp) (dd|ps) (dd|pp) (dd|ds) (dd|dp) (dd|dd)   = classes 12-14, 16-20
-//   FP32 warp: (dp|dp) (dd|pp) (dd|ds) (dd|dp) (dd|dd)                           = classes 14, 17-20
+// Classes with the warp-cooperative form instead of the thread form (whose ptxas stack frame would exceed ~1.2 KB in
+// sm_103a code at -O3):
+//   FP64: (dp|pp) (dp|ds) (dp|dp) (dd|ps) (dd|pp) (dd|ds) (dd|dp) (dd|dd)   = classes 12-14, 16-20
+//   FP32: (dp|dp) (dd|pp) (dd|ds) (dd|dp) (dd|dd)                           = classes 14, 17-20
+// In FP64 all but (dd|dd) run the chunk form below; the warp form evaluates their stored integrals.
 constexpr bool warp_form(bool fp32)
 {
     return fp32 ? (QC == 14 || QC >= 17) : (QC == 12 || QC == 13 || QC == 14 || QC >= 16);

@@ -9,7 +9,7 @@
 // Device data layout (HBM):
 //   pairs       PairRec per shell pair (a >= b within a molecule), oriented so l(sh1) >= l(sh2), by pair
 //               id and, after the Schwartz sort, in sorted-list order (spairs; the lists hold those indices)
-//   pptab64/32  per pair class, primitive-pair records of pp_stride(l1,l2) values (p, P, W, 1/p, E3),
+//   pptab64/32  per pair class, primitive-pair records of pp_stride(l1,l2) values (p, P, W, index of p, E3),
 //               renumbered in sorted order after the sort, and a field-major copy (ksoa) for the thread
 //               kernels' ket reads; primitive pairs below the screening bound are left out
 //   cls_*       per pair class, pair ids sorted by (molecule, primitive-pair count desc, Q desc), with
@@ -18,7 +18,8 @@
 //   matrices    per molecule n x n column-major blocks, concatenated (dD, X, Y, J, K)
 //
 // Streams: `stream` carries a build; mixed builds run the FP32 class kernels on stream2 concurrently with
-// the FP64 ones (fork after the list build, join before the symmetrisation).
+// the FP64 ones (fork after the list build, join before the symmetrisation); the class kernels of short lists
+// run side by side on eight side streams per precision (SideStreams).
 #include "engine.h"
 #include "eri_grad.cuh"
 #include "hfgpu.h"
@@ -1523,6 +1524,7 @@ constexpr unsigned long long kTuneMin    = 1ull << 16;
 constexpr unsigned long long kTuneSample = 1ull << 21;
 constexpr unsigned long long kTuneChunks = 16;
 constexpr int kTuneReps                  = 2;
+constexpr unsigned long long kWarpMost   = 1024; // quartets of a dd list that one wave of warps holds
 
 int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base, double* ms_tune)
 {
@@ -1544,6 +1546,10 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
     // loses in every class (12 to 53 ms of a 346 ms FP64 build of (H2O)_27/6-31G**).
     const unsigned tried       = prec == 0 ? mask & ~(1u << kFormGroup) : mask;
     const unsigned long long n = base.count_host;
+    // A short FP64 list of a dd class: its 6 to 18 chunk launches take as long as each other whatever they hold, one
+    // launch with a warp per quartet a wave of some 0.2 to 0.4 ms (two waters UHF/cc-pVDZ: 1.59 -> 0.96 ms a build).
+    if (prec == 0 && qc >= 17 && n < kWarpMost && ((mask >> kFormWarp) & 1u))
+        return kFormWarp;
     if (n < kTuneMin || !e->autotune || (tried & (tried - 1)) == 0)
         return 0; // too small to time, or tuning off: the default form runs and the class stays untuned
     const auto t0 = std::chrono::steady_clock::now();

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(32 * kGradWarps)
     const unsigned long long m = split_share(sp.prims, sp.lanes, sp.next != nullptr);
     unsigned long long round = 0, it = 0, end = 0;
     while (take_items(sp, items, (static_cast<unsigned long long>(blockIdx.x) * kGradWarps + wib) * NG + grp,
-                      static_cast<unsigned long long>(gridDim.x) * kGradWarps * NG, false, gmask, grp * GS, nullptr, round, it, end))
+                      static_cast<unsigned long long>(gridDim.x) * kGradWarps * NG, gmask, grp * GS, round, it, end))
     for (; it < end; ++it)
     {
         const Quartet qt  = list[it >> ls];
@@ -473,8 +473,7 @@ __global__ void __launch_bounds__(128)
     const int lane = threadIdx.x & 31;
 
     unsigned long long round = 0, it = 0, end = 0;
-    while (take_items(sp, items, blockIdx.x * 4ull + (threadIdx.x >> 5), gridDim.x * 4ull, false, 0xffffffffu, 0, nullptr, round,
-                      it, end))
+    while (take_items(sp, items, blockIdx.x * 4ull + (threadIdx.x >> 5), gridDim.x * 4ull, 0xffffffffu, 0, round, it, end))
     for (; it < end; ++it)
     {
         const unsigned long long base = (it >> ls) * 32;

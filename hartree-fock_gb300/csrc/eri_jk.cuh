@@ -674,23 +674,13 @@ __device__ __forceinline__ int split_lanes(int P, unsigned long long m, int smax
 }
 
 // Takes the next run of items [at, end) of `units`; false at the end of the list.  `who`: this taker's number
-// of `takers` (static order); `lead`: the lane that asks the counter, whose answer the mask's lanes share.
-// by_block: the whole block takes one run (through `box` in shared memory), else every mask's lanes theirs.
+// of `takers` (round robin); `lead`: the lane that asks the counter, whose answer the mask's lanes share.
 __device__ __forceinline__ bool take_items(const SplitArgs& sp, unsigned long long units, unsigned long long who,
-                                           unsigned long long takers, bool by_block, unsigned mask, int lead,
-                                           unsigned long long* box, unsigned long long& round, unsigned long long& at,
-                                           unsigned long long& end)
+                                           unsigned long long takers, unsigned mask, int lead, unsigned long long& round,
+                                           unsigned long long& at, unsigned long long& end)
 {
     if (sp.next == nullptr)
         at = (round++ * takers + who) * sp.run;
-    else if (by_block)
-    {
-        __syncthreads(); // every warp has read the last answer
-        if (threadIdx.x == 0)
-            *box = atomicAdd(sp.next, static_cast<unsigned long long>(sp.run));
-        __syncthreads();
-        at = *box;
-    }
     else
     {
         if ((threadIdx.x & 31) == lead)
@@ -811,11 +801,12 @@ __device__ __forceinline__ void class_body(const Quartet* __restrict__ list, uns
     // the digestion may sum the bra block over the warp.  With S >= 64 the four warps of a block take slices of
     // one window, so that they may share a quartet (G = 64, 128): their branches on G are block-uniform.
     // Runs keep the windows of one bra pair together, whose rows of D and records are then found in L1.
-    __shared__ unsigned long long box;
-    const bool by_block = S >= 64; // the four warps of a block share a quartet (G = 64, 128)
+    // The four warps of a block may share a quartet (G = 64, 128) and so walk together; lists that long in windows
+    // split to at most 32 (plan_items), so these go round robin.
+    const bool by_block = S >= 64;
     unsigned long long round = 0, at = 0, end = 0;
     while (take_items(sp, by_block ? items / 4 : items, by_block ? blockIdx.x : blockIdx.x * 4ull + wib,
-                      by_block ? gridDim.x : gridDim.x * 4ull, by_block, 0xffffffffu, 0, &box, round, at, end))
+                      by_block ? gridDim.x : gridDim.x * 4ull, 0xffffffffu, 0, round, at, end))
     for (; at < end; ++at)
     {
         const unsigned long long it = by_block ? at * 4 + wib : at;
