@@ -387,11 +387,15 @@ template <int ND, int KL0, int KL1> __host__ __device__ constexpr bool chunk_has
 }
 
 // 2x and |x| < thr without the FP64 pipe in FP64 (thr >= 0; IEEE bit patterns of non-negative numbers order
-// like the numbers, a NaN is above any thr).  Doubling drops subnormals.
+// like the numbers, a NaN is above any thr).  Doubling drops subnormals, keeps infinities and NaN, and the
+// largest binade becomes an infinity.
 __device__ __forceinline__ double twice(double x)
 {
-    const long long b = __double_as_longlong(x);
-    return (b & 0x7ff0000000000000ll) == 0 ? 0.0 : __longlong_as_double(b + 0x0010000000000000ll);
+    const int hi = __double2hiint(x), e = hi & 0x7ff00000;
+    const bool top = e >= 0x7fe00000, sub = e == 0;
+    const int h2   = e == 0x7ff00000 ? hi : top ? (hi & 0x80000000) | 0x7ff00000 : hi + 0x00100000;
+    const int l2   = e == 0x7fe00000 ? 0 : __double2loint(x);
+    return __hiloint2double(sub ? 0 : h2, sub ? 0 : l2);
 }
 __device__ __forceinline__ float twice(float x) { return 2.0f * x; }
 __device__ __forceinline__ bool below(double x, double thr)

@@ -70,6 +70,17 @@ def test_gpu_split_matches_forced_forms(port):
         assert np.max(np.abs(a - b)) <= 1e-10
 
 
+@pytest.mark.parametrize("system", ["O", "3"])
+@pytest.mark.parametrize("value", [np.inf, -np.inf])
+def test_gpu_infinite_density_reaches_j(port, system, value):
+    """No threshold: every element of J holds a multiple of the infinite element of D (0 times it is a NaN)."""
+    e, B, _, _, _ = _setup(port, "6-31G", system)
+    D = np.zeros((B.nao, B.nao))
+    D[0, 0] = value
+    J = e.fock(D, D, sthr=0.0, dthr=0.0)[0]
+    assert not np.isfinite(J).any()
+
+
 @pytest.mark.parametrize("shells", [(4, 4, 4, 4), (5, 4, 4, 0), (5, 5, 5, 5), (6, 5, 5, 4), (6, 5, 6, 5), (6, 6, 6, 6)])
 def test_gpu_store_mode_matches_oracle(port, shells):
     """One quartet alone in store mode against the oracle's integrals, where the oracle states them (with equal
