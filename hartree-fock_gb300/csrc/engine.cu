@@ -442,7 +442,7 @@ struct ClassBuild
     unsigned long long* bra_off;   // [kListSeqs][n1] exclusive offsets inside the sequence
     unsigned long long* seq_tot;   // [kListSeqs] lengths
     const unsigned* group_off;     // [n1 + 1] first candidate group of every bra pair
-    uint4* groups;                 // first ket position | ket bucket << 28; near FP64, far FP64 and FP32 survivors of
+    uint4* groups;                 // first ket position | ket bucket << 29; near FP64, far FP64 and FP32 survivors of
                                    // 32 candidates (bits)
     Quartet* out64;
     Quartet* out32;
@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) test_lists_kernel(const __gr
             if (lane == 0)
             {
                 if (group < last)
-                    a.groups[group] = make_uint4(static_cast<unsigned>(base) | bucket << 28, m64, mfar, m32);
+                    a.groups[group] = make_uint4(static_cast<unsigned>(base) | bucket << 29, m64, mfar, m32);
                 keys[2 * bucket] += __popc(m64);
                 keys[2 * bucket + 1] += __popc(mfar);
             }
@@ -633,8 +633,8 @@ __global__ void __launch_bounds__(32 * kBuildWarps) write_lists_kernel(const __g
         for (; some; some &= some - 1)
         {
             const int k          = __ffs(static_cast<int>(some)) - 1;
-            const unsigned x     = __shfl_sync(0xffffffffu, own.x, k), j = (x & 0x0fffffffu) + lane;
-            const int key        = 2 * static_cast<int>(x >> 28);
+            const unsigned x     = __shfl_sync(0xffffffffu, own.x, k), j = (x & 0x1fffffffu) + lane;
+            const int key        = 2 * static_cast<int>(x >> 29);
             const unsigned mnear = __shfl_sync(0xffffffffu, own.y, k), mfar = __shfl_sync(0xffffffffu, own.z, k),
                            m32   = __shfl_sync(0xffffffffu, own.w, k);
             const Quartet qv {static_cast<uint32_t>(a.base1 + i), static_cast<uint32_t>(a.base2) + j};
@@ -1375,6 +1375,8 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
         for (int P2 = 0; P2 <= P1; ++P2)
         {
             const int qc = quartet_class(P1, P2);
+            if (e->cls_ids[P2].size() > 1u << 29) // a group's first ket position has 29 bits
+                throw HfgError(HFG_ERR_OVERFLOW, "fock: too many shell pairs in one class");
             unsigned long long c = 0, groups = 0;
             std::vector<unsigned> group_off(1, 0u);
             group_off.reserve(e->cls_ids[P1].size() + 1);
