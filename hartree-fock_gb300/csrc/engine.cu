@@ -52,13 +52,18 @@ struct HfgError : std::runtime_error
     HfgError(int c, const std::string& m) : std::runtime_error(m), code(c) {}
 };
 
+// The runtime keeps an error until it is asked for: taken here, or the launch check of the next call, which may
+// well succeed, would report it.
 #define HFG_CUDA(call)                                                                                               \
     do                                                                                                               \
     {                                                                                                                \
         cudaError_t e_ = (call);                                                                                     \
         if (e_ != cudaSuccess)                                                                                       \
+        {                                                                                                            \
+            cudaGetLastError();                                                                                      \
             throw HfgError(e_ == cudaErrorMemoryAllocation ? HFG_ERR_NOMEM : HFG_ERR_CUDA,                           \
                            std::string(#call) + ": " + cudaGetErrorString(e_));                                      \
+        }                                                                                                            \
     } while (0)
 
 template <typename T> struct DevBuf

@@ -53,7 +53,10 @@ struct ScfError : std::runtime_error
 void ck(cudaError_t e, const char* what)
 {
     if (e != cudaSuccess)
+    {
+        cudaGetLastError(); // not left for the launch check of a later call
         throw ScfError(e == cudaErrorMemoryAllocation ? HFG_ERR_NOMEM : HFG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+    }
 }
 void ck(cublasStatus_t e, const char* what)
 {
