@@ -596,6 +596,8 @@ __global__ void __launch_bounds__(32 * kBuildWarps) test_lists_kernel(const __gr
             p32 += pp * __popc(m32);
         }
     }
+    // write_lists_kernel expands every record up to `last`, whatever the search above came to.
+    for (unsigned g = group + lane; g < last; g += 32) a.groups[g] = make_uint4(0u, 0u, 0u, 0u);
     __syncwarp();
     if (lane < kListSeqs)
         a.bra_cnt[static_cast<size_t>(lane) * a.n1 + i] = lane < kListKeys ? keys[lane] : c32;
@@ -1376,6 +1378,9 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
     if (e->cap_thr == sthr && (!mixed || e->cap_mixed))
         return;
     invalidate_graph(e);
+    // Sized class by class: after a failure between two of them the lists belong to no threshold.
+    e->cap_thr   = -1.0;
+    e->cap_mixed = false;
     for (int P1 = 0; P1 < kNumPairClasses; ++P1)
         for (int P2 = 0; P2 <= P1; ++P2)
         {

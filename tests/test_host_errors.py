@@ -67,3 +67,16 @@ e.fock(D, D, sthr=loose)
 failing(int(sys.argv[2]), e.fock, D, D, sthr=tight)
 e.fock(D, D, sthr=tight)
 """, succeed)
+
+
+@pytest.mark.parametrize("succeed", [0, 3, 11, 20])
+@pytest.mark.parametrize("retry", ["the earlier threshold", "the failed one"])
+def test_failed_sizing_of_the_lists_is_not_kept(run, succeed, retry):
+    """Lists are sized class by class; a call that fails between two classes leaves some of them sized for its own
+    threshold, so the next call, at whichever threshold, sizes all of them again."""
+    run("""
+first, again = uploads(e.fock, D, D, sthr=loose), uploads(e.fock, D, D, sthr=loose)
+assert first > again  # the second call keeps the lists
+failing(int(sys.argv[2]), e.fock, D, D, sthr=tight)
+assert uploads(e.fock, D, D, sthr=loose if sys.argv[3] == "the earlier threshold" else tight) == first
+""", succeed, retry)
