@@ -1379,8 +1379,9 @@ static void size_lists(hfg_engine* e, double sthr, bool mixed)
         return;
     invalidate_graph(e);
     // Sized class by class: after a failure between two of them the lists belong to no threshold.
-    e->cap_thr   = -1.0;
-    e->cap_mixed = false;
+    e->cap_thr    = -1.0;
+    e->cap_mixed  = false;
+    e->last_valid = false; // new buffers: the last build's quartets are gone
     for (int P1 = 0; P1 < kNumPairClasses; ++P1)
         for (int P2 = 0; P2 <= P1; ++P2)
         {

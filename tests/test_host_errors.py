@@ -80,3 +80,20 @@ assert first > again  # the second call keeps the lists
 failing(int(sys.argv[2]), e.fock, D, D, sthr=tight)
 assert uploads(e.fock, D, D, sthr=loose if sys.argv[3] == "the earlier threshold" else tight) == first
 """, succeed, retry)
+
+
+def test_survivors_of_lists_that_are_gone_are_refused(run):
+    """A call that fails while it sizes the lists has given the last build's lists back already."""
+    run("""
+e.fock(D, D, sthr=loose)
+e.survivors()
+failing(3, e.fock, D, D, sthr=tight)
+try:
+    e.survivors()
+except engine.HfgError as x:
+    assert x.code == -1, x  # HFG_ERR_INVALID
+else:
+    raise SystemExit("survivors read from new buffers")
+e.fock(D, D, sthr=loose)
+e.survivors()
+""")
