@@ -450,7 +450,7 @@ template <int N> __device__ __forceinline__ void warp_sum_spread(double* x, int 
 // 1 for most quartets) are applied before the contraction, without the FP64 pipe where nothing is to scale.
 // bra_warp: every lane of the warp calls this together and all active lanes hold the same bra pair;
 // the bra's Coulomb block X_ab is then summed over the warp and added once (inactive lanes pass
-// active = false and acc = 0).  Otherwise each active lane adds its own.
+// active = false and acc = 0, and add nothing).  Otherwise each active lane adds its own.
 template <int LA, int LB, int LC, int LD, typename Real, bool UHF, int KL0 = 0, int KL1 = ncart(LC) * ncart(LD),
           bool Normalised = false>
 __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec& ket, bool same_pair, const Real* acc,
@@ -572,8 +572,11 @@ __device__ __forceinline__ void digest_loaded(const PairRec& bra, const PairRec&
     }
     if (bra_warp)
     {
-        // Warp sum of the bra block, then one atomic per element from lane 0.
+        // Warp sum of the bra block, then one atomic per element from lane 0.  A lane without integrals of its own
+        // has loaded a quartet's densities all the same, and 0 times an infinite one is a NaN.
         const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int x = 0; x < NAB; ++x) Jab[x] = active ? Jab[x] : Real(0);
         if constexpr (sizeof(Real) == 8)
         {
             double t1, t2;

@@ -81,6 +81,21 @@ def test_gpu_infinite_density_reaches_j(port, system, value):
     assert not np.isfinite(J).any()
 
 
+@pytest.mark.parametrize("atoms", [2, 12, 16, 24])
+def test_gpu_infinite_density_is_infinite_in_j_and_k(atoms):
+    """s functions with positive coefficients: every integral is positive, so one infinite element of D makes all of
+    J and K +inf, whether a quartet has 128 lanes, some of a warp's, or one, and in a window that is not full."""
+    from hfgpu import basis
+    from hfgpu.engine import Engine
+
+    xyz = np.array([(x, y, z) for x in range(4) for y in range(3) for z in range(2)][:atoms], float) * 2.0
+    e = Engine(basis.pack("STO-6G", [1] * atoms, xyz))
+    D = np.zeros((atoms, atoms))
+    D[0, 0] = np.inf
+    J, K, _, _ = e.fock(D, D, sthr=0.0, dthr=0.0)
+    assert (J == np.inf).all() and (K == np.inf).all()
+
+
 @pytest.mark.parametrize("shells", [(4, 4, 4, 4), (5, 4, 4, 0), (5, 5, 5, 5), (6, 5, 5, 4), (6, 5, 6, 5), (6, 6, 6, 6)])
 def test_gpu_store_mode_matches_oracle(port, shells):
     """One quartet alone in store mode against the oracle's integrals, where the oracle states them (with equal
