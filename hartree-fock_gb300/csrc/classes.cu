@@ -91,11 +91,13 @@ template <typename Real> SplitArgs split_args(const ClassLaunch& c)
 }
 
 // Sets the split for the list's longest quartet (pmax) and the order its items are taken in, for `cap` resident
-// blocks of `warps` warps (each `per` windows or groups wide) and `windows` of them; returns the blocks to launch.
-// Up to four waves of blocks go round robin, more through the counter `next`.
+// blocks that take `per_block` windows or groups each, and at most `windows` of them; returns the blocks to launch.
+// Up to four waves of blocks go round robin, more through the counter `next`; `expected` windows decide that (a captured
+// build's grid holds every quartet that the thresholds allow, its lists a tenth of them, and in runs of four windows
+// those kept a quarter of the warps busy: 2.22 ms a replay of the mixed build of (H2O)_4/6-31G**, 1.79 ms eager).
 inline unsigned long long plan_items(SplitArgs& s, bool split, unsigned long long pmax, unsigned long long windows,
-                                     unsigned per_block, unsigned long long cap, unsigned long long* next, cudaStream_t stream,
-                                     cudaError_t& err)
+                                     unsigned long long expected, unsigned per_block, unsigned long long cap,
+                                     unsigned long long* next, cudaStream_t stream, cudaError_t& err)
 {
     err             = cudaSuccess;
     auto warps_for = [&](bool queued, int most) {
@@ -106,7 +108,7 @@ inline unsigned long long plan_items(SplitArgs& s, bool split, unsigned long lon
     };
     s.smax                  = warps_for(false, 128);
     unsigned long long need = (windows * s.smax + per_block - 1) / per_block;
-    if (next == nullptr || need <= 4 * cap)
+    if (next == nullptr || (expected * s.smax + per_block - 1) / per_block <= 4 * cap)
     {
         s.run = 1;
         return need < cap ? need : cap;
@@ -119,6 +121,8 @@ inline unsigned long long plan_items(SplitArgs& s, bool split, unsigned long lon
     err    = cudaMemsetAsync(next, 0, sizeof(unsigned long long), stream);
     return need < cap ? need : cap;
 }
+
+inline unsigned long long expected_windows(const ClassLaunch& c) { return ((c.listed != 0 ? c.listed : c.count_host) + 31) / 32; }
 
 // Allows the kernel its shared memory and asks how many of its blocks an SM holds, once per engine (`slot`, zero
 // before): the two calls cost more host time than the launch, 72 times in a build of two waters.
@@ -231,7 +235,7 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
                     if (err != cudaSuccess)
                         return;
                     const unsigned long long grid =
-                        plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count_host + 31) / 32, 4,
+                        plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count_host + 31) / 32, expected_windows(c), 4,
                                    static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share),
                                    c.next ? c.next + decltype(C)::value : nullptr, c.stream, err);
                     if (err != cudaSuccess)
@@ -276,7 +280,7 @@ template <typename Real, bool UHF> cudaError_t launch_t(const ClassLaunch& c)
             if (e != cudaSuccess)
                 return e;
             const unsigned long long grid =
-                plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count_host + 31) / 32, 4,
+                plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count_host + 31) / 32, expected_windows(c), 4,
                            static_cast<unsigned long long>(c.num_sms) * resident(per_sm, c.share), c.next, c.stream, e);
             if (e != cudaSuccess)
                 return e;
@@ -370,7 +374,7 @@ template <typename Real> cudaError_t launch_grad_thread(const GradLaunch& c)
     if (e != cudaSuccess)
         return e;
     SplitArgs sp                  = grad_split<Real>(c, 1);
-    const unsigned long long grid = plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count + 31) / 32, 4,
+    const unsigned long long grid = plan_items(sp, sizeof(Real) == 8, c.pmax, (c.count + 31) / 32, (c.count + 31) / 32, 4,
                                                static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1), c.next,
                                                c.stream, e);
     if (e != cudaSuccess)
@@ -394,7 +398,7 @@ template <typename Real> cudaError_t launch_grad_t(const GradLaunch& c)
         return e;
     constexpr unsigned per_block = kGradWarps * (32 / W::kGroup); // quartets in flight per block
     SplitArgs sp                  = grad_split<Real>(c, W::kGroup);
-    const unsigned long long grid = plan_items(sp, sizeof(Real) == 8, c.pmax, c.count, per_block,
+    const unsigned long long grid = plan_items(sp, sizeof(Real) == 8, c.pmax, c.count, c.count, per_block,
                                                static_cast<unsigned long long>(c.num_sms) * (per_sm > 0 ? per_sm : 1), c.next,
                                                c.stream, e);
     if (e != cudaSuccess)

@@ -1537,7 +1537,21 @@ constexpr unsigned long long kTuneMin    = 1ull << 16;
 constexpr unsigned long long kTuneSample = 1ull << 21;
 constexpr unsigned long long kTuneChunks = 16;
 constexpr int kTuneReps                  = 2;
-constexpr unsigned long long kWarpMost   = 1024; // quartets of a dd list that one wave of warps holds
+
+// The form of a class that is neither set nor timed, for a list of n quartets: the class's default, but for short FP64
+// lists of (dd|pp), (dd|ds) and (dd|dp).  Their 6 to 18 chunk launches take as long as each other whatever they hold,
+// one launch with a warp per quartet a wave of some 0.2 to 0.4 ms.  Builds with these three classes chunked and in the
+// warp form: 1.38 and 0.81 ms at 58 / 32 / 30 quartets (two waters cc-pVDZ), 3.10 and 2.81 at 1004 / 872 / 493 (four
+// waters 6-31G**), 4.65 and 4.13 at 972 / 638 / 530, 4.17 and 4.45 at 1851 / 1623 / 880, 12.6 and 13.1 at
+// 3963 / 2658 / 1975.
+constexpr unsigned long long kWarpMost = 1024;
+
+int untimed_form(int qc, int prec, unsigned long long n)
+{
+    if (prec == 0 && qc >= 17 && n < kWarpMost && ((class_form_mask(qc, false) >> kFormWarp) & 1u))
+        return kFormWarp;
+    return class_default_form(qc, prec == 1);
+}
 
 int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base, double* ms_tune)
 {
@@ -1559,12 +1573,8 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
     // loses in every class (12 to 53 ms of a 346 ms FP64 build of (H2O)_27/6-31G**).
     const unsigned tried       = prec == 0 ? mask & ~(1u << kFormGroup) : mask;
     const unsigned long long n = base.count_host;
-    // A short FP64 list of a dd class: its 6 to 18 chunk launches take as long as each other whatever they hold, one
-    // launch with a warp per quartet a wave of some 0.2 to 0.4 ms (two waters UHF/cc-pVDZ: 1.59 -> 0.96 ms a build).
-    if (prec == 0 && qc >= 17 && n < kWarpMost && ((mask >> kFormWarp) & 1u))
-        return kFormWarp;
     if (n < kTuneMin || !e->autotune || (tried & (tried - 1)) == 0)
-        return 0; // too small to time, or tuning off: the default form runs and the class stays untuned
+        return untimed_form(qc, prec, n); // too small to time, or tuning off: the class stays untuned
     const auto t0 = std::chrono::steady_clock::now();
     // FP64 quartets take some ten times as long: an eighth of the sample.
     const unsigned long long most  = prec == 0 ? kTuneSample / 8 : kTuneSample;
@@ -1588,6 +1598,7 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
     t.list        = e->d_tune_list.p;
     t.count_dev   = e->d_tune_cnt.p;
     t.count_host  = m;
+    t.listed      = m;
     t.prims       = static_cast<unsigned long long>(static_cast<double>(base.prims) * (static_cast<double>(m) / static_cast<double>(n)));
     t.prims_dev   = nullptr;
     t.view.X      = e->d_tune_acc[0].p;
@@ -1759,9 +1770,11 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             if (n == 0 || in_queue(qc))
                 continue;
             // In a graph the counts are those of the eager build before the capture: the kernels read the replay's
-            // own on the device, these only size the grids and choose the streams.
+            // own on the device, these only size the splits and choose the streams and forms, as the eager build did.
             const unsigned long long prims = h_prims ? h_prims[2 * qc + prec] : n;
-            const bool is_short = side.is_short(prims) && n < kTuneMin;
+            const unsigned long long ran   = h_prims ? e->h_counts[2 * qc + prec] : 0;
+            const unsigned long long len   = graph && ran != 0 ? ran : n; // (empty then, it may hold any number now)
+            const bool is_short = side.is_short(prims) && len < kTuneMin;
             if (is_short != (pass == 1))
                 continue;
             const int P1 = [&] { int p = 0; while ((p + 1) * (p + 2) / 2 <= qc) ++p; return p; }();
@@ -1789,6 +1802,7 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             c.stream     = is_short ? side.next() : ps;
             c.num_sms    = e->num_sms;
             c.share      = overlap ? (prec == 1 ? e->overlap_share32 : e->overlap_share) : 1.f;
+            c.listed     = len;
             c.pmax       = max_prims(e, P1, P2);
             c.prims_dev  = e->d_counts.p + 2 * kNumQuartetClasses + 2 * qc + prec;
             c.prims      = prims;
@@ -1798,12 +1812,12 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             {
                 const int set  = e->form_set[qc][prec];
                 const int pick = e->form_pick[qc][prec][uhf ? 1 : 0];
-                c.form         = set != 0 ? set : pick;
+                c.form = set != 0 ? set : pick != 0 ? pick : untimed_form(qc, prec, len);
             }
             else
                 c.form = pick_form(e, qc, prec, uhf, c, ms_tune);
             HFG_CUDA(launch_class(qc, c));
-            form_ran[qc][prec] = c.form != 0 ? c.form : class_default_form(qc, prec == 1);
+            form_ran[qc][prec] = c.form;
             launches += class_launches(qc, prec == 1, c.form);
         }
         side.join();

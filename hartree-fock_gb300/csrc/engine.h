@@ -19,7 +19,7 @@ struct ClassLaunch
 {
     const Quartet* list;
     const unsigned long long* count_dev;
-    unsigned long long count_host;
+    unsigned long long count_host; // its length, or the most it can be (a captured build): sizes the grid
     FockView view;
     const void* boys_slice; // slice of the class's total L, Real of the precision
     const void* boys_fast;  // FP64: its BoysFast slice (not used in store mode)
@@ -34,6 +34,7 @@ struct ClassLaunch
     // be null), and the most primitive quartets one quartet of the class can have.
     unsigned long long prims = 0;
     const unsigned long long* prims_dev = nullptr;
+    unsigned long long listed = 0; // the length to choose the order of the items by; 0: count_host
     int pmax = 1;
     unsigned long long* next = nullptr; // kMaxChunks item counters (SplitArgs::next), or null: static order
     int* occ = nullptr; // kOccSlots resident-block counts of the class's kernels, 0: not asked yet (or null)

@@ -188,7 +188,9 @@ int hfg_set_persistent(hfg_engine* engine, int on);
 /* Kernel-form autotuning (no reference counterpart): on (default), the first build that runs a class with at
  * least 64k surviving quartets and more than one compiled form times the forms on a sample of its list and
  * keeps the fastest (hfg_kernel_forms reports the picks); off, every class not set by hfg_set_kernel_form
- * runs its default form, with no timing trials (reproducible launch sequences, e.g. under a profiler). */
+ * runs its default form, with no timing trials (reproducible launch sequences, e.g. under a profiler).  The
+ * default form goes by class, precision and, for FP64 (dd|pp), (dd|ds) and (dd|dp), list length: WARP below 1024
+ * quartets, else CHUNK.  Classes too small to be timed run it too, also in captured builds. */
 int hfg_set_autotune(hfg_engine* engine, int on);
 
 /* Gradient kernel form (no reference counterpart): 0 (default) runs the thread-per-quartet gradient kernel

@@ -209,3 +209,37 @@ def test_gpu_autotune_off_runs_default_forms():
         # 0: untuned (the default form ran); a class with a single compiled form reports that form.
         assert all(f == 0 or (m & (m - 1)) == 0 for f, m in zip(forms, avail))
     assert np.max(np.abs(J1 - J0)) <= 1e-10 and np.max(np.abs(K1 - K0)) <= 1e-10
+
+
+@pytest.mark.parametrize("waters,form", [(2, "FORM_WARP"), (8, "FORM_CHUNK")])
+@pytest.mark.parametrize("uhf", [False, True])
+def test_gpu_short_dd_lists_run_one_form_eager_untuned_and_captured(waters, form, uhf):
+    """The form of an FP64 (dd|pp), (dd|ds) or (dd|dp) list too short to be timed depends on its length alone: the same
+    with tuning on, with tuning off, and in a captured build's replay."""
+    torch = pytest.importorskip("torch")
+    from hfgpu import basis, engine, workloads
+
+    Z, xyz = workloads.water_lattice(2, waters // 2, 1, seed=2) if waters < 8 else workloads.water_lattice(2, 2, 2, seed=2)
+    soa = basis.pack("cc-pVDZ", Z, xyz)
+    n2 = engine.Engine(soa).nao ** 2
+    n = int(round(n2 ** 0.5))
+    P = np.random.default_rng(3).standard_normal((n, n)) * 0.1
+    D = torch.from_numpy((P + P.T).ravel()).cuda()
+    outs = [torch.zeros(n2, dtype=torch.float64, device="cuda") for _ in range(3)]
+    ptrs = dict(dD_tot=D.data_ptr(), dD_alpha=D.data_ptr(), J=outs[0].data_ptr(), K_alpha=outs[1].data_ptr())
+    if uhf:
+        ptrs.update(dD_beta=D.data_ptr(), K_beta=outs[2].data_ptr())
+    torch.cuda.synchronize()
+    ran = {}
+    for mode in ("eager", "untuned", "captured"):
+        e = engine.Engine(soa)
+        if mode == "untuned":
+            e.set_autotune(False)
+        if mode == "captured":
+            e.set_graph_mode(True)
+            e.fock_device(ptrs, unrestricted=uhf)
+        st = e.fock_device(ptrs, unrestricted=uhf)
+        assert all(0 < q < 65536 for q in st["quartets_fp64"][17:20])  # too short to be timed
+        ran[mode] = st["form_fp64"]
+    assert ran["eager"] == ran["untuned"] == ran["captured"]
+    assert ran["eager"][17:20] == [getattr(engine, form)] * 3
