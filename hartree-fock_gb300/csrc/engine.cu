@@ -1569,10 +1569,13 @@ int pick_form(hfg_engine* e, int qc, int prec, bool uhf, const ClassLaunch& base
                 pick = f;
         return pick;
     }
-    // The FP64 group form is not tried: the thread form splits short lists itself, and on long ones the group form
-    // loses in every class (12 to 53 ms of a 346 ms FP64 build of (H2O)_27/6-31G**).
-    const unsigned tried       = prec == 0 ? mask & ~(1u << kFormGroup) : mask;
     const unsigned long long n = base.count_host;
+    // The group form is tried on FP32 lists that are timed whole.  The FP64 thread form splits short lists itself, and on
+    // long lists the group form loses in every class (FP64: 12 to 53 ms of a 346 ms build of (H2O)_27/6-31G**; FP32: all of
+    // (H2O)_27/6-31G takes 6.7 ms in the thread form, 10.8 with (ss|ss) and 12.9 with (ps|ss) in the group form).  On a
+    // sample of a long FP32 list it won all the same: the sample is over before the warps with its longest quartets are.
+    // On whole lists its wins are real (1.30 -> 1.07 ms for (ss|ss) of (H2O)_8/6-31G, 0.7 M quartets, all in FP32).
+    const unsigned tried = prec == 0 || n > kTuneSample ? mask & ~(1u << kFormGroup) : mask;
     if (n < kTuneMin || !e->autotune || (tried & (tried - 1)) == 0)
         return untimed_form(qc, prec, n); // too small to time, or tuning off: the class stays untuned
     const auto t0 = std::chrono::steady_clock::now();

@@ -146,7 +146,7 @@ int hfg_fock_conventional(hfg_engine* engine, const hfg_fock_request* req, hfg_f
 /* Kernel forms of a class kernel.  THREAD: one thread per shell quartet.  WARP: one warp per quartet
  * (the largest d classes).  GROUP: a power-of-two group of lanes per quartet, splitting its primitive
  * quartets (the small contracted classes, L <= 3).  AUTO: on the first build that runs the class with
- * enough quartets, its compiled forms (but the FP64 group form) run on a sample of the real list and the fastest
+ * enough quartets, its compiled forms (GROUP on short FP32 lists only) run on a sample of the real list and the fastest
  * is kept for the life of the engine (per class, precision and RHF/UHF).
  * No reference counterpart: the reference has one CPU loop (src/SCF.cpp:592-728). */
 #define HFG_FORM_AUTO 0

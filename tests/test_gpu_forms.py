@@ -243,3 +243,22 @@ def test_gpu_short_dd_lists_run_one_form_eager_untuned_and_captured(waters, form
         ran[mode] = st["form_fp64"]
     assert ran["eager"] == ran["untuned"] == ran["captured"]
     assert ran["eager"][17:20] == [getattr(engine, form)] * 3
+
+
+@pytest.mark.parametrize("waters,cutoff", [(27, 1e30), (16, 1e30), (27, 2e-4)])
+def test_gpu_tuned_forms_are_not_slower_than_the_defaults(waters, cutoff):
+    """The sample of an FP32 list is timed as the whole list runs: with the forms that it picks a build takes no longer
+    than with the default forms (15 % for what two runs differ)."""
+    from hfgpu import basis, workloads
+    from hfgpu.engine import Engine
+
+    Z, xyz = workloads.water_lattice(3, 3, 3, seed=4)
+    Z, xyz = Z[:3 * waters], xyz[:3 * waters]
+    soa = basis.pack("6-31G", Z, xyz)
+    ms = {}
+    for tuned in (True, False):
+        e = Engine(soa)
+        e.set_autotune(tuned)
+        Da, _ = e.core_guess(Z, xyz, 0, 1)
+        ms[tuned] = min(e.fock(2 * Da, Da, precision=1, fp32_cutoff=cutoff)[3]["ms_total"] for _ in range(6))
+    assert ms[True] <= 1.15 * ms[False], ms
