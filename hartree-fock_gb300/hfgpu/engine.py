@@ -128,6 +128,7 @@ def lib():
         L.hfg_measure_dmma_peak.argtypes = [ip, dpp]
         L.hfg_gradient.argtypes = [vp, ctypes.POINTER(GradRequest), dpp, dpp]
         L.hfg_boys_eval.argtypes = [ip, ip, ip, ctypes.c_longlong, dpp, dpp]
+        L.hfg_boys_scaled.argtypes = [ip, ip, ctypes.c_longlong, dpp, dpp]
         L.hfg_store_integrals.argtypes = [vp, ctypes.c_double, ctypes.POINTER(ctypes.c_size_t)]
         L.hfg_one_electron_gpu.argtypes = [vp, ip, ctypes.POINTER(ctypes.c_int), dpp, dpp, dpp, dpp]
         L.hfg_gradient_one_electron_gpu.argtypes = [vp, ip, ctypes.POINTER(ctypes.c_int), dpp, dpp, dpp, dpp]
@@ -418,6 +419,17 @@ def boys_eval(m_max: int, T, fp32: bool = False, device: int = 0) -> np.ndarray:
     rc = lib().hfg_boys_eval(device, m_max, 1 if fp32 else 0, T.size, _dp(T), _dp(F))
     if rc != HFG_OK:
         raise HfgError(rc, "hfg_boys_eval failed")
+    return F
+
+
+def boys_scaled(m_max: int, c, s, R2, device: int = 0) -> np.ndarray:
+    """c s^m F_m(T), m = 0 .. m_max, T = -s R2 / 2, from the Boys function of the FP64 thread, chunk and gradient
+    kernels; returns (len(c), m_max + 1)."""
+    x = np.ascontiguousarray(np.stack(np.broadcast_arrays(c, s, R2), axis=-1), dtype=np.float64).reshape(-1, 3)
+    F = np.zeros((len(x), m_max + 1))
+    rc = lib().hfg_boys_scaled(device, m_max, len(x), _dp(x), _dp(F))
+    if rc != HFG_OK:
+        raise HfgError(rc, "hfg_boys_scaled failed")
     return F
 
 

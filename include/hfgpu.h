@@ -346,9 +346,12 @@ int hfg_measure_fma_peak(int device, int fp64, double* tflops);
 int hfg_measure_dmma_peak(int device, double* tflops);
 
 /* The device Boys function of the ERI kernels, F_0(T) .. F_m_max(T) for n values of T (host arrays; F is
- * n x (m_max + 1), row-major), evaluated on `device` by the same code the class kernels run (FP32 when
- * fp32 != 0): a known-answer check of Boys::calculateBoys (src/Boys.cpp:14-71).  m_max <= 9, T >= 0. */
+ * n x (m_max + 1), row-major), evaluated on `device` by the code of the FP32 kernels (fp32 != 0) or
+ * of the FP64 warp, lane-group and store kernels: a known-answer check of Boys::calculateBoys (src/Boys.cpp:14-71).  m_max <= 9, T >= 0. */
 int hfg_boys_eval(int device, int m_max, int fp32, long long n, const double* T, double* F);
+/* The same for the FP64 thread, chunk and gradient kernels, which carry the prefactor through the recursion:
+ * c s^m F_m(T), T = -s R2 / 2, for n triples (c, s <= 0, R2 >= 0). */
+int hfg_boys_scaled(int device, int m_max, long long n, const double* c_s_R2, double* F);
 
 /* Library version string. */
 const char* hfg_version(void);
