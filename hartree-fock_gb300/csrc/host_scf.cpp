@@ -943,6 +943,8 @@ class Scf
             float ms = 0.f;
             if (cudaEventElapsedTime(&ms, gev_[0], gev_[1]) == cudaSuccess)
                 ms_fock_ += ms;
+            else
+                cudaGetLastError(); // the events of a capture may not be timed; not left for the next launch check
             ++replays_;
         }
     }

@@ -87,3 +87,20 @@ def test_gpu_graph_mode_scf_energy(name, precision):
     assert abs(r1["e_total"] - r0["e_total"]) <= 1e-9
     if precision == 0:
         assert abs(r1["e_total"] - float(g["e_elec"] + g["e_nuc"])) <= 1e-9
+
+
+@pytest.mark.parametrize("name", ["h2o_631g", "w2_cation_uhf_631gss"])
+def test_gpu_calls_after_graph_iterations_succeed(name):
+    """A graph SCF asks for the time between events that a capture recorded, which CUDA refuses; the refusal is not left
+    for the next call on this or a new engine."""
+    from hfgpu import inputs
+    from hfgpu.engine import Engine
+
+    g = load_golden(name)
+    job = inputs.parse(str(g["input_text"]))
+    e = Engine(g["soa"])
+    res, Da, Db = e.scf(job.Z, job.xyz, job.charge, job.multiplicity, dict(inputs.scf_options(job), graph_iterations=1))
+    assert res["graph_replays"] > 0
+    e.fock(Da + Db, Da, Db)
+    res, Da, Db = e.scf(job.Z, job.xyz, job.charge, job.multiplicity, dict(inputs.scf_options(job), graph_iterations=1))
+    Engine(g["soa"]).fock(Da + Db, Da, Db)
