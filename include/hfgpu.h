@@ -266,7 +266,9 @@ typedef struct hfg_scf_options
     double density_threshold;  /* DENSITY_THRESH (1e-10) */
     int precision;             /* HFG_PRECISION_FP64 / HFG_PRECISION_MIXED */
     double fp32_cutoff;        /* FP32 cutoff of the mixed mode (2e-4) */
-    int full_rebuild_every;    /* 0: incremental builds as the reference; k > 0: full build every k iterations */
+    int full_rebuild_every;    /* 0: incremental builds as the reference, but for one full build (FP64, no graph
+                                  iterations) whenever only the energy has not converged for 24 iterations in a row;
+                                  k > 0: full build every k iterations */
     int verbose;               /* print the iteration table to stdout */
     int graph_iterations;      /* 1: every SCF iteration after the first replays CUDA graphs captured once: the Fock
                                   build, F update, DIIS on the device, X^T F X, the orbital update, energy and

@@ -89,6 +89,32 @@ def test_w16_scf_fp64_energy_matches_reference(w16):
     assert abs(res["e_total"] - float(w16["e_total"])) <= 5e-7, (res["e_total"], float(w16["e_total"]))
 
 
+def test_w16_scf_fp64_energy_is_that_of_its_density(w16, w16_engine):
+    """SCF after SCF (atomics sum in another order each time, so their late iterations differ), each against one full
+    build: the converged density's energy within 1e-8 Eh of the reference density's (the error is second order in the
+    density, converged to 1e-7), and the energy that the SCF reports within 3.5e-7 Eh of its own density's (35 increments at
+    1e-8, the most that one of them moves the energy here: some ten until the density settles, 24 before a full build)."""
+    from hfgpu import inputs
+    from hfgpu.engine import Engine
+
+    job = inputs.parse(str(w16["input_text"]))
+    opts = dict(inputs.scf_options(job, precision=0), max_iter=400)
+    S, T, V = w16_engine.one_electron(w16["Z"], w16["xyz"])
+
+    def electronic(D):
+        J, K, _, _ = w16_engine.fock(2 * D, D)
+        return float(np.sum(D * (2 * (T + V) + J - K)))
+
+    want = electronic(w16["Da_scf"])
+    e = Engine(w16["soa"])
+    e.set_schwartz(w16["Q"])
+    for _ in range(6):
+        res, D, _ = e.scf(job.Z, job.xyz, 0, 1, opts)
+        assert res["converged"] == 1
+        assert abs(electronic(D) - want) <= 1e-8
+        assert abs(res["e_electronic"] - electronic(D)) <= 3.5e-7, res
+
+
 def test_w16_energy_at_reference_density(w16, w16_engine):
     """E = tr(D (h + F)) + E_nuc at the reference's converged density, with the GPU's one-electron integrals
     and one full FP64 Fock build, against the same expression with the reference's F (its incremental build
