@@ -313,6 +313,17 @@ __global__ void to_float_kernel(const double* __restrict__ a, float* __restrict_
         b[i] = static_cast<float>(a[i]);
 }
 
+// ExponentTable (eri_jk.cuh) of the n sums p.  Made on the host, its million square roots and divisions at 990 sums cost an
+// engine 4 ms, 40 FP64 builds' gain for a molecule of H, C, N, O and F in 6-31G.
+__global__ void exponent_table_kernel(const double* __restrict__ p, int n, double2* __restrict__ t)
+{
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)n * n; e += (long long)gridDim.x * blockDim.x)
+    {
+        const double a = p[e / n], b = p[e % n];
+        t[e] = make_double2(1.0 / sqrt(a + b), -2.0 * (a * b) / (a + b));
+    }
+}
+
 // The matrices of a build, total / alpha / beta: one launch serves them all (blockIdx.y), since for a small
 // molecule each launch costs as much as its work.
 struct SpinSet
@@ -1021,14 +1032,12 @@ static void pack_molecules(hfg_engine* e)
             for (size_t j = 0; j < nex; ++j)
                 sum_at[i * nex + j] =
                     static_cast<int>(std::lower_bound(sums.begin(), sums.end(), ex[i] + ex[j]) - sums.begin());
-        std::vector<double2> t(sums.size() * sums.size());
-        for (size_t i = 0; i < sums.size(); ++i)
-            for (size_t j = 0; j < sums.size(); ++j)
-            {
-                const double p = sums[i], q = sums[j];
-                t[i * sums.size() + j] = make_double2(1.0 / std::sqrt(p + q), -2.0 * (p * q) / (p + q));
-            }
-        e->d_exptab.upload(t, e->stream);
+        DevBuf<double> d_sums;
+        d_sums.upload(sums, e->stream);
+        e->d_exptab.alloc(sums.size() * sums.size());
+        exponent_table_kernel<<<grid_for(sums.size() * sums.size(), 256, e->num_sms), 256, 0, e->stream>>>(d_sums.p, e->nexp,
+                                                                                                        e->d_exptab.p);
+        HFG_CUDA(cudaGetLastError());
         HFG_CUDA(cudaStreamSynchronize(e->stream));
     }
     std::vector<std::vector<double>> tab(kNumPairClasses);

@@ -36,7 +36,9 @@ constexpr double kTwoPi25 = 34.98683665524972497; // 2 pi^{5/2}
 // 1/sqrt(p+q) and -2 pq/(p+q) for every two primitive-pair exponents of the basis: they depend on the
 // exponents alone, of which a molecule's pairs have few distinct ones (136 for water in 6-31G**), and cost ten
 // FP64 instructions per primitive quartet to compute against one 16-byte load.  Null where the basis has
-// more than kMaxExponents of them; the kernels compute the two numbers then.
+// more than kMaxExponents of them (16.8 MB); the kernels compute the two numbers then.  FP64 builds with and
+// without the table: 52.3 / 57.5 ms at 136 sums ((H2O)_16/6-31G**), and for 16 H2X with several X 16.8 / 20.6 at 595
+// (C N O, 6-31G), 107 / 118 at 903 (C N O, 6-311G**), 14.9 / 18.2 at 990 (C N O F, 6-31G).
 constexpr int kMaxExponents = 1024;
 struct ExponentTable
 {

@@ -164,3 +164,23 @@ def test_gpu_split_graph_replay_with_another_density(port, basis_name, system):
         Jr, Kr, _, _ = B.fock_direct(Q, 2 * D, D)
         J, K = (o.cpu().numpy().reshape(n, n, order="F") for o in outs)
         assert np.max(np.abs(J - Jr)) <= 1e-10 and np.max(np.abs(K - Kr)) <= 1e-10
+
+
+@pytest.mark.parametrize("basis_name,heavy,sums", [("6-31G", [6, 7, 8], 595), ("6-31G**", [6, 7, 8], 666), ("6-31G", [6, 7, 8, 9], 990)])
+def test_gpu_large_exponent_table_matches_oracle(port, basis_name, heavy, sums):
+    """The table of exponent pairs with several elements, up to near its limit of 1024 sums."""
+    from hfgpu import basis
+    from hfgpu.engine import Engine
+
+    Z = heavy + [1]
+    xyz = np.array([[2.4 * k, 0.3 * k * k, 0.0] for k in range(len(Z))])
+    soa = basis.pack(basis_name, Z, xyz)
+    a = np.unique(soa["alpha"])
+    assert len(np.unique(a[:, None] + a[None, :])) == sums
+    e, B = Engine(soa), port.Basis(soa)
+    Q = B.schwartz()
+    e.set_schwartz(Q)
+    D = _sym(B.nao, 4)
+    J, K, _, _ = e.fock(2 * D, D)
+    Jr, Kr, _, _ = B.fock_direct(Q, 2 * D, D, None)
+    assert np.max(np.abs(J - Jr)) <= 1e-10 and np.max(np.abs(K - Kr)) <= 1e-10
