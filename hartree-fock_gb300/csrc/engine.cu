@@ -1446,7 +1446,7 @@ static SpinSet spin_set(hfg_engine* e, bool mixed)
 }
 
 // Screening and the survival lists of every quartet class from the densities already in d_dD[0..2]
-// (the shell-pair maxima, then count pass, scan and write pass per class).  Returns the launches.
+// (the shell-pair maxima, then test, scan and write passes over all classes).  Returns the launches.
 // graph: enqueue only (no host synchronisation); the counts go to the pinned buffer, checked after replay.
 static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double dthr, double cutoff, bool graph = false,
                        bool keyed = true)
@@ -1460,7 +1460,6 @@ static int build_lists(hfg_engine* e, bool uhf, bool mixed, double sthr, double 
         e->d_nsh.p, e->d_shnao.p);
     HFG_CUDA(cudaGetLastError());
 
-    // Lists: count pass, scan, write pass, per quartet class.
     const int ncnt = kNumQuartetClasses * 2;
     e->d_counts.alloc(2 * ncnt + 1);
     e->d_seq_tot.alloc(kNumQuartetClasses * kListSeqs);
@@ -1796,16 +1795,7 @@ static int enqueue_build(hfg_engine* e, const hfg_fock_request& r, bool graph, i
             c.list       = e->d_list[qc][prec].p;
             c.count_dev  = e->d_counts.p + 2 * qc + prec;
             c.count_host = n;
-            c.view       = base_view(e, prec == 1);
-            c.view.pairs = e->d_spairs.p;
-            c.view.Dt    = prec == 1 ? static_cast<const void*>(e->d_dDf[0].p) : e->d_dD[0].p;
-            c.view.Da    = prec == 1 ? static_cast<const void*>(e->d_dDf[1].p) : e->d_dDT[1].p;
-            c.view.Db    = prec == 1 ? static_cast<const void*>(e->d_dDf[2].p) : e->d_dDT[2].p;
-            c.view.X     = e->d_acc[0].p;
-            c.view.Ya    = e->d_acc[1].p;
-            c.view.Yb    = e->d_acc[2].p;
-            c.view.ao_thr = r.schwartz_threshold;
-            c.view.ao_thr_f = static_cast<float>(r.schwartz_threshold);
+            c.view       = make_view(prec);
             c.boys_slice = prec == 1 ? static_cast<const void*>(e->d_boys32[L].p) : e->d_boys64[L].p;
             c.boys_fast  = e->d_boysf[L].p;
             c.tables     = e->d_tables.p;
