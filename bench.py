@@ -13,7 +13,8 @@ SCHWARTZ_THRESH = DENSITY_THRESH = 1e-10.  A step = one hfg_fock_direct call.
 * fp64_*     the plain all-FP64 GPU build on the same density, and the energy difference of the two
              builds' two-electron energies.
 * roofline   the dominant kernel group (the FP64 ERI class kernels), achieved algorithmic FP64 FLOP/s
-             (engine work model) over their CUDA-event time, against the FP64 FMA peak this run measures.
+             (class_flops: non-zero Hermite coefficients only) over their CUDA-event time, against the FP64
+             FMA peak this run measures.
 * scf        (N=1) full RHF SCFs of the workload, mixed and FP64 (wall time, iterations, |dE|), and the
              mixed-precision nuclear gradient after the mixed SCF; --scf adds the UHF doublet and the FP64
              gradient, --no-scf skips them.
@@ -45,12 +46,40 @@ for _p in (REPO, os.path.join(REPO, "hartree-fock_gb300")):
 
 METRIC = "Fock builds/s & SCF time, (H2O)_64/6-31G**: mixed vs FP64 GPU, |ΔE|≤1e-6 Eh"
 # DRAM traffic per mixed build of the ERI class kernels, measured with ncu on the default kernel forms.
-ERI_DRAM_BYTES_PER_BUILD = {"h2o64": 12.45e9}
+ERI_DRAM_BYTES_PER_BUILD = {"h2o64": 14.28e9}
 WORKLOADS = {
     "h2o64": dict(lattice=(4, 4, 4), basis="6-31G**", name="(H2O)_64 RHF/6-31G** direct Fock build (1600 bf)"),
     "h2o32": dict(lattice=(4, 4, 2), basis="6-31G**", name="(H2O)_32 RHF/6-31G** direct Fock build (800 bf)"),
     "h2o16": dict(lattice=(4, 2, 2), basis="6-31G**", name="(H2O)_16 RHF/6-31G** direct Fock build (400 bf)"),
 }
+
+
+def class_flops():
+    """Per quartet class (la lb|lc ld): flops of a primitive quartet and of a quartet's RHF digestion.  A primitive quartet
+    is the R recursion (one FMA per R^n_tuv), the two Hermite -> Cartesian transforms over the non-zero coefficients
+    E^{ij}_tuv alone (t <= i + j along each axis), and 2 (L + 1) + 10 for the Boys function and the scalars.
+    (The engine's own flops_fp64 counts the Hermite blocks as dense, up to five times as many in the d classes.)"""
+    import math
+
+    cart = lambda l: [(l - y - z, y, z) for x in range(l, -1, -1) for z in range(l - x + 1) for y in [l - x - z]]
+    herm = lambda l: math.comb(l + 3, 3)
+    pairs = []
+    for l1 in range(3):
+        for l2 in range(l1 + 1):
+            nnz = [math.prod(p + q + 1 for p, q in zip(a, b)) for a in cart(l1) for b in cart(l2)]
+            pairs.append((l1 + l2, len(nnz), sum(nnz)))
+    out = []
+    for P1 in range(len(pairs)):
+        for lc, ncd, zcd in pairs[:P1 + 1]:
+            lb, nab, zab = pairs[P1]
+            L = lb + lc
+            out.append((2 * math.comb(L + 4, 4) + 2 * herm(lb) * zcd + 2 * ncd * zab + 2 * (L + 1) + 10, 12 * nab * ncd))
+    return out
+
+
+def build_flops(st, prec):
+    return sum(p * np_ + d * nq for (p, d), np_, nq in
+               zip(class_flops(), st["prim_quartets_" + prec], st["quartets_" + prec]))
 
 
 def parse_args():
@@ -393,9 +422,10 @@ def gpu_arm(args, dist):
     # is weighed as (F64/peak64 + F32/peak32) over their common span, expressed as FP64-equivalent FLOP/s
     # against the FP64 peak.  The FP64 kernels alone are measured in the plain FP64 build.
     t_mix = st["ms_eri_both"] if st["ms_eri_both"] > 0 else st["ms_eri_fp64"] + st["ms_eri_fp32"]
-    ach_mix = (st["flops_fp64"] + st["flops_fp32"] * peak64 / peak32) / (t_mix * 1e-3) / 1e12 if t_mix > 0 else 0.0
-    ach64 = st64["flops_fp64"] / (st64["ms_eri_fp64"] * 1e-3) / 1e12 if st64["ms_eri_fp64"] > 0 else 0.0
-    ach32 = st["flops_fp32"] / (st["ms_eri_fp32"] * 1e-3) / 1e12 if st["ms_eri_fp32"] > 0 else 0.0
+    work64, work32 = build_flops(st, "fp64"), build_flops(st, "fp32")
+    ach_mix = (work64 + work32 * peak64 / peak32) / (t_mix * 1e-3) / 1e12 if t_mix > 0 else 0.0
+    ach64 = build_flops(st64, "fp64") / (st64["ms_eri_fp64"] * 1e-3) / 1e12 if st64["ms_eri_fp64"] > 0 else 0.0
+    ach32 = work32 / (st["ms_eri_fp32"] * 1e-3) / 1e12 if st["ms_eri_fp32"] > 0 else 0.0
 
     out = None
     if dist.rank == 0:
