@@ -343,8 +343,8 @@ namespace
 //     still takes 5.5 ms of a (H2O)_16 6-31G** gradient against 13.6 in the lane-group form);
 //   FP64, other kets: (ds|pp), (ds|ds) and (pp|pp) ((H2O)_8 cc-pVDZ 18.5 -> 15.5 ms, (H2O)_16 9.0 -> 9.8);
 //   FP32: up to 160 values ((pp|ps) (ds|ps) (dp|ss) and smaller), and to 300 with d shells: (ds|pp) (ds|ds) (dp|ps)
-//     (dd|ss), 38 -> 7 ms of a (H2O)_16 gradient.  (pp|pp) stays as it is: sums of FP32 terms in another order
-//     are 1e-9 of a 6-31G gradient away.
+//     (dd|ss), 38 -> 7 ms of a (H2O)_16 gradient.  (pp|pp) is not in it: with it mixed gradients in 6-31G take
+//     5.2 ms for 5.6 ((H2O)_8) and 66.4 for 72.1 ((H2O)_27), but its error against the lane-group form is not measured.
 template <typename Real> constexpr bool grad_thread_form()
 {
     using W = GradThread<LA, LB, LC, LD>;

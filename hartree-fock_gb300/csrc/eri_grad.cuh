@@ -20,7 +20,7 @@
 // and g_D = -(g_A + g_B + g_C) (translational invariance): the Gamma contractions run once per primitive
 // pair, not once per primitive quartet, at the price of evaluating R twice.  E/R tables are recomputed here, nothing from
 // the forward build is stored.  FP64, or FP32 for the small-bound quartets of a mixed-precision gradient
-// (FP64 accumulation).  One group of lanes per quartet (GradLayout::kGroup: 4 to 32 lanes by
+// (their sums over quartets in FP64).  One group of lanes per quartet (GradLayout::kGroup: 4 to 32 lanes by
 // class size; the groups of a warp work independently, synchronised by group masks).
 #pragma once
 
@@ -792,35 +792,51 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
                 for (int x = 0; x < 3; ++x) gA[x] = gP[x] = gC[x] = Real(0);
         }
-        // g_B = g_P - g_A, g_D = -(g_P + g_C); the bra atoms' terms summed over the warp when it shares the bra.
+        // g_B = g_P - g_A, g_D = -(g_P + g_C); the bra atoms' terms summed over the warp when it shares the bra, in FP64
+        // from here on also for FP32 quartets.  (Summed in FP32, all quartets of (H2O)_8/6-31G** in FP32: 2.0e-4 rms from
+        // the FP64 gradient, and 1.4e-3 left of the sum over the atoms; so 1.4e-4 and 7.6e-5, in the same 17.5 ms.)
         const unsigned bra0 = __shfl_sync(0xffffffffu, qt.bra, 0);
         const bool bra_warp = __all_sync(0xffffffffu, qt.bra == bra0);
-        Real gB[3], gD[3];
+        double gB[3];
+        Real gD[3];
 #pragma unroll
         for (int x = 0; x < 3; ++x)
         {
-            gB[x] = gP[x] - gA[x];
+            gB[x] = widen(gP[x]) - widen(gA[x]);
             gD[x] = -(gP[x] + gC[x]);
         }
         const int ta = v.shell_atom[bra.sh1], tb = v.shell_atom[bra.sh2];
-        if (bra_warp)
+        if (bra_warp && sizeof(Real) == 4)
         {
+            // Handed over half by half, each sum on a lane of its own: 9 FP64 additions and not 30, which this GPU
+            // takes at 1/64 of the FP32 rate.
+            double both[6] = {widen(gA[0]), widen(gA[1]), widen(gA[2]), gB[0], gB[1], gB[2]}, sum, none;
+            int at, at2;
+            warp_sum_spread<6>(both, lane, sum, at, none, at2);
+            if (at >= 0)
+                atomicAdd(grad + 3 * (at < 3 ? ta : tb) + at % 3, sum);
+        }
+        else
+        {
+            if (bra_warp)
+            {
 #pragma unroll
-            for (int x = 0; x < 3; ++x)
+                for (int x = 0; x < 3; ++x)
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
+                    for (int o = 16; o > 0; o >>= 1)
+                    {
+                        gA[x] += __shfl_xor_sync(0xffffffffu, gA[x], o);
+                        gB[x] += __shfl_xor_sync(0xffffffffu, gB[x], o);
+                    }
+            }
+            if (bra_warp ? lane == 0 : active)
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
                 {
-                    gA[x] += __shfl_xor_sync(0xffffffffu, gA[x], o);
-                    gB[x] += __shfl_xor_sync(0xffffffffu, gB[x], o);
+                    atomicAdd(grad + 3 * ta + x, widen(gA[x]));
+                    atomicAdd(grad + 3 * tb + x, gB[x]);
                 }
         }
-        if (bra_warp ? lane == 0 : active)
-#pragma unroll
-            for (int x = 0; x < 3; ++x)
-            {
-                atomicAdd(grad + 3 * ta + x, widen(gA[x]));
-                atomicAdd(grad + 3 * tb + x, widen(gB[x]));
-            }
         if (active)
         {
             const int tc = v.shell_atom[ket.sh1], td = v.shell_atom[ket.sh2];

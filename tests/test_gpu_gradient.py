@@ -130,3 +130,48 @@ def test_gradient_thread_form_matches_group_form(name):
     assert np.max(np.abs(out[False][0] - out[True][0])) <= 1e-11
     assert np.max(np.abs(out[False][1] - out[True][1])) <= 1e-7
     assert np.max(np.abs(out[False][0] - g["grad_fd"])) <= 1e-5
+
+
+def test_gradient_of_fp32_quartets_is_summed_in_fp64():
+    """Quartets of one bra pair (A, B), all in FP32: some of size 1 and most of 1e-6 in the same warps.  Switching the small
+    ones on (by the density of most other atoms, which leaves the large ones as they are) changes the forces on A and B by
+    what FP64 finds, to the small terms' own rounding: 1e-4 of the change, some hundred FP32 roundings.  A sum in FP32
+    beside the large terms rounds them at 3e-8 or more, a percent of the change."""
+    from hfgpu import basis
+    from hfgpu.engine import Engine
+
+    xyz = np.array([(x, y, z) for x in range(8) for y in range(4) for z in range(4)], float) * 2.0
+    xyz += np.random.default_rng(2).uniform(-0.2, 0.2, xyz.shape)
+    n = len(xyz)
+    Z = [1] * n
+    e = Engine(basis.pack("STO-3G", Z, xyz))
+    on = np.arange(n) % 16 == 3  # two large kets in 32
+    on[:2] = True
+    large = np.diag(on.astype(float))
+    large[0, 1] = large[1, 0] = 1.0
+    both = large + 1e-6 * np.diag(~on)
+    W = np.zeros((n, n))
+    change = {}
+    for precision in (0, 1):
+        g = [e.gradient(Z, xyz, D, D, W, sthr=0.0, dthr=0.0, precision=precision, fp32_cutoff=1e30)[0] for D in (large, both)]
+        change[precision] = (g[1] - g[0])[:2]
+    size = np.abs(change[0]).max()
+    assert 1e-8 < size < 1e-3
+    assert np.max(np.abs(change[1] - change[0])) <= 1e-4 * size, (change, size)
+
+
+@pytest.mark.parametrize("basis_name", ["6-31G**", "cc-pVDZ"])
+def test_gradient_forms_agree_on_long_lists(basis_name):
+    """Eight waters: lists of many waves, whose items the thread form takes through a counter.  1e-11 of the largest force
+    (some 10^6 terms rounded at 1e-16 of it each)."""
+    from hfgpu import basis, workloads
+    from hfgpu.engine import Engine
+
+    Z, xyz = workloads.water_lattice(2, 2, 2, seed=1)
+    e = Engine(basis.pack(basis_name, Z, xyz))
+    Da, _ = e.core_guess(Z, xyz, 0, 1)
+    W, g = np.zeros_like(Da), {}
+    for group_only in (False, True):
+        e.set_gradient_form(group_only)
+        g[group_only] = e.gradient(Z, xyz, Da, Da, W)[0]
+    assert np.max(np.abs(g[False] - g[True])) <= 1e-11 * np.abs(g[True]).max()
